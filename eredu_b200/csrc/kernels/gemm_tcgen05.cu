@@ -990,6 +990,9 @@ extern "C" int eredu_gemm_bf16_grouped(const void* X, const void* W, void* Y, co
   p.act = act;
   p.act_a = p.act_b = 0.f;
   p.act_limit = act_limit;
+  // An item holds at least one row and the used items come first: a step of few rows launches, and splits K for, no more items than it
+  // has rows. One token on 8 of 128 experts (gate_up 2 x 768 x 2048): 20.4 us with 129 items of which 121 were empty and K unsplit.
+  if (rows_cap < n_work) n_work = rows_cap;
   const int n_tiles = (N + 127) / 128;
   const int kblocks = (K + 63) / 64;
   int nsplit = 1;
