@@ -83,7 +83,7 @@ __device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t b
 
 __device__ __forceinline__ void mma_bf16_16816(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                                uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -100,25 +100,24 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
 //   sum_k (s (128 + n_k) + (b - 128 s)) x_k  =  s * sum_k (128 + n_k) x_k  +  (b - 128 s) * sum_k x_k
 // The sums of the activations come from the tensor core too (an all-ones A operand). No bf16 arithmetic is left in the
 // dequantisation (HFMA2 issues at half rate), and the weights are not rounded to bf16 at all.
-__device__ __forceinline__ void raw_word(uint32_t w, uint32_t* out) {
-  constexpr uint32_t kMask = 0x000F000Fu, kBase = 0x43004300u;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) out[j] = lop3_and_or(w >> (4 * j), kMask, kBase);
-}
+__device__ __forceinline__ uint32_t raw_pair(uint32_t w, int j) { return lop3_and_or(w >> (4 * j), 0x000F000Fu, 0x43004300u); }
 
 __device__ __forceinline__ void mma_bf16_16816_zero(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                                     uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// Per-warp ring of bulk copies. A slot holds four consecutive K blocks of the warp's row tile(s): the codes (512 bytes
+// Per-warp ring of bulk copies. A slot holds two consecutive K blocks of the warp's four row tiles: the codes (512 bytes
 // per block and tile) followed by their (scale, bias) words (64 bytes per group and tile). Both are contiguous in global
-// memory (tiled layouts), so a slot is filled by one bulk copy per tile and table: no registers are spent on prefetch
-// and a warp keeps several KB in flight, which is what the HBM latency asks for.
-constexpr int kGemvChunk = 4;
+// memory (tiled layouts), so a slot is filled by one bulk copy per tile and table, each issued by a lane of its own: no
+// registers are spent on prefetch and a warp keeps 9-14 KB in flight, which is what the HBM latency asks for.
+constexpr int kGemvChunk = 2;
+constexpr int kGemvTiles = 4;    // row tiles of a warp. What a K block costs once - its activations and their sums - is shared
+                                 // by 64 rows: with one tile per warp these were half of the instructions, and with eight tokens
+                                 // the activations were twice the bytes of the weights they met.
 
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -127,14 +126,21 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
                : "memory");
 }
 
-// GATED: two row tiles per warp (gate and up). RAW: accumulator-side affine map (group 64 / 128), else the weights are
-// dequantised to bf16 in registers (any power-of-two group from 16).
+// RAW: three slots (groups of at least 64, so that two CTAs fit an SM), else two.
+template <bool RAW>
+struct GemvRing {
+  static constexpr int kSlots = RAW ? 3 : 2;
+};
+
+// GATED: the warp's four row tiles are two of the gate and two of the up rows. RAW: accumulator-side affine map (group 64 / 128),
+// else the weights are dequantised to bf16 in registers (any power-of-two group from 16).
 template <bool GATED, bool RAW>
 __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvParams p) {
   constexpr int S = GATED ? 2 : 1;
+  constexpr int T = kGemvTiles, RT = T / S;        // tiles of a warp, of these tiles of output rows
   constexpr int TOK = 8;
   constexpr int C = kGemvChunk;
-  constexpr int SLOTS = GATED ? 2 : 4;       // 9 KB of ring per warp either way
+  constexpr int SLOTS = GemvRing<RAW>::kSlots;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);                  // [8 warps][SLOTS]
   uint8_t* ring = smem + 256;
@@ -145,24 +151,24 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int tiles_per_cta = 8 / p.wk;              // row tiles (16 rows) of this CTA
-  const int rows_cta = tiles_per_cta * 16;
-  const int wr = warp % tiles_per_cta, wkk = warp / tiles_per_cta;
+  const int groups_per_cta = 8 / p.wk;             // warps with rows of their own
+  const int rows_cta = groups_per_cta * 16 * RT;
+  const int wr = warp % groups_per_cta, wkk = warp / groups_per_cta;
   uint32_t crank = 0;
   if (p.ns > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
-  const int n0 = blockIdx.x * rows_cta + wr * 16;
+  const int n0 = blockIdx.x * rows_cta + wr * 16 * RT;
   const int split = static_cast<int>(crank) * p.wk + wkk;
   const int kb0 = min(split * p.blocks_per_split, p.kblocks);
-  const int kb1 = (n0 < p.n_out) ? min(kb0 + p.blocks_per_split, p.kblocks) : kb0;   // tiles beyond the matrix do nothing
+  const int kb1 = (n0 < p.n_out) ? min(kb0 + p.blocks_per_split, p.kblocks) : kb0;   // rows beyond the matrix do nothing
   const int nchunks = (kb1 - kb0 + C - 1) / C;
+  const int rt_live = min(RT, (p.n_out - n0 + 15) >> 4);   // row tiles that exist; the others compute on what the ring holds and are not stored
 
-  // slot layout: codes [S][C][512] | dq [S][gpc][16] words; gpc = groups per chunk
+  // slot layout: codes [T][C][512] | dq [T][gpc][16] words; gpc = groups per chunk. Tile s: output row tile s % RT, gate / up s / RT
   const int gpc = max(1, (C * 64) >> p.group_shift);
-  const int slot_bytes = S * C * 512 + S * gpc * 64;
+  const int slot_bytes = T * (C * 512 + gpc * 64);
   uint8_t* my_ring = ring + warp * SLOTS * slot_bytes;
   uint64_t* my_bars = bars + warp * SLOTS;
   const int groups_total = (p.kblocks * 64) >> p.group_shift;
-  const int tile0 = n0 >> 4;
 
   if (lane == 0) {
 #pragma unroll
@@ -171,32 +177,34 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
   }
   __syncwarp();
 
-  auto issue = [&](int c) {   // lane 0 only
-    const int kb = kb0 + c * C;
-    const int nb = min(C, kb1 - kb);
-    const int g0 = (kb * 64) >> p.group_shift;
-    const int ng = max(1, (nb * 64) >> p.group_shift);
+  // lane s < T copies the codes of tile s, lane T + s its (scale, bias) words
+  const int cs = lane % T;
+  const bool copies_dq = lane >= T;
+  const bool copies = lane < 2 * T && cs % RT < rt_live;
+  const size_t ctile = static_cast<size_t>((n0 >> 4) + cs % RT + (cs / RT) * (p.n_out >> 4));   // GATED: the up tiles follow the gate tiles
+  const uint8_t* csrc = copies_dq ? reinterpret_cast<const uint8_t*>(p.dq + (ctile * groups_total + ((kb0 * 64) >> p.group_shift)) * 16)
+                                  : p.wq + (ctile * p.kblocks + kb0) * 512;
+  const uint32_t cstep = copies_dq ? gpc * 64 : C * 512;
+  const uint32_t cdst = copies_dq ? T * C * 512 + cs * gpc * 64 : cs * C * 512;
+  auto issue = [&](int c) {   // whole warp
+    const int nb = min(C, kb1 - kb0 - c * C);
+    const uint32_t dq_bytes = max(1, (nb * 64) >> p.group_shift) * 64, code_bytes = nb * 512;
     uint8_t* slot = my_ring + (c % SLOTS) * slot_bytes;
     uint64_t* bar = &my_bars[c % SLOTS];
-    mbar_arrive_expect_tx(bar, static_cast<uint32_t>(S * (nb * 512 + ng * 64)));
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      const size_t tile = static_cast<size_t>(tile0 + s * (p.n_out >> 4));   // GATED: the up tiles follow the gate tiles
-      bulk_load(slot + s * C * 512, p.wq + (tile * p.kblocks + kb) * 512, static_cast<uint32_t>(nb * 512), bar);
-      bulk_load(slot + S * C * 512 + s * gpc * 64, p.dq + (tile * groups_total + g0) * 16, static_cast<uint32_t>(ng * 64), bar);
-    }
+    if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(rt_live * S) * (code_bytes + dq_bytes));
+    __syncwarp();
+    if (copies) bulk_load(slot + cdst, csrc + static_cast<size_t>(c) * cstep, copies_dq ? dq_bytes : code_bytes, bar);
   };
 
   // weights do not depend on the previous kernel: the ring is full before the dependency wait
-  if (lane == 0)
-    for (int c = 0; c < min(SLOTS, nchunks); ++c) issue(c);
+  for (int c = 0; c < min(SLOTS, nchunks); ++c) issue(c);
 
   pdl_wait();
   trace_mark(kTraceQGemm, kTraceAfterWait);
   pdl_launch_dependents();
   const unsigned int seq = p.use_comm ? *p.comm.seq : 0u;
 
-  // activations: token g, the 16 values that match this lane's codes; one chunk (four blocks) ahead in registers
+  // activations: token g, the 16 values that match this lane's codes; one chunk ahead in registers
   const __nv_bfloat16* xrow = p.x + static_cast<size_t>(min(g, p.M - 1)) * p.ldx + t * 16;
   uint4 xq[C][2];
 #pragma unroll
@@ -206,9 +214,9 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
     xq[j][1] = *reinterpret_cast<const uint4*>(xrow + k * 64 + 8);
   }
 
-  float acc[S][4];
+  float acc[T][4];
 #pragma unroll
-  for (int s = 0; s < S; ++s)
+  for (int s = 0; s < T; ++s)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[s][j] = 0.f;
 
@@ -218,58 +226,64 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
   constexpr uint32_t kOnes = 0x3F803F80u;
 
   bool ok = true;
+  int slot_i = 0, parity = 0;
   for (int c = 0; c < nchunks; ++c) {
-    const uint8_t* slot = my_ring + (c % SLOTS) * slot_bytes;
-    ok = mbar_wait(&my_bars[c % SLOTS], (c / SLOTS) & 1, p.status, kStatusTmaFullTimeout);
+    const uint8_t* slot = my_ring + slot_i * slot_bytes;
+    ok = mbar_wait(&my_bars[slot_i], parity, p.status, kStatusTmaFullTimeout);
     if (!ok) break;
     const int kbc = kb0 + c * C;
-    const int nb = min(C, kb1 - kbc);
+    const __nv_bfloat16* xnext = xrow + (kbc + C) * 64;
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      if (j < nb) {
+      if (kbc + j < kb1) {
         const uint32_t xb[8] = {xq[j][0].x, xq[j][0].y, xq[j][0].z, xq[j][0].w, xq[j][1].x, xq[j][1].y, xq[j][1].z, xq[j][1].w};
-        {
-          // the same block of the next chunk (clamped: a value that is never used)
-          const int k = min(kbc + C + j, p.kblocks - 1);
-          xq[j][0] = *reinterpret_cast<const uint4*>(xrow + k * 64);
-          xq[j][1] = *reinterpret_cast<const uint4*>(xrow + k * 64 + 8);
+        if (kbc + C + j < kb1) {                     // the same block of the next chunk
+          xq[j][0] = *reinterpret_cast<const uint4*>(xnext + j * 64);
+          xq[j][1] = *reinterpret_cast<const uint4*>(xnext + j * 64 + 8);
         }
         const int gi = RAW ? ((j * 64) >> p.group_shift) : (((j * 64) >> p.group_shift) + lane_group);
-        float tx[4];
+        const uint8_t* codes = slot + j * 512 + code_off;
+        const uint32_t* dqs = reinterpret_cast<const uint32_t*>(slot + T * C * 512) + gi * 16 + g;
         if (RAW) {
+          // the four tiles side by side: their chains of products do not wait for one another
+          float tx[4], tmp[T][4];
+          uint2 w_lo[T], w_hi[T];
+#pragma unroll
+          for (int s = 0; s < T; ++s) {
+            w_lo[s] = *reinterpret_cast<const uint2*>(codes + s * C * 512);
+            w_hi[s] = *reinterpret_cast<const uint2*>(codes + s * C * 512 + 8 * 32);
+          }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (i == 0) mma_bf16_16816_zero(tx, kOnes, kOnes, kOnes, kOnes, xb[0], xb[1]);
             else mma_bf16_16816(tx, kOnes, kOnes, kOnes, kOnes, xb[2 * i], xb[2 * i + 1]);
-          }
-        }
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-          const uint8_t* codes = slot + (s * C + j) * 512 + code_off;
-          const uint32_t* dq = reinterpret_cast<const uint32_t*>(slot + S * C * 512 + s * gpc * 64) + gi * 16 + g;
-          const uint2 w_lo = *reinterpret_cast<const uint2*>(codes);
-          const uint2 w_hi = *reinterpret_cast<const uint2*>(codes + 8 * 32);
-          const uint32_t sc_lo = dq[0], sc_hi = dq[8];
-          uint32_t a[2][8];
-          if (RAW) {
-            raw_word(w_lo.x, &a[0][0]);
-            raw_word(w_lo.y, &a[0][4]);
-            raw_word(w_hi.x, &a[1][0]);
-            raw_word(w_hi.y, &a[1][4]);
-            float tmp[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (i == 0) mma_bf16_16816_zero(tmp, a[0][0], a[1][0], a[0][1], a[1][1], xb[0], xb[1]);
-              else mma_bf16_16816(tmp, a[0][2 * i], a[1][2 * i], a[0][2 * i + 1], a[1][2 * i + 1], xb[2 * i], xb[2 * i + 1]);
+            for (int s = 0; s < T; ++s) {
+              const uint32_t lo = i < 2 ? w_lo[s].x : w_lo[s].y, hi = i < 2 ? w_hi[s].x : w_hi[s].y;
+              const int h = 2 * (i & 1);
+              const uint32_t a0 = raw_pair(lo, h), a1 = raw_pair(hi, h), a2 = raw_pair(lo, h + 1), a3 = raw_pair(hi, h + 1);
+              if (i == 0) mma_bf16_16816_zero(tmp[s], a0, a1, a2, a3, xb[0], xb[1]);
+              else mma_bf16_16816(tmp[s], a0, a1, a2, a3, xb[2 * i], xb[2 * i + 1]);
             }
+          }
+#pragma unroll
+          for (int s = 0; s < T; ++s) {
+            const uint32_t sc_lo = dqs[s * gpc * 16], sc_hi = dqs[s * gpc * 16 + 8];
             const float s_lo = __uint_as_float(sc_lo << 16), b_lo = __uint_as_float(sc_lo & 0xFFFF0000u);
             const float s_hi = __uint_as_float(sc_hi << 16), b_hi = __uint_as_float(sc_hi & 0xFFFF0000u);
             const float c_lo = fmaf(-128.f, s_lo, b_lo), c_hi = fmaf(-128.f, s_hi, b_hi);
-            acc[s][0] = fmaf(s_lo, tmp[0], fmaf(c_lo, tx[0], acc[s][0]));
-            acc[s][1] = fmaf(s_lo, tmp[1], fmaf(c_lo, tx[1], acc[s][1]));
-            acc[s][2] = fmaf(s_hi, tmp[2], fmaf(c_hi, tx[2], acc[s][2]));
-            acc[s][3] = fmaf(s_hi, tmp[3], fmaf(c_hi, tx[3], acc[s][3]));
-          } else {
+            acc[s][0] = fmaf(s_lo, tmp[s][0], fmaf(c_lo, tx[0], acc[s][0]));
+            acc[s][1] = fmaf(s_lo, tmp[s][1], fmaf(c_lo, tx[1], acc[s][1]));
+            acc[s][2] = fmaf(s_hi, tmp[s][2], fmaf(c_hi, tx[2], acc[s][2]));
+            acc[s][3] = fmaf(s_hi, tmp[s][3], fmaf(c_hi, tx[3], acc[s][3]));
+          }
+        } else {
+#pragma unroll
+          for (int s = 0; s < T; ++s) {
+            const uint2 w_lo = *reinterpret_cast<const uint2*>(codes + s * C * 512);
+            const uint2 w_hi = *reinterpret_cast<const uint2*>(codes + s * C * 512 + 8 * 32);
+            const uint32_t sc_lo = dqs[s * gpc * 16], sc_hi = dqs[s * gpc * 16 + 8];
+            uint32_t a[2][8];
             const uint32_t s2l = __byte_perm(sc_lo, sc_lo, 0x1010), b2l = __byte_perm(sc_lo, sc_lo, 0x3232);
             const uint32_t s2h = __byte_perm(sc_hi, sc_hi, 0x1010), b2h = __byte_perm(sc_hi, sc_hi, 0x3232);
             dequant_word(w_lo.x, s2l, b2l, &a[0][0]);
@@ -284,7 +298,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
       }
     }
     __syncwarp();                                   // every lane has its fragments of this slot in registers
-    if (lane == 0 && c + SLOTS < nchunks) issue(c + SLOTS);
+    if (c + SLOTS < nchunks) issue(c + SLOTS);
+    if (++slot_i == SLOTS) {
+      slot_i = 0;
+      parity ^= 1;
+    }
   }
   if (!ok) {
     // a copy never landed (status recorded): give the other copies of this warp their bounded wait before the ring is reused
@@ -292,14 +310,14 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
   }
 
   // ------------------------------------------------------------------ reduction over the K splits and epilogue
-  // plane of this warp's K split: [S][TOK][rows_cta + 4]; lane holds rows g / g + 8 and tokens 2t, 2t + 1 of each tile
+  // plane of this warp's K split: [gate, up][TOK][rows_cta + 4]; lane holds rows g / g + 8 and tokens 2t, 2t + 1 of each tile
   __syncthreads();                                  // every warp is done with its ring: the partial tiles take its place
   const int ldn = rows_cta + 4;
   const int plane = S * TOK * ldn;
   float* mine = red + wkk * plane;
 #pragma unroll
-  for (int s = 0; s < S; ++s) {
-    float* base = mine + (s * TOK + 2 * t) * ldn + wr * 16 + g;
+  for (int s = 0; s < T; ++s) {
+    float* base = mine + ((s / RT) * TOK + 2 * t) * ldn + (wr * RT + s % RT) * 16 + g;
     base[0] = acc[s][0];
     base[ldn] = acc[s][1];
     base[8] = acc[s][2];
@@ -445,12 +463,14 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
   trace_mark(kTraceQGemm, kTraceEnd);
 }
 
+// Rows of a CTA whose warps split K wk ways.
+static int gemv_rows(int wk, bool gated) { return 8 / wk * 16 * kGemvTiles / (gated ? 2 : 1); }
+
 // Dynamic shared memory of a launch: barriers, then the larger of the eight per-warp rings and the partial tiles.
-static int gemv_smem_bytes(const QGemvParams& p, bool gated) {
-  const int S = gated ? 2 : 1, C = kGemvChunk, slots = gated ? 2 : 4;
-  const int gpc = std::max(1, (C * 64) >> p.group_shift);
-  const int ring = 8 * slots * (S * C * 512 + S * gpc * 64);
-  const int red = p.wk * S * 8 * (128 / p.wk + 4) * 4;
+static int gemv_smem_bytes(const QGemvParams& p, bool gated, int slots) {
+  const int gpc = std::max(1, (kGemvChunk * 64) >> p.group_shift);
+  const int ring = 8 * slots * kGemvTiles * (kGemvChunk * 512 + gpc * 64);
+  const int red = p.wk * (gated ? 2 : 1) * 8 * (gemv_rows(p.wk, gated) + 4) * 4;
   return 256 + std::max(ring, red);
 }
 
@@ -459,7 +479,7 @@ static cudaError_t launch_gemv(const QGemvParams& p, int n_ctas, cudaStream_t st
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_ctas, p.ns, 1);
   cfg.blockDim = dim3(kGemvThreads, 1, 1);
-  const int smem = gemv_smem_bytes(p, GATED);
+  const int smem = gemv_smem_bytes(p, GATED, GemvRing<RAW>::kSlots);
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -533,41 +553,19 @@ extern "C" int eredu_qgemv4(const void* X, const void* wq, const void* dq, void*
     p.use_comm = 1;
     p.comm = *pc;
   }
-  // K splits. A warp streams best when it has many K blocks to itself, but an SM wants two CTAs (sixteen warps) to fill
-  // its issue slots, small CTAs spread more evenly over the SMs, and every further round of CTAs on an SM pays the fixed
-  // costs again (first data from HBM, reduction, epilogue: worth about sixteen K blocks). Estimate for each power-of-two
-  // split: the evenly spread work + half a CTA of imbalance + the fixed cost per round; take the smallest.
+  // K splits: over the warps of a CTA first, over the CTAs of a cluster when the rows alone do not give every SM its two CTAs
   const int sm = sm_count > 0 ? sm_count : 148;
-  const int row_tiles = (p.n_out + 15) / 16;
-  int ks = 1;
-  {
-    double best = 1e30;
-    for (int cand = 1; cand <= 64; cand *= 2) {
-      const int cwk = cand < 8 ? cand : 8, cns = cand / cwk;
-      if ((128 / cwk) % cns != 0) continue;
-      const int bps = ((p.kblocks + cand - 1) / cand + 3) / 4 * 4;
-      if (cand > 1 && bps * (cand - 1) >= p.kblocks) break;          // the last split would be empty
-      const long ctas = static_cast<long>((row_tiles + 8 / cwk - 1) / (8 / cwk)) * cns;
-      const long n = (ctas + sm - 1) / sm;                           // CTAs of the busiest SM
-      const double work = static_cast<double>(ctas) * 8.0 * bps / sm;   // warp-blocks per SM when spread evenly
-      const double t = work / 10.0 + 0.5 * bps + 16.0 * ((n + 1) / 2) + 2.0 * (cns - 1);
-      if (t < best) {
-        best = t;
-        ks = cand;
-      }
-    }
-  }
-  int wk = ks < 8 ? ks : 8, ns = ks / wk;
+  int wk = 8, ns = 1;
+  while (ns < 8 && static_cast<long>((p.n_out + gemv_rows(8, gated) - 1) / gemv_rows(8, gated)) * ns * 2 <= 2 * sm && p.kblocks >= 8 * ns * 2 * 4) ns *= 2;
+  while (wk > 1 && p.kblocks < wk * 2) wk >>= 1;
   if (force_wk > 0) wk = force_wk;
   if (force_ns > 0) ns = force_ns;
   if ((wk != 1 && wk != 2 && wk != 4 && wk != 8) || ns < 1 || ns > 8 || (ns & (ns - 1)) != 0) return -1;
-  // a cluster rank finishes rows_cta / ns whole columns
-  while (ns > 1 && (128 / wk) % ns != 0) ns >>= 1;
   p.wk = wk;
   p.ns = ns;
-  // splits start on multiples of four K blocks: a slot of the copy ring then starts on a group boundary for every group size
-  p.blocks_per_split = ((p.kblocks + wk * ns - 1) / (wk * ns) + 3) / 4 * 4;
-  const int n_ctas = (p.n_out + 128 / wk - 1) / (128 / wk);
+  // splits start on multiples of two K blocks: a slot of the copy ring then starts on a group boundary for every group size
+  p.blocks_per_split = ((p.kblocks + wk * ns - 1) / (wk * ns) + kGemvChunk - 1) / kGemvChunk * kGemvChunk;
+  const int n_ctas = (p.n_out + gemv_rows(wk, gated) - 1) / gemv_rows(wk, gated);
   const bool raw = group >= 64 && force_exact_bf16 == 0;
   cudaError_t e = gated ? (raw ? launch_gemv<true, true>(p, n_ctas, stream) : launch_gemv<true, false>(p, n_ctas, stream))
                         : (raw ? launch_gemv<false, true>(p, n_ctas, stream) : launch_gemv<false, false>(p, n_ctas, stream));
