@@ -498,23 +498,67 @@ __global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* __re
   const int kb = blockIdx.x, r = threadIdx.x >> 1, half = threadIdx.x & 1;
   const int n = blockIdx.y * 128 + r;
   if (n >= p.N) return;
-  constexpr int kRowK = FMT == QF_AFFINE4 ? 2 : 1;  // weights per byte
-  const size_t row_bytes = static_cast<size_t>(p.K) / kRowK;
-  const uint8_t* src = FMT == QF_AFFINE4
-                           ? wq + (static_cast<size_t>(n >> 4) * (p.K >> 6) + kb) * 512 + (n & 15) * 32 + half * 16
-                           : wq + static_cast<size_t>(n) * row_bytes + static_cast<size_t>(kb) * (64 / kRowK) + half * (32 / kRowK);
+  static_assert(FMT != QF_AFFINE4, "4-bit codes are decoded tile by tile");
+  const uint8_t* src = wq + static_cast<size_t>(n) * p.K + static_cast<size_t>(kb) * 64 + half * 32;
   __align__(16) uint8_t raw[64];
   __align__(16) uint8_t tile[128];
   // stage this thread's 32 weights as "row 0, half `half`" of a private one-row tile
-  if (FMT == QF_AFFINE4) *reinterpret_cast<uint4*>(raw + half * 16) = *reinterpret_cast<const uint4*>(src);
-  else {
-    *reinterpret_cast<uint4*>(raw + half * 32) = *reinterpret_cast<const uint4*>(src);
-    *reinterpret_cast<uint4*>(raw + half * 32 + 16) = *reinterpret_cast<const uint4*>(src + 16);
-  }
+  *reinterpret_cast<uint4*>(raw + half * 32) = *reinterpret_cast<const uint4*>(src);
+  *reinterpret_cast<uint4*>(raw + half * 32 + 16) = *reinterpret_cast<const uint4*>(src + 16);
   dequant_half_row<FMT>(p, raw, tile, 0, half, n, kb);
   uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(n) * p.K + kb * 64 + half * 32);
 #pragma unroll
   for (int c = 0; c < 4; ++c) dst[c] = *reinterpret_cast<const uint4*>(tile + ((half * 4 + c) << 4));
+}
+
+// The 4-bit form of it, bound by the bytes: a warp owns a row tile (16 rows) and four K blocks of it, which lie one after the other.
+// Loads are whole 128-byte lines (word w of a tile is row w / 8, codes 8 (w % 8) ..), sixteen of them in flight per lane, and eight
+// lanes write the 128 bytes of a row and block; the mapping above leaves a lane 64 bytes of its own, so that each of its stores touches
+// half a sector in 32 places. The four matrices of a layer 8192 wide (2.2 GB read and written): 597 us with that mapping.
+// grid (ceil(K / 256), ceil(N / 128)), 8 warps.
+__global__ void __launch_bounds__(256) dequant4_tiles_kernel(const uint32_t* __restrict__ wq, QGemmParams p, __nv_bfloat16* __restrict__ out) {
+  pdl_launch_early();
+  pdl_wait();
+  pdl_launch_dependents();
+  constexpr int kBlocks = 4;
+  const int lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * 16;
+  if (n0 >= p.N) return;
+  const int kblocks = p.K >> 6, kb0 = blockIdx.x * kBlocks;
+  const int c8 = (lane & 7) * 8;
+  const uint16_t* sc = reinterpret_cast<const uint16_t*>(p.scales_t);
+  const uint16_t* bi = reinterpret_cast<const uint16_t*>(p.biases_t);
+  const uint32_t* src = wq + (static_cast<size_t>(n0 >> 4) * kblocks + kb0) * 128 + lane;
+  uint32_t w[kBlocks][4], s2[kBlocks][4], b2[kBlocks][4];
+#pragma unroll
+  for (int b = 0; b < kBlocks; ++b) {
+    if (kb0 + b >= kblocks) break;
+    const size_t g = static_cast<size_t>(group_of(p, (kb0 + b) * 64 + c8)) * p.N;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[b][i] = src[b * 128 + i * 32];
+      const int n = min(n0 + i * 4 + (lane >> 3), p.N - 1);
+      s2[b][i] = sc[g + n];
+      b2[b][i] = bi[g + n];
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < kBlocks; ++b) {
+    if (kb0 + b >= kblocks) break;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int n = n0 + i * 4 + (lane >> 3);
+      const uint32_t s = s2[b][i] * 0x10001u, bb = b2[b][i] * 0x10001u;
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t pair = ((w[b][i] >> (4 * j)) & 0x000F000Fu) | 0x43004300u;   // (128 + n_2j, 128 + n_2j+1)
+        asm("sub.bf16x2 %0, %0, %1;" : "+r"(pair) : "r"(0x43004300u));
+        o[j] = bf16x2_fma(pair, s, bb);
+      }
+      if (n < p.N) *reinterpret_cast<uint4*>(out + static_cast<size_t>(n) * p.K + (kb0 + b) * 64 + c8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
 }
 
 }  // namespace eredu
@@ -535,7 +579,8 @@ static int dequant_impl(int fmt, const void* wq, const void* scales_t, const voi
   dim3 grid(K / 64, (N + 127) / 128);
   const uint8_t* w = static_cast<const uint8_t*>(wq);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
-  if (fmt == QF_AFFINE4) launch_pdl(dequant_matrix_kernel<QF_AFFINE4>, grid, dim3(256), 0, stream, w, p, o);
+  if (fmt == QF_AFFINE4)
+    launch_pdl(dequant4_tiles_kernel, dim3((K / 64 + 3) / 4, (N + 127) / 128), dim3(256), 0, stream, reinterpret_cast<const uint32_t*>(wq), p, o);
   else if (fmt == QF_FP8) launch_pdl(dequant_matrix_kernel<QF_FP8>, grid, dim3(256), 0, stream, w, p, o);
   else launch_pdl(dequant_matrix_kernel<QF_AFFINE8>, grid, dim3(256), 0, stream, w, p, o);
   eredu_count_launches(1);

@@ -145,9 +145,10 @@ def _linear_simt(x, w, bias, out_dtype, activation, out=None):
     return out
 
 
-def gated_linear(x, w_gate_up, inter, bias=None, out=None, force_split=0, row_ssq=None, norm_eps=0.0, activation="silu"):
+def gated_linear(x, w_gate_up, inter, bias=None, out=None, force_split=0, row_ssq=None, norm_eps=0.0, activation="silu",
+                 dynamic_weight=False):
     """Fused gated up-projection (SwiGLU; ``activation`` "relu": ReLU of the gate): one GEMM kernel, activation applied in the
-    epilogue (``row_ssq``: see linear). fp32 operands, and bf16 rows a TMA descriptor cannot describe, take the CUDA-core kernel."""
+    epilogue (``row_ssq``, ``dynamic_weight``: see linear). fp32 operands, and bf16 rows a TMA descriptor cannot describe, take the CUDA-core kernel."""
     if activation not in ("silu", "relu"):
         raise ValueError(f"unknown activation {activation!r}")
     if not x.is_cuda:
@@ -167,7 +168,8 @@ def gated_linear(x, w_gate_up, inter, bias=None, out=None, force_split=0, row_ss
     code = lib().eredu_gemm_bf16(
         ptr(x), ptr(w_gate_up), ptr(out), None, ptr(bias), M, inter, K, x.stride(0), w_gate_up.stride(0),
         out.stride(0), 0, w_gate_up.shape[0], 1, inter, 0, force_split, _sm_count(x.device),
-        ptr(status_word(x.device)), ptr(ssq_in), parts, eps, dim, None, 4 if activation == "relu" else 0, 0.0, 0.0, stream_ptr(x.device))
+        ptr(status_word(x.device)), ptr(ssq_in), parts, eps, dim, None,
+        (1 if dynamic_weight else 0) | (4 if activation == "relu" else 0), 0.0, 0.0, stream_ptr(x.device))
     check(code, "eredu_gemm_bf16(dual)")
     return out
 

@@ -1,0 +1,95 @@
+"""Kernels of the serving path at the edges of their tiles and at the borders between their variants, against fp32 references."""
+import pytest
+import torch
+
+from eredu_b200 import ops
+from eredu_b200.ops import moe as moe_ops
+from eredu_b200.ops.native import check_status
+from eredu_b200.ops.quant import QuantLinear
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF16 = 2.0 ** -8        # what rounding to bf16 changes at the most, relative to the number
+
+
+def rel_l2(a, b):
+    return float((a.float() - b.float()).norm() / b.float().norm())
+
+
+@pytest.fixture(autouse=True)
+def _status():
+    torch.manual_seed(0)
+    yield
+    check_status(torch.device("cuda", torch.cuda.current_device()))
+
+
+@pytest.mark.parametrize("M,n_q,n_kv", [(1, 8, 2), (3, 5, 1), (300, 32, 8), (17, 64, 8)])
+@pytest.mark.parametrize("D,rot,interleaved", [(128, 128, False), (64, 64, True), (128, 32, False), (64, 16, True), (64, 24, False), (128, 40, True)])
+def test_rotation_and_append_rows(M, n_q, n_kv, D, rot, interleaved):
+    """Token counts and head counts around what a CTA takes in one pass; rotated parts that are whole pairs of 16-byte pieces and such that
+    are not; rows that are part of wider ones, norms on queries only."""
+    wide = torch.randn(M, (n_q + 2 * n_kv) * D + 16, device=DEV).bfloat16()
+    qkv = wide[:, :(n_q + 2 * n_kv) * D]
+    pos = torch.randint(0, 9000, (M,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(40 * 16, device=DEV)[:M].long()
+    slots[M // 2] = -1 if M > 1 else 5
+    inv = 1.0 / (10000.0 ** (torch.arange(0, rot, 2, device=DEV).float() / rot))
+    qn = torch.rand(D, device=DEV) + 0.5 if M != 3 else None
+    kc, vc = (torch.zeros(40, n_kv, 16, D, device=DEV).bfloat16() for _ in range(2))
+    kr, vr = kc.clone(), vc.clone()
+    args = dict(rot=rot, interleaved=interleaved, q_norm_w=qn, attn_factor=1.25)
+    q = ops.rope_kv(qkv, pos, slots, inv, kc, vc, n_q, n_kv, D, **args)
+    ref = ops.rope_kv_ref(qkv.contiguous(), pos, slots, inv, kr, vr, n_q, n_kv, D, **args)
+    # sums in another order move a number by one place at the most, and few of them
+    assert rel_l2(q, ref) < BF16 and rel_l2(kc, kr) < BF16
+    assert torch.equal(vc, vr)
+
+
+@pytest.mark.parametrize("N,K,group", [(16, 64, 64), (650, 320, 32), (8, 1024, 128), (130, 192, 96), (256, 448, 16)])
+def test_decoded_weights(N, K, group):
+    """K blocks that are no multiple of a warp's four, rows that are no whole tiles, group sizes below, at and above a block."""
+    ql = QuantLinear.from_dense((torch.randn(N, K, device=DEV) * 0.05).bfloat16(), 4, group)
+    got, want = ql._dense().float(), ql.dequantize(torch.float32)
+    assert bool(((got - want).abs() <= 1.001 * BF16 * want.abs()).all())
+
+
+@pytest.mark.parametrize("M,inter,K,bits", [(257, 320, 512, 4), (300, 72, 192, 4), (513, 128, 256, 8)])
+def test_gated_projection_of_prompts(M, inter, K, bits):
+    ql = QuantLinear.from_dense((torch.randn(2 * inter, K, device=DEV) * 0.05).bfloat16(), bits, 64)
+    x = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    bias = torch.randn(2 * inter, device=DEV).bfloat16()
+    w = ql._dense().float()
+    y = x.float() @ w.t() + bias.float()
+    for limit in (0.0, 1.5):
+        ref = moe_ops.gated_act_ref(y[:, :inter], y[:, inter:], limit=limit)
+        # without a limit only the result is rounded; with one, gate and up are rounded in between as well
+        assert rel_l2(ql.gated(x, bias=bias, limit=limit), ref) < (BF16 if not limit else 3 * BF16)
+
+
+@pytest.mark.parametrize("M", [1, 2, 7, 8])
+@pytest.mark.parametrize("N,K,group,gated", [(48, 64, 64, False), (208, 192, 64, False), (2 * 48, 8192, 64, True), (1040, 4096, 128, False),
+                                             (2 * 4112, 2048, 32, True), (16, 320, 16, False)])
+def test_four_bit_rows_of_few_tokens(M, N, K, group, gated):
+    """Row tiles that do not fill a warp's four, K blocks that do not fill a slot of its ring or leave splits without any."""
+    ql = QuantLinear.from_dense((torch.randn(N, K, device=DEV) * 0.05).bfloat16(), 4, group)
+    x = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    y = x.float() @ ql.dequantize(torch.float32).t()
+    ref = moe_ops.gated_act_ref(y[:, :N // 2], y[:, N // 2:]) if gated else y
+    got = ql.gated(x) if gated else ql(x)
+    # the result is rounded; groups below 64 round the decoded weights too
+    assert rel_l2(got, ref) < (BF16 if group >= 64 else 2 * BF16)
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 64])
+@pytest.mark.parametrize("H,inter", [(256, 96), (2048, 768)])
+def test_experts_of_few_tokens(T, H, inter):
+    """Steps with fewer routes than the plan has room for items."""
+    E, k = 64, 8
+    x = torch.randn(T, H, device=DEV).bfloat16()
+    gu = (torch.randn(E, 2 * inter, H, device=DEV) / H ** 0.5).bfloat16()
+    dn = (torch.randn(E, H, inter, device=DEV) / inter ** 0.5).bfloat16()
+    logits = torch.randn(T, E, device=DEV)
+    ids, w, plan, xp = moe_ops.route_plan_gather(logits, x, k, "softmax", True, 1.0, None, 0, E)
+    got = moe_ops.experts_forward(x, ids, w, gu, dn, plan=plan, xp=xp)
+    # the product of gate and up and every expert's row are rounded to bf16 on both sides, the sum on this one
+    assert rel_l2(got, moe_ops.experts_ref(x, ids, w, gu, dn)) < 2 * BF16
