@@ -9,7 +9,7 @@
 //   * a 4-stage TMA ring (48 KB per stage) runs ahead across tile boundaries;
 //   * the epilogue transposes through a 16 KB staging buffer so that Y leaves the SM as 16-byte row chunks;
 //   * grouped (MoE) form: the tiles come from a work table {expert, first row, rows, -} built on the device, an item of at most 256 rows
-//     each; a short item shortens the MMA instead of multiplying rows nobody stores;
+//     each; a short item shortens the MMA and its copies (64 rows apiece) instead of fetching and multiplying rows nobody stores;
 //   * SwiGLU ("dual") tiles load 64 gate rows and 64 up rows into ONE 128-row operand tile, so gate and up use the
 //     same single 128x256 MMA stream as a plain GEMM; silu(gate) * up is formed when the staged rows are combined.
 //
@@ -33,6 +33,8 @@ constexpr int kStages = 4;
 constexpr int kATile = 128 * 64 * 2;             // 16 KB: 128 weight rows x 64 k
 constexpr int kBTile = kTN * 64 * 2;             // 32 KB: 256 tokens x 64 k
 constexpr int kStageBytes = kATile + kBTile;     // 48 KB
+constexpr int kBoxRows = 64;                     // grouped form: token rows of one copy
+constexpr int kBoxBytes = kBoxRows * 64 * 2;
 constexpr int kStagingBytes = 16 * 1024;
 constexpr int kCtrlBytes = 1024;
 constexpr int kSmemBytes = 1024 + kCtrlBytes + kStages * kStageBytes + kStagingBytes;
@@ -151,14 +153,20 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           ok = mbar_wait(&empty_bar[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
           if (!ok) break;
           uint8_t* a = stages + s * kStageBytes;
-          mbar_arrive_expect_tx(&full_bar[s], kStageBytes);
+          const int boxes = (tl.m_cnt + kBoxRows - 1) / kBoxRows;
+          mbar_arrive_expect_tx(&full_bar[s], GROUPED ? kATile + boxes * kBoxBytes : kStageBytes);
           if (DUAL) {
             tma_load_2d_hint(a, &tmW, kb * 64, w_row0, &full_bar[s], pol_w);
             tma_load_2d_hint(a + kATile / 2, &tmW, kb * 64, p.dual_row_offset + w_row0, &full_bar[s], pol_w);
           } else {
             tma_load_2d_hint(a, &tmW, kb * 64, w_row0, &full_bar[s], pol_w);
           }
-          tma_load_2d_hint(a + kATile, &tmX, kb * 64, m_base, &full_bar[s], pol_x);
+          if (GROUPED) {
+            for (int i = 0; i < boxes; ++i)
+              tma_load_2d_hint(a + kATile + i * kBoxBytes, &tmX, kb * 64, m_base + i * kBoxRows, &full_bar[s], pol_x);
+          } else {
+            tma_load_2d_hint(a + kATile, &tmX, kb * 64, m_base, &full_bar[s], pol_x);
+          }
           issued = it + 1;
         }
       }
@@ -404,7 +412,7 @@ int launch_gemm_persistent_grouped(const void* X, const void* W, void* Y, const 
   CUtensorMap tmW, tmX;
   int r = make_tma_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_rows_total, K, ldw, dual ? 64 : 128, 64);
   if (r != 0) return -100 + r;
-  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_cap, K, ldx, kTN, 64);
+  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_cap, K, ldx, kBoxRows, 64);
   if (r != 0) return -200 + r;
   PGemmParams p = {};
   p.y = Y;
