@@ -27,6 +27,8 @@
 // common exit (TMEM is freed there).
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "../common/elem.cuh"
 #include "../common/launch.h"
 #include "../common/launch_count.h"
@@ -59,6 +61,8 @@ struct AttnTcParams {
   // POOL form (window > 0): all whole blocks of `pool` tokens of a sequence as dense rows from pool_first[b] on
   const int* pool_first;
   int pool;
+  // SPLIT form: 2^gshift query heads of a key / value head share a tile, row = (token << gshift) + head
+  int gshift;
 };
 
 constexpr int kTcThreads = 320;
@@ -119,7 +123,12 @@ __device__ __forceinline__ int tc_query_tile(const AttnTcParams& p, int tiles, i
 
 // NK / NV: 64-wide halves of the key and of the value width. POOL: key tiles of 128 mean keys come in front of the tiles of the window; tile
 // index u walks the pooled tiles 0 .. pooled - 1, then the token tiles from j0 on.
-template <int NK, int NV, bool ROWS, bool POOL>
+//
+// SPLIT: for portions that are short against their context (the next message of a chat, a few drafted tokens). The form above gives such a
+// portion a CTA per query head that walks all keys with most of its rows empty, bound by that serial walk. Here the query heads of a key / value head share the rows of a tile, and the CTAs of a cluster take a part of the key tiles each;
+// their accumulators, maxima and sums meet in shared memory, where every CTA finishes some of the rows. 45 tokens behind 4096, 32 heads
+// of 128 over 8: 57.6 -> 18.5 us (behind 8192: 111 -> 26.6); 5 behind 2048: 30.8 -> 9.7.
+template <int NK, int NV, bool ROWS, bool POOL, bool SPLIT>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmR,
@@ -148,21 +157,42 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // heads vary fastest: the first wave holds the longest query tiles of every head (longest-first balances the causal
   // triangle), and neighbouring CTAs are query heads of one key / value head reading the same pages
-  const int b = blockIdx.z, head = blockIdx.x, qt = tc_query_tile(p, gridDim.y, blockIdx.y);
+  const int gs = SPLIT ? p.gshift : 0;
+  const int tile_tokens = kTcTile >> gs;
+  int nsplit = 1, rank = 0;
+  if (SPLIT) {
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(nsplit));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  }
+  const int b = blockIdx.z, head = SPLIT ? static_cast<int>(blockIdx.x) / nsplit << gs : blockIdx.x, qt = tc_query_tile(p, gridDim.y, blockIdx.y);
   const int4 seq = ROWS ? p.table[b] : make_int4(p.cu_q[b], p.cu_q[b + 1] - p.cu_q[b], 0, p.seq_lens[b]);
   const int q0 = seq.x, q_len = seq.y, kv_len = seq.w;
-  const int row0 = qt * kTcRows;
+  const int row0 = qt * 2 * tile_tokens;
   if (row0 >= q_len) return;                                            // uniform: before any barrier or allocation
   const int kv_head = head / (p.n_q_heads / p.n_kv_heads);
   const int pos0 = kv_len - q_len + row0;                               // position of the CTA's first query row
   // causal: nothing beyond the position of a tile's last row
-  const int n_a = min(kv_len - 1, pos0 + kTcTile - 1) / kTcTile + 1;
-  const int n_b = row0 + kTcTile < q_len ? min(kv_len - 1, pos0 + kTcRows - 1) / kTcTile + 1 : 0;
-  const int n_tiles = max(n_a, n_b);
+  int n_a = min(kv_len - 1, pos0 + tile_tokens - 1) / kTcTile + 1;
+  int n_b = row0 + tile_tokens < q_len ? min(kv_len - 1, pos0 + 2 * tile_tokens - 1) / kTcTile + 1 : 0;
+  int n_tiles = max(n_a, n_b);
   // window / chunk: key tiles that lie wholly before what a tile's FIRST row sees are skipped
-  const int j0_a = tc_lowest_key(p, pos0) / kTcTile;
-  const int j0_b = tc_lowest_key(p, pos0 + kTcTile) / kTcTile;
-  const int j0 = n_b > 0 ? min(j0_a, j0_b) : j0_a;
+  int j0_a = tc_lowest_key(p, pos0) / kTcTile;
+  int j0_b = tc_lowest_key(p, pos0 + tile_tokens) / kTcTile;
+  int j0 = n_b > 0 ? min(j0_a, j0_b) : j0_a;
+  if (SPLIT) {
+    // this CTA's key tiles; a query tile that sees none of them has an empty range at j0
+    const int per = (n_tiles - j0 + nsplit - 1) / nsplit;
+    const int begin = j0 + rank * per, end = min(n_tiles, begin + per);
+    j0_a = max(j0_a, begin);
+    n_a = min(n_a, end);
+    j0_b = max(j0_b, begin);
+    n_b = min(n_b, end);
+    const bool any_a = j0_a < n_a, any_b = j0_b < n_b;
+    j0 = any_a && any_b ? min(j0_a, j0_b) : any_a ? j0_a : any_b ? j0_b : 0;
+    if (!any_a) j0_a = n_a = j0;
+    if (!any_b) j0_b = n_b = j0;
+    n_tiles = max(n_a, n_b);
+  }
   // pooled tiles some row of query tile a, b sees (the last row sees most)
   const int np_a = POOL ? (pooled_seen(min(kv_len - 1, pos0 + kTcTile - 1), p.window, p.pool) + kTcTile - 1) / kTcTile : 0;
   const int np_b = POOL && n_b > 0 ? (pooled_seen(min(kv_len - 1, pos0 + kTcRows - 1), p.window, p.pool) + kTcTile - 1) / kTcTile : 0;
@@ -200,14 +230,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   pdl_launch_dependents();
 
   bool ok = true;
+  float m_row = -INFINITY, l_row = 0.f;      // SPLIT: a softmax thread's row
+  bool live_row = false;
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (lane == 0 && (!SPLIT || total > 0)) {
       mbar_arrive_expect_tx(q_full, 2 * NK * kTcHalf);
       for (int w = 0; w < 2; ++w)
         for (int h = 0; h < NK; ++h)
           // ROWS: the last half starts where the shared part does; a box that reaches beyond the per-head part meets zeros on the key side
-          tma_load_3d(q_s + (w * NK + h) * kTcHalf, &tmQ, ROWS && h == NK - 1 ? p.dk - p.rot : h * 64, head, q0 + row0 + w * kTcTile, q_full);
+          tma_load_3d(q_s + (w * NK + h) * kTcHalf, &tmQ, ROWS && h == NK - 1 ? p.dk - p.rot : h * 64, head, q0 + row0 + w * tile_tokens, q_full);
       const int* pages = p.block_table + static_cast<size_t>(b) * p.max_pages;
       const int pool_row = POOL ? p.pool_first[b] : 0;
       for (int jj = 0; jj < total && ok; ++jj) {
@@ -254,7 +286,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (lane == 0 && (!SPLIT || total > 0)) {
       const uint32_t q_addr = smem_u32(q_s);
       // jj: this CTA's iteration (selects the K / V stage); tile w is active on key tiles [first_w, n_w)
       const int first[2] = {j0_a, j0_b}, last[2] = {n_a, n_b};
@@ -324,9 +356,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int j0_w = w == 0 ? j0_a : j0_b;
     const int quarter = warp & 3;                                        // TMEM lanes this warp may touch
     const int row = quarter * 32 + lane;
-    const int tile_row0 = row0 + w * kTcTile;
-    const int tile_pos0 = pos0 + w * kTcTile;
-    const int qpos = tile_pos0 + row;
+    const int tile_row0 = row0 + w * tile_tokens;
+    const int tile_pos0 = pos0 + w * tile_tokens;
+    const int qpos = tile_pos0 + (row >> gs);
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t s_addr = tmem + lane_addr + w * 128;
     const uint32_t o_addr = tmem + lane_addr + 256 + w * 128;
@@ -343,7 +375,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       for (int c = 0; c < 8; ++c) tmem_ld16(s_addr + c * 16, sc[c]);
       tmem_wait_ld();
       const int key0 = j * kTcTile;
-      const bool before = key0 < tc_lowest_key(p, tile_pos0 + kTcTile - 1);     // some row's visible keys start inside or after this tile
+      const bool before = key0 < tc_lowest_key(p, tile_pos0 + tile_tokens - 1);     // some row's visible keys start inside or after this tile
       if (means) {
         const int blocks = pooled_seen(qpos, p.window, p.pool) - key0;   // of this tile's
         if (key0 + kTcTile > pooled_seen(tile_pos0, p.window, p.pool)) {
@@ -418,8 +450,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       unpack_f32x2(add_f32x2(add_f32x2(acc[0], acc[1]), add_f32x2(acc[2], acc[3])), s0, s1);
       l += s0 + s1;
     }
-    if (ok && n_w > 0) ok = mbar_wait(&o_final[w], 0, p.status, kStatusAccumTimeout);
-    if (ok && n_w > 0) {
+    if (ok && n_w > j0_w) ok = mbar_wait(&o_final[w], 0, p.status, kStatusAccumTimeout);
+    if (SPLIT) {
+      m_row = m;
+      l_row = l;
+      live_row = ok && n_w > j0_w;
+    } else if (ok && n_w > 0) {
       tc_fence_after_sync();
       const bool store = tile_row0 + row < q_len;
       if (p.sinks != nullptr) l += ex2_approx(p.sinks[head] * 1.4426950408889634f - m);
@@ -456,6 +492,74 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
     }
   }
+  if (SPLIT) {
+    // Both query tiles are done: operand tiles make room for the accumulators, [256 rows][dv] fp32 with the 16-byte pieces of a row
+    // permuted by its index (threads of a warp write different banks), and {maximum, sum} of the rows behind them.
+    __syncthreads();
+    constexpr int kPieces = NV * 16;                                     // 16-byte pieces of a row: dv = 64 NV here
+    float4* part = reinterpret_cast<float4*>(smem);
+    float2* ml = reinterpret_cast<float2*>(smem + kTcRows * kPieces * 16);
+    if (warp >= 2) {
+      const int w = (warp - 2) >> 2, quarter = warp & 3;
+      const int r = w * kTcTile + quarter * 32 + lane;
+      const bool any = __any_sync(0xffffffffu, live_row);
+      if (any) {
+        tc_fence_after_sync();
+        const uint32_t o_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + 256 + w * 128;
+#pragma unroll 1
+        for (int c = 0; c < kPieces / 4; ++c) {
+          uint32_t o[16];
+          tmem_ld16(o_addr + c * 16, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            part[r * kPieces + ((c * 4 + i) ^ (r & (kPieces - 1)))] =
+                make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]), __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3]));
+        }
+      }
+      ml[r] = make_float2(live_row ? m_row : -INFINITY, live_row ? l_row : 0.f);
+    }
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    const uint32_t part_addr = smem_u32(part), ml_addr = smem_u32(ml);
+    const int rows = min(2 * tile_tokens, q_len - row0) << gs;
+    constexpr int kLanes = kPieces;                                      // lanes that share a row
+    for (int r = rank + nsplit * (warp * (32 / kLanes) + lane / kLanes); r < rows; r += nsplit * (kTcThreads / kLanes)) {
+      const int piece = lane % kLanes;
+      const uint32_t at = part_addr + static_cast<uint32_t>(r * kPieces + (piece ^ (r & (kPieces - 1)))) * 16u;
+      float2 v[8];
+      float top = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        v[s] = make_float2(-INFINITY, 0.f);
+        if (s < nsplit) asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[s].x), "=f"(v[s].y) : "r"(mapa_shared(ml_addr + r * 8u, s)));
+        top = fmaxf(top, v[s].x);
+      }
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      float l = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        if (s < nsplit && v[s].x > -INFINITY) {
+          const float a = ex2_approx(v[s].x - top);
+          float4 o;
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(mapa_shared(at, s)));
+          l += a * v[s].y;
+          sum.x += a * o.x;
+          sum.y += a * o.y;
+          sum.z += a * o.z;
+          sum.w += a * o.w;
+        }
+      }
+      const int h = head + (r & ((1 << gs) - 1));
+      if (p.sinks != nullptr) l += ex2_approx(p.sinks[h] * 1.4426950408889634f - top);
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      uint2* dst = reinterpret_cast<uint2*>(p.out + (static_cast<size_t>(q0 + row0 + (r >> gs)) * p.n_q_heads + h) * p.dv);
+      dst[piece] = make_uint2(pack_bf16x2(sum.x * inv, sum.y * inv), pack_bf16x2(sum.z * inv, sum.w * inv));
+    }
+    __syncwarp();
+    cluster_arrive_release();                                            // nobody leaves while a peer reads its rows
+    cluster_wait_acquire();
+  }
   // common exit: every role comes here, also after a timed-out wait; the tensor memory goes back
   tc_fence_before_sync();
   __syncthreads();
@@ -469,32 +573,70 @@ using namespace eredu;
 
 // Causal prefill attention over the paged cache, key / value widths up to 128, optional window or chunks and sink logits.
 // q: [tokens, n_q, key_dim] bf16 (contiguous); k_cache / v_cache: [pages, n_kv, 16, width] bf16 (contiguous); sinks: fp32 [n_q] or
-// null. Same arguments as eredu_attn_prefill otherwise. Returns -2 for shapes it does not take.
-template <int NK, int NV, bool ROWS = false, bool POOL = false>
+// null. max_kv_len: the longest context, where the host knows it (0 otherwise): short portions are then split over the keys. Same
+// arguments as eredu_attn_prefill otherwise. Returns -2 for shapes it does not take.
+template <int NK, int NV, bool ROWS = false, bool POOL = false, bool SPLIT = false>
 static int launch_attn_tc(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmR, const CUtensorMap& tmS,
-                          const AttnTcParams& p, dim3 grid, cudaStream_t stream) {
+                          const AttnTcParams& p, dim3 grid, cudaStream_t stream, int nsplit = 1) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(attn_prefill_tc_kernel<NK, NV, ROWS, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem(NK, NV)) != cudaSuccess) return -1;
+    if (cudaFuncSetAttribute(attn_prefill_tc_kernel<NK, NV, ROWS, POOL, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem(NK, NV)) != cudaSuccess) return -1;
     configured[dev] = true;
   }
-  return static_cast<int>(launch_pdl(attn_prefill_tc_kernel<NK, NV, ROWS, POOL>, grid, dim3(kTcThreads), tc_smem(NK, NV), stream, tmQ, tmK, tmV, tmR, tmS, p));
+  if (SPLIT) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = tc_smem(NK, NV);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nsplit;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return static_cast<int>(cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel<NK, NV, ROWS, POOL, SPLIT>, tmQ, tmK, tmV, tmR, tmS, p));
+  }
+  return static_cast<int>(launch_pdl(attn_prefill_tc_kernel<NK, NV, ROWS, POOL, SPLIT>, grid, dim3(kTcThreads), tc_smem(NK, NV), stream, tmQ, tmK, tmV, tmR, tmS, p));
 }
 
 static int attn_prefill_tc_impl(const void* q, const void* k_cache, const void* v_cache, const void* k_rows, const void* v_rows, void* out,
                                 const int* block_table, const int* seq_lens, const int* cu_q, const int* pool_first, const float* sinks, int batch,
                                 int total_q, int max_q_len, int max_pages, int num_pages, int rows, int n_q_heads, int n_kv_heads, int key_dim,
-                                int value_dim, int window, int chunk, int pool, float scale, int* status, cudaStream_t stream) {
+                                int value_dim, int window, int chunk, int pool, int max_kv_len, int sm_count, float scale, int* status,
+                                cudaStream_t stream) {
   if (key_dim <= 0 || key_dim > 128 || key_dim % 8 != 0 || value_dim <= 0 || value_dim > 128 || value_dim % 8 != 0 || batch <= 0 ||
       total_q <= 0 || n_kv_heads <= 0 || n_q_heads % n_kv_heads != 0 || window < 0 || chunk < 0)
     return -2;
   const uint64_t D = static_cast<uint64_t>(key_dim), V = static_cast<uint64_t>(value_dim);
   CUtensorMap tmQ, tmK, tmV;
-  // q as [tokens][heads][D]: box = 128 tokens x 1 head x 64 values
+  // Short portions (see SPLIT above the kernel): heads of 64 or 128, no chunks or pooled blocks, a context that the host has stated.
+  // Up to eight splits (a portable cluster) while they find SMs of their own and two key tiles each - eight only on half of the SMs:
+  // a GPC does not always have room for two such clusters, and then the rest waits (33.6 us with 16 clusters, 18.5 with eight). The estimates
+  // in us are what either form measured with heads of 128: start and end of a CTA, and a key tile.
+  int gshift = 0, nsplit = 1;
+  bool split_form = false;
+  if (max_kv_len > 0 && pool == 0 && chunk == 0 && key_dim == value_dim && (key_dim == 64 || key_dim == 128)) {
+    const int group = n_q_heads / n_kv_heads, sm = sm_count > 0 ? sm_count : 148;
+    if (max_q_len <= kTcRows && group <= 16 && (group & (group - 1)) == 0)
+      while ((1 << gshift) < group) ++gshift;
+    const int tokens = kTcRows >> gshift;
+    const long ctas = static_cast<long>(n_q_heads >> gshift) * ((max_q_len + tokens - 1) / tokens) * batch;
+    const int seen = window > 0 ? std::min(max_kv_len, window + tokens + kTcTile) : max_kv_len;
+    const int tiles = (seen + kTcTile - 1) / kTcTile;
+    while (nsplit < 8 && ctas * nsplit * 2 <= (nsplit < 4 ? sm : sm / 2) && tiles >= nsplit * 2 * 2) nsplit *= 2;
+    const long whole = static_cast<long>(n_q_heads) * ((max_q_len + kTcRows - 1) / kTcRows) * batch;
+    const double t_whole = ((whole + sm - 1) / sm) * (5.0 + 1.75 * tiles), t_split = 9.0 + 2.0 * ((tiles + nsplit - 1) / nsplit);
+    split_form = nsplit > 1 && t_split < t_whole;
+    if (!split_form) gshift = 0, nsplit = 1;
+  }
+  // q as [tokens][heads][D]: box = 128 rows (128 tokens x 1 head, or fewer tokens x the heads that share a tile) x 64 values
   int r = make_tma_3d(&tmQ, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, D, static_cast<uint64_t>(n_q_heads),
-                      static_cast<uint64_t>(total_q), D * 2, static_cast<uint64_t>(n_q_heads) * D * 2, 64, 1, 128);
+                      static_cast<uint64_t>(total_q), D * 2, static_cast<uint64_t>(n_q_heads) * D * 2, 64, 1 << gshift, 128 >> gshift);
   if (r != 0) return -100 + r;
   r = make_tma_4d(&tmK, k_cache, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, D, 16, static_cast<uint64_t>(n_kv_heads),
                   static_cast<uint64_t>(num_pages), D * 2, 16 * D * 2, static_cast<uint64_t>(n_kv_heads) * 16 * D * 2, 64, 16, 1, 1);
@@ -540,6 +682,14 @@ static int attn_prefill_tc_impl(const void* q, const void* k_cache, const void* 
     eredu_count_launches(1);
     return e;
   }
+  if (split_form) {
+    p.gshift = gshift;
+    grid = dim3((n_q_heads >> gshift) * nsplit, (max_q_len + (kTcRows >> gshift) - 1) / (kTcRows >> gshift), batch);
+    e = key_dim > 64 ? launch_attn_tc<2, 2, false, false, true>(tmQ, tmK, tmV, tmK, tmV, p, grid, stream, nsplit)
+                     : launch_attn_tc<1, 1, false, false, true>(tmQ, tmK, tmV, tmK, tmV, p, grid, stream, nsplit);
+    eredu_count_launches(1);
+    return e;
+  }
   if (key_dim > 64) e = value_dim > 64 ? launch_attn_tc<2, 2>(tmQ, tmK, tmV, tmK, tmV, p, grid, stream) : launch_attn_tc<2, 1>(tmQ, tmK, tmV, tmK, tmV, p, grid, stream);
   else e = value_dim > 64 ? launch_attn_tc<1, 2>(tmQ, tmK, tmV, tmK, tmV, p, grid, stream) : launch_attn_tc<1, 1>(tmQ, tmK, tmV, tmK, tmV, p, grid, stream);
   eredu_count_launches(1);
@@ -549,9 +699,9 @@ static int attn_prefill_tc_impl(const void* q, const void* k_cache, const void* 
 extern "C" int eredu_attn_prefill_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
                                      const int* seq_lens, const int* cu_q, const float* sinks, int batch, int total_q, int max_q_len,
                                      int max_pages, int num_pages, int n_q_heads, int n_kv_heads, int key_dim, int value_dim, int window,
-                                     int chunk, float scale, int* status, cudaStream_t stream) {
+                                     int chunk, int max_kv_len, int sm_count, float scale, int* status, cudaStream_t stream) {
   return attn_prefill_tc_impl(q, k_cache, v_cache, nullptr, nullptr, out, block_table, seq_lens, cu_q, nullptr, sinks, batch, total_q, max_q_len,
-                              max_pages, num_pages, 0, n_q_heads, n_kv_heads, key_dim, value_dim, window, chunk, 0, scale, status, stream);
+                              max_pages, num_pages, 0, n_q_heads, n_kv_heads, key_dim, value_dim, window, chunk, 0, max_kv_len, sm_count, scale, status, stream);
 }
 
 // The POOL form: over the `window` newest tokens and the means of the blocks of `pool` tokens that end before them. k_rows / v_rows [rows,
@@ -562,7 +712,7 @@ extern "C" int eredu_attn_prefill_tc_pooled(const void* q, const void* k_cache, 
                                             int key_dim, int value_dim, int window, int pool, float scale, int* status, cudaStream_t stream) {
   if (window <= 0 || pool <= 0 || rows < 0 || pool_first == nullptr || (rows > 0 && (k_rows == nullptr || v_rows == nullptr))) return -2;
   return attn_prefill_tc_impl(q, k_cache, v_cache, k_rows, v_rows, out, block_table, seq_lens, cu_q, pool_first, nullptr, batch, total_q, max_q_len,
-                              max_pages, num_pages, rows, n_q_heads, n_kv_heads, key_dim, value_dim, window, 0, pool, scale, status, stream);
+                              max_pages, num_pages, rows, n_q_heads, n_kv_heads, key_dim, value_dim, window, 0, pool, 0, 0, scale, status, stream);
 }
 
 // The ROWS form. q [total_q rows of ldq elements], head h at column h * (dim + rot): [per-head part (dim) | shared part (rot)]; k [rows of

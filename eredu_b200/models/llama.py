@@ -304,7 +304,8 @@ class CausalLM:
                         norm_w_off=cfg.norm_weight_offset, mrope_section=(cfg.rope_scaling or {}).get("mrope_section"))
         if batch.is_prefill:
             attn = ops.attention_prefill(q, k_cache, v_cache, batch.block_table, batch.seq_lens, batch.cu_q,
-                                         batch.max_q_len, self.scale, window=window, sinks=lw.sinks)
+                                         batch.max_q_len, self.scale, window=window, sinks=lw.sinks,
+                                         max_kv_len=max((a + n for a, n in batch.portions), default=0) if batch.portions else 0)
         else:
             attn = ops.attention_decode(q, k_cache, v_cache, batch.block_table, batch.seq_lens, batch.q_per_seq,
                                         self.scale, splits=batch.splits, window=window, sinks=lw.sinks,

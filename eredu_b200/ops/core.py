@@ -570,9 +570,10 @@ def _tensor_core_dims(q, k_cache, v_cache) -> bool:
 
 
 def attention_prefill(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_len, scale, window=0, sinks=None,
-                      out=None, chunk=0):
+                      out=None, chunk=0, max_kv_len=0):
     """``window`` > 0: a query at position p sees keys in (p - window, p]; ``chunk`` > 0: the keys of its own chunk of
-    positions. Key and value widths are those of the caches. Returns [total_q, n_q, value width]."""
+    positions. ``max_kv_len``: the largest of ``seq_lens`` where the host knows it (it chooses how the work is split, never what is
+    computed; 0: unknown). Key and value widths are those of the caches. Returns [total_q, n_q, value width]."""
     if q.is_cuda and (chunk > 0 or q.dtype == torch.float32 or v_cache.shape[3] != q.shape[2]):
         if not _tensor_core_dims(q, k_cache, v_cache):
             return _attention_simt(q, k_cache, v_cache, block_table, seq_lens, cu_q, 0, max_q_len, scale, window, chunk, sinks)
@@ -592,8 +593,8 @@ def attention_prefill(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_le
         # tcgen05 kernel (csrc/kernels/attention_tc.cu): QK^T and PV on the 5th-generation tensor cores, pages by TMA
         code = lib().eredu_attn_prefill_tc(ptr(q), ptr(k_cache), ptr(v_cache), ptr(out), ptr(block_table), ptr(seq_lens),
                                            ptr(cu_q), ptr(sinks), B, q.shape[0], max_q_len, block_table.stride(0),
-                                           k_cache.shape[0], q.shape[1], k_cache.shape[1], dk, dv, int(window), int(chunk), scale,
-                                           ptr(status_word(q.device)), stream_ptr(q.device))
+                                           k_cache.shape[0], q.shape[1], k_cache.shape[1], dk, dv, int(window), int(chunk), int(max_kv_len),
+                                           _sm_count(q.device), scale, ptr(status_word(q.device)), stream_ptr(q.device))
         check(code, "eredu_attn_prefill_tc")
         return out
     code = lib().eredu_attn_prefill(ptr(q), ptr(k_cache), ptr(v_cache), ptr(out), ptr(block_table), ptr(seq_lens),

@@ -93,3 +93,32 @@ def test_experts_of_few_tokens(T, H, inter):
     got = moe_ops.experts_forward(x, ids, w, gu, dn, plan=plan, xp=xp)
     # the product of gate and up and every expert's row are rounded to bf16 on both sides, the sum on this one
     assert rel_l2(got, moe_ops.experts_ref(x, ids, w, gu, dn)) < 2 * BF16
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(128, 32, 8), (64, 8, 8), (128, 16, 1), (64, 12, 2), (128, 32, 1)])
+@pytest.mark.parametrize("q_lens,kv_lens,window,sinks", [
+    ([45], [4141], 0, False),                       # the next message of a chat
+    ([1, 5, 130], [2000, 77, 130], 0, True),        # beside each other: one that sees fewer tiles than there are splits
+    ([16, 17, 64, 65], [1024, 1025, 639, 1153], 0, False),
+    ([33, 2], [1500, 3000], 200, True),             # parts of the keys that no row of a cluster's CTA sees
+    ([300, 7], [3000, 900], 0, False)])             # more than one tile of rows
+def test_attention_of_short_portions(D, n_q, n_kv, q_lens, kv_lens, window, sinks):
+    pages = [(n + 15) // 16 for n in kv_lens]
+    kc, vc = (torch.randn(sum(pages) + 1, n_kv, 16, D, device=DEV).bfloat16() for _ in range(2))
+    bt = torch.zeros(len(pages), max(pages) + 3, dtype=torch.int32, device=DEV)
+    ids, at = torch.randperm(sum(pages), device=DEV).int() + 1, 0
+    for i, n in enumerate(pages):
+        bt[i, :n] = ids[at:at + n]
+        at += n
+    q = (torch.randn(sum(q_lens), n_q, D, device=DEV) * 1.5).bfloat16()
+    cu = torch.tensor([0] + torch.tensor(q_lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    lens = torch.tensor(kv_lens, dtype=torch.int32, device=DEV)
+    sink = torch.randn(n_q, device=DEV) if sinks else None
+    args = (q, kc, vc, bt, lens, cu, max(q_lens), D ** -0.5)
+    got = ops.attention_prefill(*args, window=window, sinks=sink, max_kv_len=max(kv_lens))
+    ref = ops.attention_ref(q, kc, vc, bt, lens, q_lens, D ** -0.5, window, sink)
+    whole = ops.attention_prefill(*args, window=window, sinks=sink)       # unsplit, a query head per CTA
+    # probabilities and the result are rounded to bf16; the two forms sum in another order
+    assert rel_l2(got, ref) < 2 * BF16 and rel_l2(got, whole) < 2 * BF16
+    # a context the host understates only changes the split
+    assert rel_l2(ops.attention_prefill(*args, window=window, sinks=sink, max_kv_len=600), whole) < 2 * BF16
