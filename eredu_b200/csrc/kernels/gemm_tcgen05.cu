@@ -745,6 +745,8 @@ static cudaError_t launch_gemm_split(const CUtensorMap& tmW, const CUtensorMap& 
 
 }  // namespace eredu
 
+#include "gemv_rows.cuh"
+
 using namespace eredu;
 
 EREDU_TRACE_INSTALLER(gemm)
@@ -773,6 +775,19 @@ static bool staged_epilogue_ok(const void* Y, const void* residual, int N, int l
   if (out_fp32 || N % 8 != 0 || ldy % 8 != 0 || (reinterpret_cast<uintptr_t>(Y) & 15) != 0) return false;
   if (residual != nullptr && (ldr % 8 != 0 || (reinterpret_cast<uintptr_t>(residual) & 15) != 0)) return false;
   return true;
+}
+
+// Whether the call runs on gemv_rows_kernel: one or two tokens, whole 16-byte pieces of rows, whole CTAs of columns, weights that no
+// kernel just before this one writes - and few enough of them. With one token the kernel alone is the faster one at any size (2048 x
+// 2048 5.8 -> 4.5 us, 6144 x 4096 12.2 -> 10.9, 4096 x 14336 21.3 -> 20.4), but in a decode step, behind other kernels, the copy
+// rings of the tensor-core kernel start with 160 KB an SM where this one holds 64 KB a CTA: taking matrices up to 16 MB makes a
+// step of 16 layers 2048 wide 766 -> 728 us, up to 24 MB one of 8 expert layers 672 -> 628; 33 MB and above lose it again (759 us, and
+// 912 -> 945 for 8 layers 4096 wide). Two tokens are twice the arithmetic on the CUDA cores: 3072 x 2048 5.7 -> 5.1 us, 5120 x 2048
+// 6.8 -> 7.8.
+static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K, int ldx, int ldw, int dual, int flags, int force_split) {
+  if (force_split > 0 || dual || M > 2 || (flags & 1) || K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || N % kRowsOut != 0) return false;
+  if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) != 0) return false;
+  return static_cast<long long>(N) * K * 2 <= (M == 1 ? 24LL : 13LL) << 20;
 }
 
 // Number of K splits the launcher would use (exposed for tests and tuning).
@@ -811,11 +826,6 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
                                           stream);
     if (pr != kPersistentUnsupported) return pr;
   }
-  CUtensorMap tmW, tmX;
-  int r = make_tma_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_rows, K, ldw, 128, 64);
-  if (r != 0) return -100 + r;
-  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, ldx, tn, 64);
-  if (r != 0) return -200 + r;
   GemmParams p;
   p.y = Y;
   p.residual = residual;
@@ -846,13 +856,23 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   // first stages are fetched before the dependency wait (level 1), and for matrices that fit L2 many times over
   // the remaining tiles are prefetched into L2 as well (level 2). EREDU_GEMM_PREFETCH overrides the level.
   p.w_static = (flags & 1) ? 0 : prefetch_level(static_cast<long long>(w_rows) * K * 2);
+  cudaError_t e;
+  if (rows_kernel_takes(X, W, M, N, K, ldx, ldw, dual, flags, force_split)) {
+    e = M == 1 ? launch_rows<1>(p, X, W, ldx, ldw, stream) : launch_rows<2>(p, X, W, ldx, ldw, stream);
+    eredu_count_launches(1);
+    return static_cast<int>(e);
+  }
+  CUtensorMap tmW, tmX;
+  int r = make_tma_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_rows, K, ldw, 128, 64);
+  if (r != 0) return -100 + r;
+  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, ldx, tn, 64);
+  if (r != 0) return -200 + r;
   const int n_tiles = (N + 127) / 128;
   const int m_tiles = (M + tn - 1) / tn;
   int nsplit = force_split > 0 ? force_split : eredu_gemm_pick_split(M, N, K, sm_count > 0 ? sm_count : 148);
   const int kblocks = (K + 63) / 64;
   while (nsplit > 1 && (kblocks + nsplit - 1) / nsplit * (nsplit - 1) >= kblocks) nsplit >>= 1;  // no empty split
   p.staged = staged_epilogue_ok(Y, residual, N, ldy, ldr, out_fp32) && tn >= 64 && nsplit == 1;
-  cudaError_t e;
 #define ER_DISPATCH(TN_)                                                                     \
   case TN_:                                                                                  \
     e = dual ? launch_gemm_split<TN_, true>(tmW, tmX, p, n_tiles, m_tiles, nsplit, stream)   \

@@ -122,3 +122,47 @@ def test_attention_of_short_portions(D, n_q, n_kv, q_lens, kv_lens, window, sink
     assert rel_l2(got, ref) < 2 * BF16 and rel_l2(got, whole) < 2 * BF16
     # a context the host understates only changes the split
     assert rel_l2(ops.attention_prefill(*args, window=window, sinks=sink, max_kv_len=600), whole) < 2 * BF16
+
+
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("N,K", [(16, 8), (128, 2048), (144, 2056), (2048, 1000), (1040, 4096), (256, 6152)])
+def test_rows_of_one_and_two_tokens(M, N, K):
+    """Pieces of K that do not fill a pass of the CTA or its two batches, columns that do not fill a cluster; all of the epilogue."""
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    bias, res = torch.randn(N, device=DEV).bfloat16(), torch.randn(M, N, device=DEV).bfloat16()
+    parts = torch.rand(M, 5, device=DEV) * K
+    scale = torch.rsqrt(parts.sum(-1, keepdim=True) / K + 1e-5)
+    ref = (x.float() @ w.float().t()) * scale + bias.float() + res.float()
+    for split in (0, 1):          # 1: the tensor-core kernel
+        y, ssq = ops.linear(x, w, bias=bias, residual=res, row_ssq=parts, norm_eps=1e-5, want_ssq=True, force_split=split)
+        assert rel_l2(y, ref) < BF16 and ssq.shape == (M, (N + 127) // 128)
+        want = torch.nn.functional.pad(y.float() ** 2, (0, -N % 128)).view(M, -1, 128).sum(-1)
+        assert bool(((ssq - want).abs() <= 128 * 2.0 ** -24 * want + 1e-30).all())
+    y = ops.linear(x, w, out_dtype=torch.float32, activation="relu2")
+    assert rel_l2(y, torch.relu(x.float() @ w.float().t()) ** 2) < 1e-5
+
+
+@pytest.mark.parametrize("M", [257, 2049, 2304, 4100])
+def test_prompt_gemm_bands(M):
+    """Token tiles that do not fill a band, and a last one that is nearly empty."""
+    w, x = (torch.randn(1160, 192, device=DEV) / 14).bfloat16(), torch.randn(M, 192, device=DEV).bfloat16()
+    assert rel_l2(ops.linear(x, w), x.float() @ w.float().t()) < BF16
+
+
+@pytest.mark.parametrize("R,V", [(1, 128256), (1, 4097), (7, 32002), (33, 40000), (300, 1000)])
+def test_largest_logit_over_a_cluster(R, V):
+    from eredu_b200.ops.sampling import SamplingParams, pack_rows
+
+    logits = torch.randn(R, V, device=DEV).round(decimals=1)           # many equal ones: the smallest token wins
+    rows = torch.from_numpy(pack_rows([SamplingParams(temperature=0.0)] * R, [1] * R, hist_lens=[0] * R, stream_ids=[0] * R).view("u1").copy()).view(R, -1).to(DEV)
+    allow = torch.rand(V, device=DEV) < 0.5
+    mask = ops.pack_allow_mask(allow)
+    for a, m in ((None, torch.ones_like(allow)), (mask[None], allow)):
+        want = logits.masked_fill(~m, float("-inf"))
+        want = (want == want.amax(-1, keepdim=True)).int().argmax(-1)
+        probs = torch.full((R, V), 7.0, device=DEV)
+        got = ops.sample(logits.clone(), rows, allow=a, probs=probs, all_greedy=True)
+        assert torch.equal(got.long(), want) and torch.equal(probs.argmax(-1), want) and bool((probs.sum(-1) == 1).all())
+    logits[0, V - 1] = 100.0
+    assert int(ops.sample(logits, rows, all_greedy=True)[0]) == V - 1
