@@ -327,6 +327,8 @@ class CausalLM:
             normed, _ = ops.rmsnorm(h, lw.ffn_norm, cfg.rms_norm_eps, weight_offset=cfg.norm_weight_offset)
             if self.observer is not None:
                 return lw.moe.observed_call(normed, h, self.observer), None
+            if next_folded and h.shape[0] <= self.FUSED_NORM_MAX_TOKENS:
+                return lw.moe.with_ssq(normed, h)
             return lw.moe(normed, residual=h), None
         inter = (lw.qlin["gate_up"].out_features if "gate_up" in lw.qlin else lw.w_gate_up.shape[0]) // 2
         act = self._normed_linear(h, ssq, lw.fold_ffn, lw.ffn_norm, lw.w_gate_up, lw, "gate_up", gated_inter=inter)

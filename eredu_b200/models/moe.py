@@ -122,7 +122,14 @@ class MoEBlock:
         out = combined + (residual.float() if residual is not None else 0.0)
         return out.to(x.dtype)
 
-    def __call__(self, x, residual=None):
+    def with_ssq(self, x, residual):
+        """residual + MoE(x) and, where the combining kernel of a single rank writes it, the partial sums of squares of its rows (else
+        None), for a norm folded into the next layer's projection."""
+        fused = x.is_cuda and x.dtype == torch.bfloat16 and self.ep_size == 1 and getattr(self, "expert_cache", None) is None
+        out = self(x, residual, want_ssq=fused)
+        return out if fused else (out, None)
+
+    def __call__(self, x, residual=None, want_ssq=False):
         """x: normalised hidden states [T, H]; returns residual + MoE(x)."""
         self.stats["calls"] += 1
         a2a = getattr(self, "ep_a2a", None)
@@ -153,7 +160,7 @@ class MoEBlock:
         if self.ep_size == 1:
             return moe_ops.experts_forward(x, ids, w, self.w_gate_up, self.w_down, self.e0, residual=residual,
                                            extra=extra, limit=self.cfg.swiglu_limit, plan=plan, xp=xp, gu_bias=self.gu_bias,
-                                           down_bias=self.down_bias, act=self.act)
+                                           down_bias=self.down_bias, act=self.act, want_ssq=want_ssq)
         # shared experts are replicated: add them on one rank only so that the group sum counts them once
         own_extra = extra if self.e0 == 0 else None
         comm = getattr(self.ep_ops, "fused_comm", lambda tokens, hidden: None)(x.shape[0], x.shape[1]) if x.is_cuda else None

@@ -16,6 +16,7 @@ native.register("eredu_moe_route", I, [P, I, P, P, P, I, I, I, I, I, native.F, I
 native.register("eredu_moe_plan", I, [P, I, I, I, I, I, P, P, P, P, I, P, P])
 native.register("eredu_moe_gather", I, [P, P, P, P, I, I, P])
 native.register("eredu_moe_combine", I, [P, P, P, P, P, P, I, I, I, P])
+native.register("eredu_moe_combine_ssq", I, [P, P, P, P, P, P, P, I, I, I, P])
 native.register("eredu_moe_route_plan_gather", I, [P, I, P, P, P, I, I, I, I, I, native.F, I, I, I, I, I, P, P, P, P, I, P, P, P, I, P])
 native.register("eredu_gemm_simt_grouped", I, [P, P, P, P, I, P, I, I, I, I, I, I, I, P])
 native.register("eredu_moe_combine_ar", I, [P, P, P, P, P, P, I, I, I, P, P, P])
@@ -248,12 +249,14 @@ def expert_rows(x, ids, w_gate_up, w_down, e0=0, limit=0.0, act="swiglu", plan=N
 
 
 def experts_forward(x, ids, weights, w_gate_up, w_down, e0=0, residual=None, extra=None, limit=0.0, rows_cap=None,
-                    comm=None, plan=None, xp=None, gu_bias=None, down_bias=None, act="swiglu", rows_only=False):
+                    comm=None, plan=None, xp=None, gu_bias=None, down_bias=None, act="swiglu", rows_only=False,
+                    want_ssq=False):
     """Local-expert MoE computation. x: [T, H] bf16; ids / weights: [T, k]; w_gate_up: [E_local, 2I, H];
     w_down: [E_local, H, I]. Returns residual + extra + sum over local routes (bf16 [T, H]). With ``comm`` (a peer
     communication context of the expert group) the combine kernel also sums the partial outputs of all ranks:
     ``extra`` is then counted once per rank that passes it, ``residual`` once in total. ``rows_only`` (CUDA, with a
-    ``plan`` and permuted rows ``xp``): stop after the two grouped GEMMs and return the rows in plan order."""
+    ``plan`` and permuted rows ``xp``): stop after the two grouped GEMMs and return the rows in plan order. ``want_ssq`` (CUDA bf16,
+    without ``comm``): also return partial sums of squares of the output rows, fp32 [T, parts]."""
     if not x.is_cuda:
         out = experts_ref(x, ids, weights, w_gate_up, w_down, e0, limit, gu_bias, down_bias, act)
         if residual is not None:
@@ -306,6 +309,12 @@ def experts_forward(x, ids, weights, w_gate_up, w_down, e0=0, residual=None, ext
                                           T, k, H, comm, ptr(st), stream_ptr(dev))
         check(code, "eredu_moe_combine_ar")
         return out
+    if want_ssq:
+        ssq = torch.empty((T, (H + 1023) // 1024), dtype=torch.float32, device=dev)
+        code = lib().eredu_moe_combine_ssq(ptr(y), ptr(plan.route_pos), ptr(weights), ptr(residual), ptr(extra), ptr(out), ptr(ssq), T, k,
+                                           H, stream_ptr(dev))
+        check(code, "eredu_moe_combine_ssq")
+        return out, ssq
     code = lib().eredu_moe_combine(ptr(y), ptr(plan.route_pos), ptr(weights), ptr(residual), ptr(extra), ptr(out), T, k,
                                    H, stream_ptr(dev))
     check(code, "eredu_moe_combine")

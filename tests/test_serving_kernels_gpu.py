@@ -166,3 +166,32 @@ def test_largest_logit_over_a_cluster(R, V):
         assert torch.equal(got.long(), want) and torch.equal(probs.argmax(-1), want) and bool((probs.sum(-1) == 1).all())
     logits[0, V - 1] = 100.0
     assert int(ops.sample(logits, rows, all_greedy=True)[0]) == V - 1
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 8, 2048), (3, 1, 1000), (64, 6, 4104), (2, 32, 64)])
+def test_weighted_expert_rows(T, k, H):
+    """Slots that do not fill a batch, columns that do not fill a CTA, routes of other ranks; sums of squares of what is stored."""
+    rows, w = torch.randn(T * k, H, device=DEV).bfloat16(), torch.rand(T, k, device=DEV)
+    res, extra = torch.randn(T, H, device=DEV).bfloat16(), torch.randn(T, H, device=DEV).bfloat16()
+    pos = torch.randperm(T * k, device=DEV).int()
+    if k > 1:
+        pos[1::5] = -1
+    out, ssq = torch.empty_like(res), torch.empty(T, (H + 1023) // 1024, device=DEV)
+    code = moe_ops.lib().eredu_moe_combine_ssq(*map(moe_ops.ptr, (rows, pos, w, res, extra, out, ssq)), T, k, H, moe_ops.stream_ptr(out.device))
+    assert code == 0
+    ref = res.float() + extra.float() + moe_ops.RoutedRows(rows, pos, w).summed()
+    assert rel_l2(out, ref) < BF16
+    assert torch.allclose(ssq.sum(-1), out.float().square().sum(-1), rtol=H * 2.0 ** -24, atol=0)
+
+
+@pytest.mark.parametrize("E,e0,e1,routes,k", [(128, 0, 128, 8192, 8), (8, 2, 6, 4096, 2), (512, 0, 512, 5000, 10), (60, 0, 30, 33, 3), (1, 0, 1, 40, 1)])
+def test_expert_plan_keeps_the_order_of_the_routes(E, e0, e1, routes, k):
+    ids = torch.randint(0, E, (routes // k, k), device=DEV, dtype=torch.int32)
+    plan = moe_ops.ExpertPlan(ids, k, e0, e1, 64, ids.numel())
+    flat = ids.flatten().cpu()
+    order = [r for e in range(e0, e1) for r in (flat == e).nonzero().flatten().tolist()]
+    want = torch.full((flat.numel(),), -1, dtype=torch.int32)
+    want[order] = torch.arange(len(order), dtype=torch.int32)
+    assert torch.equal(plan.route_pos.cpu(), want)
+    assert torch.equal(plan.row_token[:len(order)].cpu(), torch.tensor(order, dtype=torch.int32) // k)
+    assert plan.seg.tolist() == [int(((flat >= e0) & (flat < e0 + i)).sum()) for i in range(e1 - e0 + 1)]
