@@ -23,8 +23,15 @@ from .native import check, lib, ptr, status_word, stream_ptr
 PAGE = 16
 
 
+_sms: dict = {}
+
+
 def _sm_count(device) -> int:
-    return torch.cuda.get_device_properties(device).multi_processor_count
+    """SMs of a device, asked once (the property call costs as much as a launch)."""
+    n = _sms.get(device)
+    if n is None:
+        n = _sms[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return n
 
 
 # ------------------------------------------------------------------------------------------ linear

@@ -90,6 +90,8 @@ def ptr(t: torch.Tensor | None):
 
 
 def stream_ptr(device=None) -> int:
+    if isinstance(device, torch.device) and device.index is not None:
+        return torch._C._cuda_getCurrentRawStream(device.index)      # without a Stream object around it
     return torch.cuda.current_stream(device).cuda_stream
 
 
