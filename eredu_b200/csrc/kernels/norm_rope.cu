@@ -28,11 +28,18 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const __nv_bfloat16* _
   __shared__ float red[32];
   pdl_launch_early();
   trace_mark(kTraceRmsNorm, kTraceStart);
+  const size_t row = blockIdx.x;
+  const int nch = H >> 3;
+  // THREADS = 1024 (a thread has one piece of the row): weights are on their way before the dependency wait, like those of the GEMMs
+  constexpr bool kAhead = THREADS == 1024;
+  float4 wa[2] = {};
+  if (kAhead && static_cast<int>(threadIdx.x) < nch) {
+    wa[0] = reinterpret_cast<const float4*>(w)[2 * threadIdx.x];
+    wa[1] = reinterpret_cast<const float4*>(w)[2 * threadIdx.x + 1];
+  }
   pdl_wait();
   trace_mark(kTraceRmsNorm, kTraceAfterWait);
   pdl_launch_dependents();
-  const size_t row = blockIdx.x;
-  const int nch = H >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
   const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + row * H) : nullptr;
   float vals[MAXCH][8];
@@ -84,8 +91,8 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const __nv_bfloat16* _
   for (int i = 0; i < MAXCH; ++i) {
     const int c = threadIdx.x + i * THREADS;
     if (c < nch) {
-      const float4 w0 = reinterpret_cast<const float4*>(w)[2 * c];
-      const float4 w1 = reinterpret_cast<const float4*>(w)[2 * c + 1];
+      const float4 w0 = kAhead ? wa[0] : reinterpret_cast<const float4*>(w)[2 * c];
+      const float4 w1 = kAhead ? wa[1] : reinterpret_cast<const float4*>(w)[2 * c + 1];
       uint4 o;
       o.x = pack_bf16x2(vals[i][0] * inv * (w0.x + w_off), vals[i][1] * inv * (w0.y + w_off));
       o.y = pack_bf16x2(vals[i][2] * inv * (w0.z + w_off), vals[i][3] * inv * (w0.w + w_off));
@@ -423,7 +430,10 @@ extern "C" int eredu_rmsnorm(const void* x, const void* residual, const float* w
   auto Y = static_cast<__nv_bfloat16*>(y);
   auto Ho = static_cast<__nv_bfloat16*>(h_out);
   const int nch = H / 8;
-  if (nch <= 128) launch_pdl(rmsnorm_kernel<128, 1>, dim3(M), dim3(128), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
+  // few wide rows: a row over 1024 threads, whose latency is what a decode step waits for (one row of 8192 with four pieces a thread and
+  // the weights behind the sum: 5.8 us)
+  if (M <= 64 && nch > 256 && nch <= 1024) launch_pdl(rmsnorm_kernel<1024, 1>, dim3(M), dim3(1024), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
+  else if (nch <= 128) launch_pdl(rmsnorm_kernel<128, 1>, dim3(M), dim3(128), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
   else if (nch <= 256) launch_pdl(rmsnorm_kernel<256, 1>, dim3(M), dim3(256), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
   else if (nch <= 512) launch_pdl(rmsnorm_kernel<256, 2>, dim3(M), dim3(256), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
   else if (nch <= 1024) launch_pdl(rmsnorm_kernel<256, 4>, dim3(M), dim3(256), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
