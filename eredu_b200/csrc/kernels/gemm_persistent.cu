@@ -2,7 +2,7 @@
 // epilogues as the one-tile-per-CTA kernel (RMSNorm row scale, bias, residual, SwiGLU, sums of squares for the
 // next norm), built so that the tensor cores never wait for an epilogue:
 //
-//   * one CTA per SM walks a list of [128 weight rows x 256 tokens] tiles (swap-AB: the weight tile is the MMA M
+//   * one CTA per SM walks a list of [128 weight rows x up to 256 tokens] tiles (swap-AB: the weight tile is the MMA M
 //     operand, the token tile the MMA N operand);
 //   * the fp32 accumulator is double-buffered in TMEM (2 x 256 columns): while the epilogue warps drain tile i,
 //     the MMA warp already accumulates tile i+1;
@@ -17,6 +17,8 @@
 // (eredu-architectures/src/llama.rs:270-286,418-431; safemlx/src/ops/arithmetic.rs matmul).
 #include "gemm_persistent.h"
 
+#include <algorithm>
+
 #include "../common/elem.cuh"
 #include "../common/launch.h"
 #include "../common/launch_count.h"
@@ -29,16 +31,22 @@ namespace eredu {
 namespace {
 
 constexpr int kTN = 256;                         // tokens per tile (MMA N)
-constexpr int kStages = 4;
 constexpr int kATile = 128 * 64 * 2;             // 16 KB: 128 weight rows x 64 k
 constexpr int kBTile = kTN * 64 * 2;             // 32 KB: 256 tokens x 64 k
-constexpr int kStageBytes = kATile + kBTile;     // 48 KB
+constexpr int kTileFixed = 268;                  // of a tile's time, in token rows
 constexpr int kBand = 8;                         // token tiles that vary fastest
-constexpr int kBoxRows = 64;                     // grouped form: token rows of one copy
-constexpr int kBoxBytes = kBoxRows * 64 * 2;
+// Stages of the ring. BOX: grouped form, token rows of one copy - 64, or 16 for the items of a decode step (at most 16 rows): such a step
+// streams the weights of nearly all experts, and what counts are the bytes on their way, 160 KB an SM with ten small stages.
+template <int BOX>
+struct Ring {
+  static constexpr int kBoxBytes = BOX * 64 * 2;
+  static constexpr int kStageBytes = kATile + (BOX == 16 ? kBoxBytes : kBTile);    // 18 or 48 KB
+  static constexpr int kStages = BOX == 16 ? 10 : 4;
+};
 constexpr int kStagingBytes = 16 * 1024;
 constexpr int kCtrlBytes = 1024;
-constexpr int kSmemBytes = 1024 + kCtrlBytes + kStages * kStageBytes + kStagingBytes;
+template <int BOX>
+constexpr int kSmemBytes = 1024 + kCtrlBytes + Ring<BOX>::kStages * Ring<BOX>::kStageBytes + kStagingBytes;
 
 struct PGemmParams {
   void* y;
@@ -57,6 +65,7 @@ struct PGemmParams {
   float act_a, act_b;  // xIELU
   int act;  // plain tiles: 2 = squared ReLU before the residual, 4 = xIELU; dual tiles: 0 = silu(g) * u, 3 = relu(g) * u
   int n_tiles, m_tiles;
+  int tn;  // token rows of a tile: 256, or fewer where that saves a round of tiles
   // grouped form: m_tiles work items, used ones first (the rest have no rows); the expert's weights start at row expert * w_rows_per_expert
   const int4* work;
   int w_rows_per_expert;
@@ -89,17 +98,18 @@ __device__ __forceinline__ bool tile_at(const PGemmParams& p, int t, PTile& o) {
     o.m_cnt = min(item.z, kTN);
     return item.z > 0;
   }
-  o.m_base = tile_m * kTN;
-  o.m_cnt = min(kTN, p.M - o.m_base);
+  o.m_base = tile_m * p.tn;
+  o.m_cnt = min(p.tn, p.M - o.m_base);
   return true;
 }
 
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
-template <bool DUAL, bool GROUPED>
+template <bool DUAL, bool GROUPED, int BOX>
 __global__ void __launch_bounds__(192, 1)
 gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, PGemmParams p) {
+  constexpr int kStages = Ring<BOX>::kStages, kStageBytes = Ring<BOX>::kStageBytes, kBoxBytes = Ring<BOX>::kBoxBytes;
   pdl_launch_early();
   trace_mark(kTraceGemmPersistent, kTraceStart);
   extern __shared__ uint8_t smem_raw[];
@@ -150,7 +160,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      const uint64_t pol_w = l2_policy_evict_last();   // both operands are re-read by other CTAs from L2
+      // both operands are re-read by other CTAs from L2; the weights of a decode step are not
+      const uint64_t pol_w = BOX == 16 ? l2_policy_evict_first() : l2_policy_evict_last();
       const uint64_t pol_x = l2_policy_evict_last();
       int it = 0, issued = 0;
       bool ok = true;
@@ -164,8 +175,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           ok = mbar_wait(&empty_bar[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
           if (!ok) break;
           uint8_t* a = stages + s * kStageBytes;
-          const int boxes = (tl.m_cnt + kBoxRows - 1) / kBoxRows;
-          mbar_arrive_expect_tx(&full_bar[s], GROUPED ? kATile + boxes * kBoxBytes : kStageBytes);
+          const int boxes = (tl.m_cnt + BOX - 1) / BOX;
+          mbar_arrive_expect_tx(&full_bar[s], kATile + (GROUPED ? boxes * kBoxBytes : p.tn * 128));
           if (DUAL) {
             tma_load_2d_hint(a, &tmW, kb * 64, w_row0, &full_bar[s], pol_w);
             tma_load_2d_hint(a + kATile / 2, &tmW, kb * 64, p.dual_row_offset + w_row0, &full_bar[s], pol_w);
@@ -174,7 +185,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           }
           if (GROUPED) {
             for (int i = 0; i < boxes; ++i)
-              tma_load_2d_hint(a + kATile + i * kBoxBytes, &tmX, kb * 64, m_base + i * kBoxRows, &full_bar[s], pol_x);
+              tma_load_2d_hint(a + kATile + i * kBoxBytes, &tmX, kb * 64, m_base + i * BOX, &full_bar[s], pol_x);
           } else {
             tma_load_2d_hint(a + kATile, &tmX, kb * 64, m_base, &full_bar[s], pol_x);
           }
@@ -188,7 +199,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      uint32_t idesc = umma_idesc_bf16(128, kTN);
+      uint32_t idesc = 0;
       int it = 0, lt = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++lt) {
@@ -359,6 +370,24 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
 
 }  // namespace
 
+// Token rows of a tile. A CTA walks ceil(tiles / SMs) tiles, and with 256 rows the last of these walks is often nearly empty (1250 x 4096:
+// 160 tiles on 148 SMs). A round of smaller tiles is shorter, but by much less than its rows: weights have to be fetched and read all
+// the same. Rounds of 256, 160, 128 and 96 rows at K = 4096 took 29.4, 24.4, 22.6 and 21.5 us, which is kTileFixed rows and the tile's own;
+// 1250 x 4096 x 14336 165 -> 157 us, 300 x 2 x 28672 x 8192 368 -> 317.
+static int pick_token_tile(int M, int n_tiles, int sms) {
+  int best = kTN;
+  long cost = -1;
+  for (int tn = kTN; tn >= 96; tn -= 16) {
+    const long tiles = static_cast<long>(n_tiles) * ((M + tn - 1) / tn);
+    const long c = (tiles + sms - 1) / sms * (std::min(tn, M) + kTileFixed);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = tn;
+    }
+  }
+  return best;
+}
+
 int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* residual, const void* bias, int M, int N,
                            int K, int ldx, int ldw, int ldy, int ldr, int w_rows, int dual, int dual_row_offset,
                            int sm_count, int* status, const float* ssq_in, int ssq_parts, float norm_eps, int norm_dim,
@@ -370,7 +399,10 @@ int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* re
   CUtensorMap tmW, tmX;
   int r = make_tma_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_rows, K, ldw, dual ? 64 : 128, 64);
   if (r != 0) return -100 + r;
-  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, ldx, kTN, 64);
+  const int sms = sm_count > 0 ? sm_count : 148;
+  const int n_tiles = dual ? (N + 63) / 64 : (N + 127) / 128;
+  const int tn = pick_token_tile(M, n_tiles, sms);
+  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, ldx, tn, 64);
   if (r != 0) return -200 + r;
   PGemmParams p = {};
   p.y = Y;
@@ -392,10 +424,10 @@ int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* re
   p.act_a = act_a;
   p.act_b = act_b;
   p.out_fp32 = out_fp32;
-  p.n_tiles = dual ? (N + 63) / 64 : (N + 127) / 128;
-  p.m_tiles = (M + kTN - 1) / kTN;
+  p.n_tiles = n_tiles;
+  p.tn = tn;
+  p.m_tiles = (M + tn - 1) / tn;
   const int total = p.n_tiles * p.m_tiles;
-  const int sms = sm_count > 0 ? sm_count : 148;
   // equal rounds for every CTA where possible: ceil(total / rounds) CTAs, never more than the SM count
   const int rounds = (total + sms - 1) / sms;
   const int grid = (total + rounds - 1) / rounds;
@@ -403,25 +435,42 @@ int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* re
     static bool configured_plain = false, configured_dual = false;
     bool& configured = dual ? configured_dual : configured_plain;
     if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<64>);
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    return launch_pdl(kern, dim3(grid), dim3(192), kSmemBytes, stream, tmW, tmX, p);
+    return launch_pdl(kern, dim3(grid), dim3(192), kSmemBytes<64>, stream, tmW, tmX, p);
   };
-  const cudaError_t e = dual ? launch(gemm_persistent_kernel<true, false>) : launch(gemm_persistent_kernel<false, false>);
+  const cudaError_t e = dual ? launch(gemm_persistent_kernel<true, false, 64>) : launch(gemm_persistent_kernel<false, false, 64>);
   eredu_count_launches(1);
   return static_cast<int>(e);
 }
 
-int launch_gemm_persistent_grouped(const void* X, const void* W, void* Y, const int* work, int n_work, int rows_cap, int N, int K, int ldx,
-                                   int ldw, int ldy, int w_rows_total, int w_rows_per_expert, int dual, int sm_count, int* status,
+template <bool DUAL, int BOX>
+static cudaError_t launch_grouped(const CUtensorMap& tmW, const CUtensorMap& tmX, const PGemmParams& p, int sms, cudaStream_t stream) {
+  static bool configured[64] = {};  // the attribute is a per-device setting
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(gemm_persistent_kernel<DUAL, true, BOX>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<BOX>);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  const int total = p.n_tiles * p.m_tiles;
+  return launch_pdl(gemm_persistent_kernel<DUAL, true, BOX>, dim3(total < sms ? total : sms), dim3(192), kSmemBytes<BOX>, stream, tmW, tmX, p);
+}
+
+int launch_gemm_persistent_grouped(const void* X, const void* W, void* Y, const int* work, int n_work, int item_rows, int rows_cap, int N, int K,
+                                   int ldx, int ldw, int ldy, int w_rows_total, int w_rows_per_expert, int dual, int sm_count, int* status,
                                    cudaStream_t stream) {
   if (N % 8 != 0 || ldy % 8 != 0 || (reinterpret_cast<uintptr_t>(Y) & 15) != 0 || (dual && N % 64 != 0)) return kPersistentUnsupported;
+  const int sms = sm_count > 0 ? sm_count : 148, box = item_rows <= 16 ? 16 : 64;
   CUtensorMap tmW, tmX;
   int r = make_tma_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_rows_total, K, ldw, dual ? 64 : 128, 64);
   if (r != 0) return -100 + r;
-  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_cap, K, ldx, kBoxRows, 64);
+  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_cap, K, ldx, box, 64);
   if (r != 0) return -200 + r;
   PGemmParams p = {};
   p.y = Y;
@@ -435,18 +484,9 @@ int launch_gemm_persistent_grouped(const void* X, const void* W, void* Y, const 
   p.m_tiles = n_work;
   p.work = reinterpret_cast<const int4*>(work);
   p.w_rows_per_expert = w_rows_per_expert;
-  const int sms = sm_count > 0 ? sm_count : 148;
-  const int total = p.n_tiles * n_work;
-  static bool configured[2] = {};
-  if (!configured[dual ? 1 : 0]) {
-    const cudaError_t e = dual ? cudaFuncSetAttribute(gemm_persistent_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes)
-                               : cudaFuncSetAttribute(gemm_persistent_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured[dual ? 1 : 0] = true;
-  }
-  const dim3 grid(total < sms ? total : sms);
-  const cudaError_t e = dual ? launch_pdl(gemm_persistent_kernel<true, true>, grid, dim3(192), kSmemBytes, stream, tmW, tmX, p)
-                             : launch_pdl(gemm_persistent_kernel<false, true>, grid, dim3(192), kSmemBytes, stream, tmW, tmX, p);
+  cudaError_t e;
+  if (box == 16) e = dual ? launch_grouped<true, 16>(tmW, tmX, p, sms, stream) : launch_grouped<false, 16>(tmW, tmX, p, sms, stream);
+  else e = dual ? launch_grouped<true, 64>(tmW, tmX, p, sms, stream) : launch_grouped<false, 64>(tmW, tmX, p, sms, stream);
   eredu_count_launches(1);
   return static_cast<int>(e);
 }

@@ -791,16 +791,20 @@ static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K,
 }
 
 // Number of K splits the launcher would use (exposed for tests and tuning).
-extern "C" int eredu_gemm_pick_split(int M, int N, int K, int sm_count) {
-  const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+static int pick_split(int M, int N, int K, int tn, int ctas_per_sm, int sm_count) {
   if (tn > 64) return 1;
   const int tiles = ((N + 127) / 128) * ((M + tn - 1) / tn);
   const int kblocks = (K + 63) / 64;
   int s = 1;
-  // Split while the grid still fits two CTAs per SM: besides streaming the weights in parallel, a split CTA
+  // Split while the grid still fits the CTAs an SM takes: besides streaming the weights in parallel, a split CTA
   // finishes only every s-th token column, and the serial per-column epilogue is what a small GEMM pays for.
-  while (s < 8 && tiles * s * 2 <= 2 * sm_count && kblocks / (s * 2) >= 2) s *= 2;
+  while (s < 8 && tiles * s * 2 <= ctas_per_sm * sm_count && kblocks / (s * 2) >= 2) s *= 2;
   return s;
+}
+
+extern "C" int eredu_gemm_pick_split(int M, int N, int K, int sm_count) {
+  const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  return pick_split(M, N, K, tn, 2, sm_count);
 }
 
 // Y = X W^T (+bias) (+residual), or with dual != 0: Y = silu(X Wg^T) * (X Wu^T) where Wg = W[0:N],
@@ -869,7 +873,9 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   if (r != 0) return -200 + r;
   const int n_tiles = (N + 127) / 128;
   const int m_tiles = (M + tn - 1) / tn;
-  int nsplit = force_split > 0 ? force_split : eredu_gemm_pick_split(M, N, K, sm_count > 0 ? sm_count : 148);
+  // The ring of a gated tile of 64 tokens leaves an SM room for one CTA: 2 x 14336 x 4096 split twice was 224 CTAs in two rounds. The split
+  // goes by the tile in use, also where a router's is smaller than its tokens say (1024 x 128 x 2048 unsplit: 23 us on 16 SMs).
+  int nsplit = force_split > 0 ? force_split : pick_split(M, N, K, tn, tn == 64 && dual ? 1 : 2, sm_count > 0 ? sm_count : 148);
   const int kblocks = (K + 63) / 64;
   while (nsplit > 1 && (kblocks + nsplit - 1) / nsplit * (nsplit - 1) >= kblocks) nsplit >>= 1;  // no empty split
   p.staged = staged_epilogue_ok(Y, residual, N, ldy, ldr, out_fp32) && tn >= 64 && nsplit == 1;
@@ -987,7 +993,7 @@ extern "C" int eredu_gemm_bf16_grouped(const void* X, const void* W, void* Y, co
   if (n_work <= 0 || N <= 0 || K <= 0) return 0;
   if (tile == 256) {
     if (bias != nullptr || act != 0 || act_limit > 0.f) return -1;
-    return launch_gemm_persistent_grouped(X, W, Y, work, n_work, rows_cap, N, K, ldx, ldw, ldy, w_rows_total, w_rows_per_expert, dual, sm_count,
+    return launch_gemm_persistent_grouped(X, W, Y, work, n_work, tile, rows_cap, N, K, ldx, ldw, ldy, w_rows_total, w_rows_per_expert, dual, sm_count,
                                           status, stream);
   }
   CUtensorMap tmW, tmX;
@@ -1013,6 +1019,15 @@ extern "C" int eredu_gemm_bf16_grouped(const void* X, const void* W, void* Y, co
   // An item holds at least one row and the used items come first: a step of few rows launches, and splits K for, no more items than it
   // has rows. One token on 8 of 128 experts (gate_up 2 x 768 x 2048): 20.4 us with 129 items of which 121 were empty and K unsplit.
   if (rows_cap < n_work) n_work = rows_cap;
+  // Items of at most 16 rows that give every SM two tiles or more: a step that reads most experts. The persistent form streams their weights
+  // without a start and an end of a CTA per tile: both GEMMs of 128 experts (768 x 2048), 8 tokens 101 -> 93 us, 64 tokens 194 -> 188; in a
+  // decode step of 32 sequences, behind and in front of other kernels, 12.5 us a layer (8275 -> 7877 for 32 of them).
+  if (tile == 16 && bias == nullptr && act == 0 && act_limit <= 0.f && force_split <= 0 &&
+      static_cast<long long>(n_work) * ((N + 127) / 128) >= 2LL * (sm_count > 0 ? sm_count : 148)) {
+    const int pr = launch_gemm_persistent_grouped(X, W, Y, work, n_work, tile, rows_cap, N, K, ldx, ldw, ldy, w_rows_total, w_rows_per_expert, dual,
+                                                  sm_count, status, stream);
+    if (pr != kPersistentUnsupported) return pr;
+  }
   const int n_tiles = (N + 127) / 128;
   const int kblocks = (K + 63) / 64;
   int nsplit = 1;

@@ -195,3 +195,34 @@ def test_expert_plan_keeps_the_order_of_the_routes(E, e0, e1, routes, k):
     assert torch.equal(plan.route_pos.cpu(), want)
     assert torch.equal(plan.row_token[:len(order)].cpu(), torch.tensor(order, dtype=torch.int32) // k)
     assert plan.seg.tolist() == [int(((flat >= e0) & (flat < e0 + i)).sum()) for i in range(e1 - e0 + 1)]
+
+
+@pytest.mark.parametrize("M", [1, 64, 65])
+@pytest.mark.parametrize("H", [2048, 2056, 4104, 8192])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_of_few_wide_rows(M, H, residual):
+    x, w = torch.randn(M, H, device=DEV).bfloat16(), torch.rand(H, device=DEV) + 0.5
+    r = torch.randn(M, H, device=DEV).bfloat16() if residual else None
+    y, h = ops.rmsnorm(x, w, 1e-5, residual=r, weight_offset=0.25)
+    yr, hr = ops.rmsnorm_ref(x, w, 1e-5, r, 0.25)
+    assert rel_l2(y, yr) < BF16 and (h is None if not residual else torch.equal(h, hr))
+
+
+@pytest.mark.parametrize("M,N,K", [(1024, 128, 512), (300, 96, 320), (700, 60, 2048)])
+def test_router_of_prompts(M, N, K):
+    """A narrow fp32 output over many tokens: token tiles of 64 with K split over a cluster."""
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    y = ops.linear(x, w, out_dtype=torch.float32)
+    assert rel_l2(y, x.float() @ w.float().t()) < 1e-5
+
+
+@pytest.mark.parametrize("M,N,K", [(130, 1096, 256), (400, 4736, 128), (1250, 4096, 192), (1900, 2048, 128)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_prompt_gemm_tiles_of_fewer_tokens(M, N, K, gated):
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = (torch.randn(2 * N if gated else N, K, device=DEV) / K ** 0.5).bfloat16()
+    y = x.float() @ w.float().t()
+    if gated:
+        assert rel_l2(ops.gated_linear(x, w, N), moe_ops.gated_act_ref(y[:, :N], y[:, N:])) < BF16
+    else:
+        assert rel_l2(ops.linear(x, w), y) < BF16
