@@ -296,7 +296,7 @@ class CausalLM:
                                              interleaved=cfg.rope_traditional, attn_factor=self.attn_factor,
                                              q_norm_w=lw.q_norm, k_norm_w=lw.k_norm, norm_eps=cfg.rms_norm_eps,
                                              norm_w_off=cfg.norm_weight_offset, splits=batch.splits, window=window,
-                                             sinks=lw.sinks, scratch=batch.scratch)
+                                             sinks=lw.sinks, scratch=batch.scratch, settled=True)
             return self._attn_out(lw, attn, gate, h, next_folded)
         q = ops.rope_kv(qkv, rope_pos, batch.slots, self.inv_freq, k_cache, v_cache, self.n_q_local,
                         self.n_kv_local, cfg.head_dim, rot=cfg.rotary_dim, interleaved=cfg.rope_traditional,

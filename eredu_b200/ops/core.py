@@ -667,12 +667,14 @@ def attention_decode(q, k_cache, v_cache, block_table, seq_lens, q_per_seq, scal
 def attention_decode_rope(qkv, k_cache, v_cache, block_table, seq_lens, q_per_seq, scale, positions, slots, inv_freq,
                           n_q, n_kv, head_dim, rot=None, interleaved=False, attn_factor=1.0, q_norm_w=None, k_norm_w=None,
                           norm_eps=1e-6, norm_w_off=0.0, splits=1, window=0, sinks=None, scratch=None, chunk=0, value_dim=None,
-                          norm_whole=False, value_norm=False, append=True):
+                          norm_whole=False, value_norm=False, append=True, settled=False):
     """Decode attention straight from the qkv projection output [B * q_per_seq, >= (n_q + 2 n_kv) * D]: per-head
     q/k norm, RoPE and the KV append run inside the attention kernel (one launch instead of two). CPU tensors and
     head sizes without a kernel compose the two reference operators.
     ``norm_whole`` / ``value_norm`` / ``append``: the preparation of :func:`qkv_prepare` (norms over whole projections, value
-    heads of width ``value_dim``, rows that hold queries only) instead of that of :func:`rope_kv`."""
+    heads of width ``value_dim``, rows that hold queries only) instead of that of :func:`rope_kv`.
+    ``settled``: the kernel enqueued just before this call writes ``qkv`` only, not the pages, ``block_table`` or ``seq_lens`` (the
+    projection of a decode step); these are then read ahead of the stream dependency on it."""
     value_dim = value_dim or head_dim
     if norm_whole or value_norm or not append or value_dim != head_dim or chunk:
         whole = (qkv.is_cuda and qkv.dtype == torch.bfloat16 and _tma_rows(qkv) and head_dim % 8 == 0 and value_dim % 8 == 0
@@ -704,7 +706,7 @@ def attention_decode_rope(qkv, k_cache, v_cache, block_table, seq_lens, q_per_se
                                         ptr(slots), ptr(inv_freq), ptr(q_norm_w), ptr(k_norm_w), B, q_per_seq,
                                         block_table.stride(0), n_q, n_kv, head_dim, value_dim,
                                         head_dim if rot is None else rot, 1 if interleaved else 0, splits, window, chunk,
-                                        int(norm_whole), int(value_norm), int(append), scale, attn_factor, norm_eps,
+                                        int(norm_whole), int(value_norm), int(append) | (2 if settled else 0), scale, attn_factor, norm_eps,
                                         norm_w_off, stream_ptr(qkv.device))
     check(code, "eredu_attn_decode_rope")
     return out

@@ -226,3 +226,38 @@ def test_prompt_gemm_tiles_of_fewer_tokens(M, N, K, gated):
         assert rel_l2(ops.gated_linear(x, w, N), moe_ops.gated_act_ref(y[:, :N], y[:, N:])) < BF16
     else:
         assert rel_l2(ops.linear(x, w), y) < BF16
+
+
+@pytest.mark.parametrize("D,n_q,n_kv,new,lens", [(128, 32, 8, 1, [2040]), (64, 8, 8, 1, [15, 16, 17, 1, 640]), (128, 64, 2, 5, [33, 700])])
+def test_decode_attention_ahead_of_its_projection(D, n_q, n_kv, new, lens):
+    """Steps of projection, attention and output projection without a synchronisation between them, each reading what the step before has
+    appended: pages fetched ahead of the projection give the same bits as pages fetched behind it."""
+    B, width, hidden, steps = len(lens), (n_q + 2 * n_kv) * D, 512, 6
+    pages = [(n + steps * new + 15) // 16 for n in lens]
+    bt = torch.zeros(B, max(pages), dtype=torch.int32, device=DEV)
+    ids, at = torch.randperm(sum(pages), device=DEV).int(), 0
+    for i, n in enumerate(pages):
+        bt[i, :n] = ids[at:at + n]
+        at += n
+    w = (torch.randn(width, hidden, device=DEV) / hidden ** 0.5).bfloat16()
+    wo = (torch.randn(hidden, n_q * D, device=DEV) / (n_q * D) ** 0.5).bfloat16()
+    start = [torch.randn(sum(pages), n_kv, 16, D, device=DEV).bfloat16() for _ in range(2)]
+    x0 = torch.randn(B * new, hidden, device=DEV).bfloat16()
+    inv = 1.0 / (10000.0 ** (torch.arange(0, D, 2, device=DEV).float() / D))
+    table, plan = bt.cpu().long(), []
+    for s in range(steps):
+        pos = torch.tensor([n + s * new + i for n in lens for i in range(new)])
+        rows = torch.arange(B).repeat_interleave(new)
+        plan.append((pos.int().to(DEV), (table[rows, pos // 16] * 16 + pos % 16).to(DEV), torch.tensor([n + (s + 1) * new for n in lens], dtype=torch.int32, device=DEV)))
+    results = []
+    for settled in (False, True):
+        kc, vc = start[0].clone(), start[1].clone()
+        torch.cuda.synchronize()
+        x, outs = x0, []
+        for pos, slots, seq in plan:
+            qkv = ops.linear(x, w)
+            a = ops.attention_decode_rope(qkv, kc, vc, bt, seq, new, D ** -0.5, pos, slots, inv, n_q, n_kv, D, splits=2, settled=settled)
+            x = ops.linear(a.view(B * new, -1), wo)
+            outs.append(x)
+        results.append((torch.stack(outs), kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
