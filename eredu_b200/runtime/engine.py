@@ -23,6 +23,7 @@ from .. import ops
 from ..models.llama import CausalLM, ForwardBatch
 from ..ops.sampling import ROW_DTYPE, SamplingParams, pack_rows
 from ..utils import nvtx
+from ..utils.capture import captured
 from .kv_cache import PAGE, PagedKVCache
 
 
@@ -654,7 +655,7 @@ class Engine:
                 for t, copy in saved_rec:
                     t.copy_(copy)
                 g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g):
+                with captured(g):
                     self._decode_body(st)
                 # capture does not execute: state is still the pre-step state
                 st["graph"] = g

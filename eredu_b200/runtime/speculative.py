@@ -21,6 +21,7 @@ import torch
 from .. import ops
 from ..models.llama import ForwardBatch
 from ..ops.sampling import ROW_DTYPE, SamplingParams, pack_rows
+from ..utils.capture import captured
 from .engine import Engine, Sequence
 from .kv_cache import PAGE
 
@@ -804,7 +805,7 @@ class GraphSpeculativeDecoder(SpeculativeDecoder):
                     torch.cuda.current_stream(dev).wait_stream(side)
                     torch.cuda.synchronize(dev)
                     g = torch.cuda.CUDAGraph()
-                    with torch.cuda.graph(g):
+                    with captured(g):
                         self._device_round(st)
                     st["graph"] = g
                 st["graph"].replay()
