@@ -431,7 +431,7 @@ extern "C" int eredu_rmsnorm(const void* x, const void* residual, const float* w
   auto Ho = static_cast<__nv_bfloat16*>(h_out);
   const int nch = H / 8;
   // few wide rows: a row over 1024 threads, whose latency is what a decode step waits for (one row of 8192 with four pieces a thread and
-  // the weights behind the sum: 5.8 us)
+  // the weights behind the sum: 5.8 us; 1.8 less in a decode step, 6470 -> 6354 us with 64 of them)
   if (M <= 64 && nch > 256 && nch <= 1024) launch_pdl(rmsnorm_kernel<1024, 1>, dim3(M), dim3(1024), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
   else if (nch <= 128) launch_pdl(rmsnorm_kernel<128, 1>, dim3(M), dim3(128), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
   else if (nch <= 256) launch_pdl(rmsnorm_kernel<256, 1>, dim3(M), dim3(256), 0, stream, X, R, w, Y, Ho, H, eps, w_off);
