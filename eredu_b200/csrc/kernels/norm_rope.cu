@@ -120,6 +120,15 @@ struct RopeParams {
   float norm_w_off;
 };
 
+// The arithmetic of the two kernels below, with the product that is rounded and the one that is fused written out: left to the compiler,
+// the two chose differently, and a number in 10^5 differed by a bf16 place between them.
+__device__ __forceinline__ float pair_squares(float a, float b) { return fmaf(a, a, __fmul_rn(b, b)); }
+__device__ __forceinline__ void rotate_pair(float& a, float& b, float cs, float sn) {
+  const float ra = fmaf(a, cs, -__fmul_rn(b, sn));
+  b = fmaf(b, cs, __fmul_rn(a, sn));
+  a = ra;
+}
+
 // grid (M, n_q + 2 n_kv), D/2 threads: thread i owns one rotation pair (or a pass-through pair).
 __global__ void rope_kv_kernel(RopeParams p) {
   __shared__ float red[8];
@@ -147,7 +156,7 @@ __global__ void rope_kv_kernel(RopeParams p) {
   float b = __bfloat162float(src[i1]);
   const float* nw = is_q ? p.q_norm_w : (is_k ? p.k_norm_w : nullptr);
   if (nw != nullptr) {
-    float ss = warp_sum(a * a + b * b);
+    float ss = warp_sum(pair_squares(a, b));
     if ((i & 31) == 0) red[i >> 5] = ss;
     __syncthreads();
     float t = 0.f;
@@ -162,10 +171,7 @@ __global__ void rope_kv_kernel(RopeParams p) {
     sincosf(static_cast<float>(p.positions[m]) * p.inv_freq[i], &sn, &cs);
     sn *= p.attn_factor;
     cs *= p.attn_factor;
-    const float ra = a * cs - b * sn;
-    const float rb = b * cs + a * sn;
-    a = ra;
-    b = rb;
+    rotate_pair(a, b, cs, sn);
   }
   if (is_q) {
     __nv_bfloat16* dst = p.q_out + (static_cast<size_t>(m) * p.n_q + head) * p.D;
@@ -187,7 +193,8 @@ __global__ void rope_kv_kernel(RopeParams p) {
 
 // The same with 16-byte accesses, for rows and widths that allow them: one CTA per token. The kernel above is bound by its grid - a
 // CTA of two warps per (token, head), each with its own sincosf and 2-byte accesses; here the angles of a token are evaluated once for
-// all heads, and a thread owns two 16-byte pieces that rotate into each other (16 elements). Bound by the bytes of one read and
+// all heads, and a thread owns two 16-byte pieces that rotate into each other (16 elements). Same bits as the kernel above: which of the
+// two runs hangs on alignment, and the routing of the experts behind it hangs on every bit. Bound by the bytes of one read and
 // one write. 2048 tokens of 48 heads of 128 (50 MB): 122 -> 10.3 us.
 constexpr int kRopeThreads = 128;
 constexpr int kRopeBatch = 4;   // pieces a thread has in flight: the 384 of a token with 48 heads of 128 go in one pass
@@ -252,10 +259,24 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kv_rows_kernel(RopeParams p
       unpack8(raw[b][1], c);
       const float* nw = is_q ? p.q_norm_w : (is_k ? p.k_norm_w : nullptr);
       if (p.q_norm_w != nullptr || p.k_norm_w != nullptr) {
-        float ss = 0.f;
+        // thread u has the pairs 8 u .. 8 u + 7. They are added up as the lanes above add theirs - pairs 16 apart, then 8, 4, 2, 1, then
+        // the halves of a head of 128: every exchange of the first two leaves a thread half of its sums
+        float sq[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss += a[j] * a[j] + c[j] * c[j];
-        for (int o = 1; o < (1 << upw_shift); o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        for (int j = 0; j < 8; ++j)
+          sq[j] = !p.interleaved && u < rc ? pair_squares(a[j], c[j]) : j < 4 ? pair_squares(a[2 * j], a[2 * j + 1]) : pair_squares(c[2 * j - 8], c[2 * j - 7]);
+        const bool up2 = (u & 2) != 0, up1 = (u & 1) != 0;
+        float s4[4], s2[2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s4[j] = (up2 ? sq[j + 4] : sq[j]) + __shfl_xor_sync(0xffffffffu, up2 ? sq[j] : sq[j + 4], 2);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) s2[j] = (up1 ? s4[j + 2] : s4[j]) + __shfl_xor_sync(0xffffffffu, up1 ? s4[j] : s4[j + 2], 1);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 2);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 1);
+        float ss = s2[0] + s2[1];
+        if (upw_shift == 3) ss += __shfl_xor_sync(0xffffffffu, ss, 4);
         if (nw != nullptr) {
           const float inv = rsqrtf(ss / static_cast<float>(p.D) + p.norm_eps);
 #pragma unroll
@@ -271,20 +292,14 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kv_rows_kernel(RopeParams p
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float c0 = s_cos[8 * u + j], s0 = s_sin[8 * u + j], c1 = s_cos[8 * u + 4 + j], s1 = s_sin[8 * u + 4 + j];
-              const float x0 = a[2 * j], y0 = a[2 * j + 1], x1 = c[2 * j], y1 = c[2 * j + 1];
-              a[2 * j] = x0 * c0 - y0 * s0;
-              a[2 * j + 1] = y0 * c0 + x0 * s0;
-              c[2 * j] = x1 * c1 - y1 * s1;
-              c[2 * j + 1] = y1 * c1 + x1 * s1;
+              rotate_pair(a[2 * j], a[2 * j + 1], c0, s0);
+              rotate_pair(c[2 * j], c[2 * j + 1], c1, s1);
             }
           }
         } else if (u < rc) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float cs = s_cos[8 * u + j], sn = s_sin[8 * u + j];
-            const float x = a[j], y = c[j];
-            a[j] = x * cs - y * sn;
-            c[j] = y * cs + x * sn;
+            rotate_pair(a[j], c[j], s_cos[8 * u + j], s_sin[8 * u + j]);
           }
         }
       }
@@ -470,7 +485,7 @@ extern "C" int eredu_rope_kv(const void* qkv, void* q_out, void* k_cache, void* 
   // 16-byte pieces: heads and rotated parts of whole pairs of pieces, rows and pages on 16-byte boundaries. Everything else (and
   // angles that do not fit the shared table) keeps the kernel with 2-byte accesses.
   const auto aligned = [](const void* t) { return (reinterpret_cast<uintptr_t>(t) & 15) == 0; };
-  if ((D == 32 || D == 64 || D == 128 || D == 256) && rot % 16 == 0 && ld % 8 == 0 && aligned(qkv) && aligned(q_out) && aligned(k_cache) &&
+  if ((D == 64 || D == 128) && rot % 16 == 0 && ld % 8 == 0 && aligned(qkv) && aligned(q_out) && aligned(k_cache) &&
       aligned(v_cache))
     launch_pdl(rope_kv_rows_kernel, dim3(M), dim3(kRopeThreads), 0, stream, p, __builtin_ctz(static_cast<unsigned>(D)) - 4);
   else

@@ -45,6 +45,26 @@ def test_rotation_and_append_rows(M, n_q, n_kv, D, rot, interleaved):
     assert torch.equal(vc, vr)
 
 
+@pytest.mark.parametrize("norms", ["none", "queries", "both"])
+@pytest.mark.parametrize("D,rot,interleaved", [(128, 128, False), (128, 128, True), (64, 64, False), (64, 48, True), (128, 16, False)])
+def test_rotation_gives_the_same_bits_on_either_kernel(D, rot, interleaved, norms):
+    """Whole 16-byte pieces, and the same numbers one element further on in rows of odd pitch, which the kernel of single elements takes."""
+    M, n_q, n_kv = 700, 12, 2
+    width = (n_q + 2 * n_kv) * D
+    odd = torch.randn(M, width + 1, device=DEV).bfloat16()
+    pos = torch.randint(0, 9000, (M,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(48 * 16, device=DEV)[:M].long()
+    inv = 1.0 / (10000.0 ** (torch.arange(0, rot, 2, device=DEV).float() / rot))
+    qn = torch.rand(D, device=DEV) + 0.5 if norms != "none" else None
+    kn = torch.rand(D, device=DEV) + 0.5 if norms == "both" else None
+    outs = []
+    for qkv in (odd[:, 1:].contiguous(), odd[:, 1:]):
+        kc, vc = (torch.zeros(48, n_kv, 16, D, device=DEV).bfloat16() for _ in range(2))
+        outs.append((ops.rope_kv(qkv, pos, slots, inv, kc, vc, n_q, n_kv, D, rot=rot, interleaved=interleaved, q_norm_w=qn, k_norm_w=kn,
+                                 attn_factor=1.25), kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("N,K,group", [(16, 64, 64), (650, 320, 32), (8, 1024, 128), (130, 192, 96), (256, 448, 16)])
 def test_decoded_weights(N, K, group):
     """K blocks that are no multiple of a warp's four, rows that are no whole tiles, group sizes below, at and above a block."""
