@@ -821,8 +821,17 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   const int act = dual ? ((flags & 4) ? 3 : 0) : (flags & 2) ? 2 : (flags & 8) ? 4 : 0;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-  // a narrow output over many tokens (a router) fills the machine with small token tiles instead
-  if (tn == 256 && out_fp32 && ((N + 127) / 128) * ((M + 255) / 256) * 2 <= sm_count) tn = 64;
+  // A narrow output over many tokens (a router) fills the machine with small token tiles instead. K is not split: experts that score alike
+  // change places with the order of a sum, and this one is the same for every number of tokens. Its products hang on one another (0.29 us
+  // per 64 of K, whatever the tile); what smaller tiles save is the serial epilogue of their columns, as long as one round of CTAs holds
+  // them: 1024 x 128 x 2048 19.9 us with 64 tokens, 13.5 with 16; 4096 tokens 20.2, 17.3 with 32. Few rows of weights that all CTAs fetch
+  // at once stand a quarter of the CTAs (1024 x 8 x 2048: 15.5 to 24.8 us with 16 tokens, by where the rows lie, 16.0 with 32).
+  const bool narrow = tn == 256 && out_fp32 && ((N + 127) / 128) * ((M + 255) / 256) * 2 <= sm_count;
+  if (narrow) {
+    const int ctas = N > 16 ? sm_count : sm_count / 4;
+    tn = 64;
+    while (tn > 16 && ((N + 127) / 128) * ((M + tn / 2 - 1) / (tn / 2)) <= ctas) tn >>= 1;
+  }
   if (tn == 256 && force_split <= 1 && persistent_enabled()) {
     // prefill-sized: persistent kernel with double-buffered accumulators
     const int pr = launch_gemm_persistent(X, W, Y, residual, bias, M, N, K, ldx, ldw, ldy, ldr, w_rows, dual, dual_row_offset,
@@ -873,9 +882,8 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   if (r != 0) return -200 + r;
   const int n_tiles = (N + 127) / 128;
   const int m_tiles = (M + tn - 1) / tn;
-  // The ring of a gated tile of 64 tokens leaves an SM room for one CTA: 2 x 14336 x 4096 split twice was 224 CTAs in two rounds. The split
-  // goes by the tile in use, also where a router's is smaller than its tokens say (1024 x 128 x 2048 unsplit: 23 us on 16 SMs).
-  int nsplit = force_split > 0 ? force_split : pick_split(M, N, K, tn, tn == 64 && dual ? 1 : 2, sm_count > 0 ? sm_count : 148);
+  // The ring of a gated tile of 64 tokens leaves an SM room for one CTA: 2 x 14336 x 4096 split twice was 224 CTAs in two rounds.
+  int nsplit = force_split > 0 ? force_split : narrow ? 1 : pick_split(M, N, K, tn, tn == 64 && dual ? 1 : 2, sm_count > 0 ? sm_count : 148);
   const int kblocks = (K + 63) / 64;
   while (nsplit > 1 && (kblocks + nsplit - 1) / nsplit * (nsplit - 1) >= kblocks) nsplit >>= 1;  // no empty split
   p.staged = staged_epilogue_ok(Y, residual, N, ldy, ldr, out_fp32) && tn >= 64 && nsplit == 1;

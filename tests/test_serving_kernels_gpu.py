@@ -230,10 +230,20 @@ def test_norm_of_few_wide_rows(M, H, residual):
 
 @pytest.mark.parametrize("M,N,K", [(1024, 128, 512), (300, 96, 320), (700, 60, 2048)])
 def test_router_of_prompts(M, N, K):
-    """A narrow fp32 output over many tokens: token tiles of 64 with K split over a cluster."""
+    """A narrow fp32 output over many tokens: small token tiles."""
     x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
     y = ops.linear(x, w, out_dtype=torch.float32)
     assert rel_l2(y, x.float() @ w.float().t()) < 1e-5
+
+
+@pytest.mark.parametrize("M", [257, 300, 1024, 2048, 4099, 9000])
+@pytest.mark.parametrize("N,K", [(128, 2048), (96, 320), (256, 4096)])
+def test_router_sums_have_one_order(M, N, K):
+    """Logits that decide between experts do not depend on how many tokens stand beside them: every tile size adds K in one order."""
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    y = ops.linear(x, w, out_dtype=torch.float32)
+    alone = torch.cat([ops.linear(x[i:i + 128], w, out_dtype=torch.float32, force_split=1) for i in range(0, M, 128)])
+    assert torch.equal(y, alone)
 
 
 @pytest.mark.parametrize("M,N,K", [(130, 1096, 256), (400, 4736, 128), (1250, 4096, 192), (1900, 2048, 128)])
