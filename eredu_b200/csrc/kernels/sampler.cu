@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(kSampThreads) sampler_kernel(SamplerParams p) 
 
   pdl_launch_early();
   trace_mark(kTraceSampler, kTraceStart);
+  cluster_arrive_relaxed();         // waited for in front of the exchange below, when its result has long been there
   pdl_wait();
   trace_mark(kTraceSampler, kTraceAfterWait);
   pdl_launch_dependents();
@@ -238,8 +239,11 @@ __global__ void __launch_bounds__(kSampThreads) sampler_kernel(SamplerParams p) 
         row[tok] = x;
       }
     }
+    __syncwarp();
+    cluster_wait_acquire();
     cluster_arrive_release();
     cluster_wait_acquire();
+    cluster_arrive_relaxed();
   }
 
   // ---- 2. max / argmax (the greedy answer; also the softmax shift)
@@ -276,11 +280,13 @@ __global__ void __launch_bounds__(kSampThreads) sampler_kernel(SamplerParams p) 
     }
   }
   block_argmax(vmax, imax, scr);
+  cluster_wait_acquire();           // every CTA of the cluster has started: its shared memory may be written
   if (nrank > 1) {
     if (tid == 0) {
       const uint32_t at = mapa_shared(smem_u32(&part[rank]), 0u);
       asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_int(vmax)), "r"(imax) : "memory");
     }
+    __syncwarp();
     cluster_arrive_release();
     cluster_wait_acquire();
     if (rank != 0) return;

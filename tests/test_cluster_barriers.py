@@ -1,0 +1,40 @@
+"""Stores into the shared memory of another CTA: the CTAs of a cluster are placed together, but only a cluster barrier says that they run."""
+import re
+from pathlib import Path
+
+import pytest
+
+KERNELS = Path(__file__).resolve().parents[1] / "eredu_b200" / "csrc" / "kernels"
+
+
+def unguarded_stores(source):
+    """Lines of remote stores that no wait on the cluster barrier dominates: a wait counts while the block that it stands in is open."""
+    found, depth, waits = [], 0, []
+    for number, line in enumerate(source.splitlines(), 1):
+        code = re.sub(r"//.*", "", line)
+        if "st.shared::cluster" in code and not waits:
+            found.append(number)
+        code = re.sub(r'"[^"]*"', '""', code)
+        for token in re.findall(r"[{}]|cluster_wait_acquire\(\)", code):
+            if token == "{":
+                depth += 1
+            elif token == "}":
+                depth -= 1
+                waits = [d for d in waits if d <= depth]
+            else:
+                waits.append(depth)
+    assert depth == 0
+    return found
+
+
+@pytest.mark.parametrize("text, lines", [
+    ("void f() {\n cluster_wait_acquire();\n if (a) {\n  asm(\"st.shared::cluster.f32 [%0], {%1};\");\n }\n}", []),
+    ("void f() {\n if (a) {\n  cluster_wait_acquire();\n }\n asm(\"st.shared::cluster.f32\");\n}", [5]),
+    ("void f() {\n cluster_wait_acquire();\n}\nvoid g() {\n asm(\"st.shared::cluster.f32\");\n}", [5])])
+def test_reading_of_blocks(text, lines):
+    assert unguarded_stores(text) == lines
+
+
+@pytest.mark.parametrize("name", ["sampler.cu"])
+def test_remote_stores_wait_for_their_target(name):
+    assert unguarded_stores((KERNELS / name).read_text()) == []
