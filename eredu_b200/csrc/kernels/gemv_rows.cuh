@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) gemv_rows_kernel(GemmParams p
   __shared__ float s_parts[8][MT];      // cluster rank 0: of every CTA
   pdl_launch_early();
   trace_mark(kTraceGemm, kTraceStart);
+  if (p.ssq_out != nullptr) cluster_arrive_relaxed();     // waited for in front of the store into CTA 0
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, side = warp / WARPS;
   const int n0 = blockIdx.x * kRowsOut;
   const int pieces = p.K >> 3;
@@ -145,10 +146,13 @@ __global__ void __launch_bounds__(kRowsThreads, 2) gemv_rows_kernel(GemmParams p
     // the 128 columns whose sum of squares is one number belong to the cluster's eight CTAs
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    __syncwarp();
+    cluster_wait_acquire();                               // CTA 0 has started: its shared memory may be written
     if (threadIdx.x < MT)
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_shared(smem_u32(&s_parts[0][0]) + (rank * MT + threadIdx.x) * 4u, 0u)),
                    "f"(s_sq[threadIdx.x])
                    : "memory");
+    __syncwarp();
     cluster_arrive_release();
     cluster_wait_acquire();
     if (rank == 0 && threadIdx.x < p.M) {

@@ -35,6 +35,6 @@ def test_reading_of_blocks(text, lines):
     assert unguarded_stores(text) == lines
 
 
-@pytest.mark.parametrize("name", ["sampler.cu"])
+@pytest.mark.parametrize("name", sorted(p.name for p in KERNELS.glob("*.cu*")))
 def test_remote_stores_wait_for_their_target(name):
     assert unguarded_stores((KERNELS / name).read_text()) == []
