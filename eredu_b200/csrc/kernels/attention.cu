@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(AttnParams p) {
 // A step of one sequence is bound by a chain of latencies: length, table, first pages, rows of the projection, then little arithmetic and the
 // exchange of the splits. With p.settled only the projection comes from the kernel before this one - what the lengths, tables and pages
 // hold was written by kernels that had ended when that one passed its own dependency wait - so the first three links run ahead of the
-// wait, under the tail of the projection. Measured over whole decode steps: one sequence, 16 layers of 64-wide heads, three draft passes
+// wait, under the tail of the projection. That holds because a kernel releases the next one behind its own wait; a build that releases at
+// entry (EREDU_PDL_EARLY=1) waits first. Measured over whole decode steps: one sequence, 16 layers of 64-wide heads, three draft passes
 // 2917 -> 2870 us; one sequence, 32 layers of 128-wide heads 3687 -> 3660 us; 32 sequences of the same 5499 -> 5475 us.
 template <int DK, int DV, int MT, bool EXT, bool POOL>
 __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) attn_decode_kernel(AttnParams p) {
@@ -963,7 +964,7 @@ static int launch_decode_all(AttnParams p, int batch, int q_per_seq, int n_q_hea
   const int settled = p.settled;
   for (int t0 = 0; t0 < q_per_seq; t0 += t_per) {
     p.t0 = t0;
-    p.settled = settled && t0 == 0 && p.qkv != nullptr && p.pool == 0;   // a second launch reads what the first one appends
+    p.settled = !EREDU_PDL_EARLY && settled && t0 == 0 && p.qkv != nullptr && p.pool == 0;   // a second launch reads what the first one appends
     p.t_count = (q_per_seq - t0 < t_per) ? q_per_seq - t0 : t_per;
     const int rows = p.t_count * group;
     cudaError_t e;

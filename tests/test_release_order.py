@@ -1,0 +1,15 @@
+"""Reads ahead of a kernel's dependency wait that are right only where every kernel releases the next one behind its own wait."""
+import re
+from pathlib import Path
+
+KERNELS = Path(__file__).resolve().parents[1] / "eredu_b200" / "csrc" / "kernels"
+
+
+def test_lengths_and_pages_are_not_read_ahead_in_builds_that_release_at_entry():
+    decode = (KERNELS / "attention.cu").read_text()
+    writes = re.findall(r"p\.settled = ([^;]*);", decode)
+    launches = [w for w in writes if "t0" in w]          # what the kernel sees; the entry point's flag only passes through it
+    assert launches and all("!EREDU_PDL_EARLY &&" in w for w in launches)
+    assert "settled = p.settled != 0" in decode and decode.count("settled = p.settled") == 2
+    latent = (KERNELS / "latent_attention.cu").read_text()
+    assert "if (EREDU_PDL_EARLY) pdl_wait();" in latent
