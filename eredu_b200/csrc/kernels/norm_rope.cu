@@ -30,16 +30,19 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const __nv_bfloat16* _
   trace_mark(kTraceRmsNorm, kTraceStart);
   const size_t row = blockIdx.x;
   const int nch = H >> 3;
-  // THREADS = 1024 (a thread has one piece of the row): weights are on their way before the dependency wait, like those of the GEMMs
+  // THREADS = 1024 (a thread has one piece of the row): the weights are on their way to L2 before the dependency wait, and are read next to
+  // the row. They are not read ahead of the wait: a caller may have filled them with the kernel in front of this one.
   constexpr bool kAhead = THREADS == 1024;
+  if (kAhead && (threadIdx.x & 3) == 0 && static_cast<int>(threadIdx.x) < nch)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(w + 8 * threadIdx.x));
+  pdl_wait();
+  trace_mark(kTraceRmsNorm, kTraceAfterWait);
+  pdl_launch_dependents();
   float4 wa[2] = {};
   if (kAhead && static_cast<int>(threadIdx.x) < nch) {
     wa[0] = reinterpret_cast<const float4*>(w)[2 * threadIdx.x];
     wa[1] = reinterpret_cast<const float4*>(w)[2 * threadIdx.x + 1];
   }
-  pdl_wait();
-  trace_mark(kTraceRmsNorm, kTraceAfterWait);
-  pdl_launch_dependents();
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
   const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + row * H) : nullptr;
   float vals[MAXCH][8];

@@ -13,3 +13,11 @@ def test_lengths_and_pages_are_not_read_ahead_in_builds_that_release_at_entry():
     assert "settled = p.settled != 0" in decode and decode.count("settled = p.settled") == 2
     latent = (KERNELS / "latent_attention.cu").read_text()
     assert "if (EREDU_PDL_EARLY) pdl_wait();" in latent
+
+
+def test_norm_weights_are_read_behind_the_wait():
+    """They may be what the kernel just in front has written (a vector of ones, a converted weight)."""
+    source = (KERNELS / "norm_rope.cu").read_text()
+    kernel = source[source.index("rmsnorm_kernel(const"):]
+    ahead = kernel[:kernel.index("pdl_wait();")]
+    assert not re.search(r"\(w\)\[|= w\[", ahead)
