@@ -257,6 +257,8 @@ class QuantLinear:
         137 us and a round trip of 470 MB less per layer than with the activation kernel), the projection followed by the activation
         kernel otherwise."""
         inter = self.out_features // 2
+        if x.is_cuda:
+            assert x.shape[1] == self.in_features and x.dtype == torch.bfloat16 and x.stride(1) == 1
         if self._gemv_ok(x) and self.out_features % 32 == 0:
             return self._gemv(x, bias, None, None, torch.bfloat16, True, limit or 0.0)
         from .core import gated_linear, silu_mul

@@ -145,3 +145,19 @@ def test_gguf_q4k_q6k_model_runs_on_native_codes(tmp_path):
     a, b = native.prefill_logits(prompt), dense.prefill_logits(prompt)
     rel = float((a - b).norm() / b.norm())
     assert rel < 0.05 and torch.nn.functional.cosine_similarity(a, b, dim=0) > 0.995
+
+
+@pytest.mark.parametrize("shape, dtype", [((300, 192), torch.bfloat16), ((300, 320), torch.bfloat16), ((4, 192), torch.bfloat16), ((300, 256), torch.float32)])
+def test_gated_projection_refuses_rows_of_another_width_or_type(shape, dtype):
+    """Before anything is launched: the kernels take the width from the rows."""
+    class Rows:
+        is_cuda = True
+
+        def stride(self, dim):
+            return (self.shape[1], 1)[dim]
+
+    x = Rows()
+    x.shape, x.dtype = shape, dtype
+    ql = QuantLinear.from_dense(torch.randn(128, 256), 4, 64)
+    with pytest.raises(AssertionError):
+        ql.gated(x)
