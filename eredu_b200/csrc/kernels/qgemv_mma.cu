@@ -7,7 +7,7 @@
 //
 //   warp          : a 16-row weight tile x a K range. The codes are stored tile by tile (16 rows x 64 columns = 512
 //                   contiguous bytes, consecutive K blocks of a row tile adjacent), so the warp's stream is one contiguous
-//                   run that it fetches with bulk copies (cp.async.bulk, 2 KB each) into a private four-slot ring in
+//                   run that it fetches with bulk copies (cp.async.bulk, 1 or 2 KB each) into a private ring of slots in
 //                   shared memory: several KB in flight per warp at no register cost. A lane then reads its 16 codes of
 //                   rows g and g + 8 with two 8-byte shared-memory loads.
 //   dequant       : one shift + one lop3 place two nibbles into the mantissas of a bf16 pair (128 + n). Groups of 64 or
@@ -110,14 +110,18 @@ __device__ __forceinline__ void mma_bf16_16816_zero(float* d, uint32_t a0, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// Per-warp ring of bulk copies. A slot holds two consecutive K blocks of the warp's four row tiles: the codes (512 bytes
+// Per-warp ring of bulk copies. A slot holds two or four consecutive K blocks of the warp's T row tiles: the codes (512 bytes
 // per block and tile) followed by their (scale, bias) words (64 bytes per group and tile). Both are contiguous in global
 // memory (tiled layouts), so a slot is filled by one bulk copy per tile and table, each issued by a lane of its own: no
 // registers are spent on prefetch and a warp keeps 9-14 KB in flight, which is what the HBM latency asks for.
-constexpr int kGemvChunk = 2;
-constexpr int kGemvTiles = 4;    // row tiles of a warp. What a K block costs once - its activations and their sums - is shared
-                                 // by 64 rows: with one tile per warp these were half of the instructions, and with eight tokens
-                                 // the activations were twice the bytes of the weights they met.
+// What a K block costs once - its activations and their sums - is shared by the 16 T rows of a warp: with one tile per warp these
+// are half of the instructions, and with eight tokens the activations are twice the bytes of the weights they meet. How many tiles
+// a launch takes, see eredu_qgemv4.
+template <bool RAW, int T>
+struct GemvRing {
+  static constexpr int kChunk = T == 4 ? 2 : 4;
+  static constexpr int kSlots = T == 4 ? (RAW ? 3 : 2) : T == 2 ? 2 : 4;     // of four tiles, groups of at least 64: two CTAs fit an SM
+};
 
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -126,21 +130,15 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
                : "memory");
 }
 
-// RAW: three slots (groups of at least 64, so that two CTAs fit an SM), else two.
-template <bool RAW>
-struct GemvRing {
-  static constexpr int kSlots = RAW ? 3 : 2;
-};
-
-// GATED: the warp's four row tiles are two of the gate and two of the up rows. RAW: accumulator-side affine map (group 64 / 128),
+// GATED: half of the warp's T row tiles are gate rows, half up rows. RAW: accumulator-side affine map (group 64 / 128),
 // else the weights are dequantised to bf16 in registers (any power-of-two group from 16).
-template <bool GATED, bool RAW>
+template <bool GATED, bool RAW, int T>
 __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvParams p) {
   constexpr int S = GATED ? 2 : 1;
-  constexpr int T = kGemvTiles, RT = T / S;        // tiles of a warp, of these tiles of output rows
+  constexpr int RT = T / S;        // of a warp's T tiles, tiles of output rows
   constexpr int TOK = 8;
-  constexpr int C = kGemvChunk;
-  constexpr int SLOTS = GemvRing<RAW>::kSlots;
+  constexpr int C = GemvRing<RAW, T>::kChunk;
+  constexpr int SLOTS = GemvRing<RAW, T>::kSlots;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);                  // [8 warps][SLOTS]
   uint8_t* ring = smem + 256;
@@ -245,7 +243,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
         const uint8_t* codes = slot + j * 512 + code_off;
         const uint32_t* dqs = reinterpret_cast<const uint32_t*>(slot + T * C * 512) + gi * 16 + g;
         if (RAW) {
-          // the four tiles side by side: their chains of products do not wait for one another
+          // the tiles side by side: their chains of products do not wait for one another
           float tx[4], tmp[T][4];
           uint2 w_lo[T], w_hi[T];
 #pragma unroll
@@ -463,28 +461,28 @@ __global__ void __launch_bounds__(kGemvThreads, 2) qgemv4_kernel(const QGemvPara
   trace_mark(kTraceQGemm, kTraceEnd);
 }
 
-// Rows of a CTA whose warps split K wk ways.
-static int gemv_rows(int wk, bool gated) { return 8 / wk * 16 * kGemvTiles / (gated ? 2 : 1); }
+// Rows of a CTA whose warps split K wk ways, with `tiles` row tiles to a warp.
+static int gemv_rows(int wk, bool gated, int tiles) { return 8 / wk * 16 * tiles / (gated ? 2 : 1); }
 
 // Dynamic shared memory of a launch: barriers, then the larger of the eight per-warp rings and the partial tiles.
-static int gemv_smem_bytes(const QGemvParams& p, bool gated, int slots) {
-  const int gpc = std::max(1, (kGemvChunk * 64) >> p.group_shift);
-  const int ring = 8 * slots * kGemvTiles * (kGemvChunk * 512 + gpc * 64);
-  const int red = p.wk * (gated ? 2 : 1) * 8 * (gemv_rows(p.wk, gated) + 4) * 4;
+static int gemv_smem_bytes(const QGemvParams& p, bool gated, int tiles, int chunk, int slots) {
+  const int gpc = std::max(1, (chunk * 64) >> p.group_shift);
+  const int ring = 8 * slots * tiles * (chunk * 512 + gpc * 64);
+  const int red = p.wk * (gated ? 2 : 1) * 8 * (gemv_rows(p.wk, gated, tiles) + 4) * 4;
   return 256 + std::max(ring, red);
 }
 
-template <bool GATED, bool RAW>
+template <bool GATED, bool RAW, int T>
 static cudaError_t launch_gemv(const QGemvParams& p, int n_ctas, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_ctas, p.ns, 1);
   cfg.blockDim = dim3(kGemvThreads, 1, 1);
-  const int smem = gemv_smem_bytes(p, GATED, GemvRing<RAW>::kSlots);
+  const int smem = gemv_smem_bytes(p, GATED, T, GemvRing<RAW, T>::kChunk, GemvRing<RAW, T>::kSlots);
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(qgemv4_kernel<GATED, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(qgemv4_kernel<GATED, RAW, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
@@ -506,7 +504,7 @@ static cudaError_t launch_gemv(const QGemvParams& p, int n_ctas, cudaStream_t st
   }
   cfg.attrs = attr;
   cfg.numAttrs = nattr;
-  return cudaLaunchKernelEx(&cfg, qgemv4_kernel<GATED, RAW>, p);
+  return cudaLaunchKernelEx(&cfg, qgemv4_kernel<GATED, RAW, T>, p);
 }
 
 }  // namespace eredu
@@ -553,22 +551,39 @@ extern "C" int eredu_qgemv4(const void* X, const void* wq, const void* dq, void*
     p.use_comm = 1;
     p.comm = *pc;
   }
-  // K splits: over the warps of a CTA first, over the CTAs of a cluster when the rows alone do not give every SM its two CTAs
+  // Row tiles of a warp and K splits. Four tiles take the fewest instructions per row and win wherever the kernel is bound by issue; a matrix
+  // that gives the SMs only a round of CTAs, or less, is bound by the first copies and the end of each, and wants more and smaller ones:
+  // two tiles while these make no more than two CTAs an SM, one (a plain matrix) while they make no more than one. Above 256 K blocks
+  // the instructions count again (8192 x 28672, eight tokens: 43.5 us with two tiles, 38.0 with four). Microseconds of one token with
+  // 1 / 2 / 4 tiles: 2048 x 2048 2.8 / 3.0 / 3.9, 4096 x 4096 5.1 / 4.5 / 6.3, 4096 x 14336 12.6 / 12.7 / 12.9, 8192 x 8192 - / 11.6 / 13.0,
+  // 10240 x 8192 22.4 / 19.1 / 19.6, 57344 x 8192 92 / 72 / 70.
   const int sm = sm_count > 0 ? sm_count : 148;
+  const auto ctas = [&](int wk, int tiles) { return (p.n_out + gemv_rows(wk, gated, tiles) - 1) / gemv_rows(wk, gated, tiles); };
+  int tiles = 4;
+  if (p.kblocks <= 256) tiles = !gated && ctas(8, 1) <= sm ? 1 : ctas(8, 2) <= 2 * sm ? 2 : 4;
+  // K is split over the warps of a CTA. Half of them where that makes one round of two CTAs an SM out of two rounds (28672 x 4096: 22.2 -> 20.4
+  // us). Over the CTAs of a cluster as well where the rows leave SMs idle and a warp keeps six blocks (1024 x 8192: 5.6 -> 5.1), or, with
+  // four tiles, four (8192 x 28672: 36.7).
   int wk = 8, ns = 1;
-  while (ns < 8 && static_cast<long>((p.n_out + gemv_rows(8, gated) - 1) / gemv_rows(8, gated)) * ns * 2 <= 2 * sm && p.kblocks >= 8 * ns * 2 * 4) ns *= 2;
+  if (ctas(8, tiles) > 2 * sm && ctas(4, tiles) <= 2 * sm) wk = 4;
+  while (ns < 8 && ctas(8, tiles) * ns * 2 <= (tiles == 4 ? 2 : 1) * sm && p.kblocks >= 8 * ns * 2 * (tiles == 4 ? 4 : 6)) ns *= 2;
   while (wk > 1 && p.kblocks < wk * 2) wk >>= 1;
   if (force_wk > 0) wk = force_wk;
   if (force_ns > 0) ns = force_ns;
   if ((wk != 1 && wk != 2 && wk != 4 && wk != 8) || ns < 1 || ns > 8 || (ns & (ns - 1)) != 0) return -1;
   p.wk = wk;
   p.ns = ns;
-  // splits start on multiples of two K blocks: a slot of the copy ring then starts on a group boundary for every group size
-  p.blocks_per_split = ((p.kblocks + wk * ns - 1) / (wk * ns) + kGemvChunk - 1) / kGemvChunk * kGemvChunk;
-  const int n_ctas = (p.n_out + gemv_rows(wk, gated) - 1) / gemv_rows(wk, gated);
+  // splits start on whole slots of the copy ring, which start on a group boundary for every group size
+  const int chunk = tiles == 4 ? 2 : 4;
+  p.blocks_per_split = ((p.kblocks + wk * ns - 1) / (wk * ns) + chunk - 1) / chunk * chunk;
+  const int n_ctas = ctas(wk, tiles);
   const bool raw = group >= 64 && force_exact_bf16 == 0;
-  cudaError_t e = gated ? (raw ? launch_gemv<true, true>(p, n_ctas, stream) : launch_gemv<true, false>(p, n_ctas, stream))
-                        : (raw ? launch_gemv<false, true>(p, n_ctas, stream) : launch_gemv<false, false>(p, n_ctas, stream));
+  cudaError_t e;
+  if (tiles == 4) e = gated ? (raw ? launch_gemv<true, true, 4>(p, n_ctas, stream) : launch_gemv<true, false, 4>(p, n_ctas, stream))
+                            : (raw ? launch_gemv<false, true, 4>(p, n_ctas, stream) : launch_gemv<false, false, 4>(p, n_ctas, stream));
+  else if (tiles == 2) e = gated ? (raw ? launch_gemv<true, true, 2>(p, n_ctas, stream) : launch_gemv<true, false, 2>(p, n_ctas, stream))
+                                 : (raw ? launch_gemv<false, true, 2>(p, n_ctas, stream) : launch_gemv<false, false, 2>(p, n_ctas, stream));
+  else e = raw ? launch_gemv<false, true, 1>(p, n_ctas, stream) : launch_gemv<false, false, 1>(p, n_ctas, stream);
   eredu_count_launches(1);
   return static_cast<int>(e);
 }

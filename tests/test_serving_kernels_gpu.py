@@ -100,6 +100,16 @@ def test_four_bit_rows_of_few_tokens(M, N, K, group, gated):
     assert rel_l2(got, ref) < (BF16 if group >= 64 else 2 * BF16)
 
 
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("N,K,group,gated", [(148 * 16, 320, 64, False), (148 * 16 + 16, 320, 64, False), (296 * 32, 128, 32, False),
+                                             (296 * 32 + 16, 192, 64, False), (80, 64 * 257, 64, False), (2 * 48, 64 * 258, 32, True),
+                                             (2 * 296 * 16, 192, 64, True), (2 * (296 * 16 + 16), 192, 64, True), (296 * 64 + 16, 512, 128, False),
+                                             (128, 8192, 64, False)])
+def test_four_bit_rows_at_the_borders_of_the_plan(M, N, K, group, gated):
+    """Matrices on either side of where a warp takes one, two and four row tiles and where fewer warps, or a cluster, split K."""
+    test_four_bit_rows_of_few_tokens(M, N, K, group, gated)
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 5, 64])
 @pytest.mark.parametrize("H,inter", [(256, 96), (2048, 768)])
 def test_experts_of_few_tokens(T, H, inter):
