@@ -35,6 +35,7 @@ _SIGNATURES = {
     "eredu_sampler_row_bytes": (I, []),
     "eredu_launch_count": (L, []),
     "eredu_selftest_bounded_wait": (I, [P, L, P]),
+    "eredu_sample_row_ctas": (I, [I, I, I]),
     "eredu_sample": (I, [P, P, I, P, P, I, P, P, I, I, P]),
     "eredu_spec_verify": (I, [P, P, P, P, P, I, I, I, P]),
 }

@@ -198,6 +198,11 @@ def test_largest_logit_over_a_cluster(R, V):
     assert int(ops.sample(logits, rows, all_greedy=True)[0]) == V - 1
 
 
+@pytest.mark.parametrize("R,V", [(13, 48000), (14, 50257), (32, 24004), (33, 47999), (37, 48000), (74, 50000), (75, 50000), (2, 23996)])
+def test_largest_logit_at_the_borders_of_the_rule(R, V):
+    test_largest_logit_over_a_cluster(R, V)
+
+
 @pytest.mark.parametrize("T,k,H", [(1, 8, 2048), (3, 1, 1000), (64, 6, 4104), (2, 32, 64)])
 def test_weighted_expert_rows(T, k, H):
     """Slots that do not fill a batch, columns that do not fill a CTA, routes of other ranks; sums of squares of what is stored."""
