@@ -45,6 +45,12 @@ def test_rotation_and_append_rows(M, n_q, n_kv, D, rot, interleaved):
     assert torch.equal(vc, vr)
 
 
+@pytest.mark.parametrize("M", [125, 126])
+def test_rotation_of_few_tokens(M):
+    """On either side of where a token has a CTA of its own (20 heads of 128 with norms: from 126 tokens on)."""
+    test_rotation_and_append_rows(M, 16, 2, 128, 128, False)
+
+
 @pytest.mark.parametrize("norms", ["none", "queries", "both"])
 @pytest.mark.parametrize("D,rot,interleaved", [(128, 128, False), (128, 128, True), (64, 64, False), (64, 48, True), (128, 16, False)])
 def test_rotation_gives_the_same_bits_on_either_kernel(D, rot, interleaved, norms):
