@@ -238,6 +238,12 @@ def test_expert_plan_keeps_the_order_of_the_routes(E, e0, e1, routes, k):
     assert plan.seg.tolist() == [int(((flat >= e0) & (flat < e0 + i)).sum()) for i in range(e1 - e0 + 1)]
 
 
+@pytest.mark.parametrize("E,e0,e1,routes,k", [(8, 0, 8, 3000, 2), (9, 0, 9, 3000, 3), (20, 4, 20, 130, 2)])
+def test_expert_plan_of_few_experts(E, e0, e1, routes, k):
+    """On either side of where lanes find their like by values instead of bits; batches of routes that end early."""
+    test_expert_plan_keeps_the_order_of_the_routes(E, e0, e1, routes, k)
+
+
 @pytest.mark.parametrize("M", [1, 64, 65])
 @pytest.mark.parametrize("H", [2048, 2056, 4104, 8192])
 @pytest.mark.parametrize("residual", [False, True])
