@@ -225,6 +225,20 @@ def test_weighted_expert_rows(T, k, H):
     assert torch.allclose(ssq.sum(-1), out.float().square().sum(-1), rtol=H * 2.0 ** -24, atol=0)
 
 
+@pytest.mark.parametrize("T,k,H", [(1023, 1, 1000), (1024, 1, 1000), (1500, 2, 4104), (1024, 3, 64)])
+def test_weighted_expert_rows_of_prompts(T, k, H):
+    """Few slots of many tokens have a kernel of their own; both add in one order."""
+    rows, w = torch.randn(T * k, H, device=DEV).bfloat16(), torch.rand(T, k, device=DEV)
+    res = torch.randn(T, H, device=DEV).bfloat16()
+    pos = torch.randperm(T * k, device=DEV).int()
+    pos[1::5] = -1
+    out, other, ssq = torch.empty_like(res), torch.empty_like(res), torch.empty(T, (H + 1023) // 1024, device=DEV)
+    p, stream = moe_ops.ptr, moe_ops.stream_ptr(out.device)
+    assert moe_ops.lib().eredu_moe_combine(p(rows), p(pos), p(w), p(res), None, p(out), T, k, H, stream) == 0
+    assert moe_ops.lib().eredu_moe_combine_ssq(p(rows), p(pos), p(w), p(res), None, p(other), p(ssq), T, k, H, stream) == 0
+    assert torch.equal(out, other) and rel_l2(out, res.float() + moe_ops.RoutedRows(rows, pos, w).summed()) < BF16
+
+
 @pytest.mark.parametrize("E,e0,e1,routes,k", [(128, 0, 128, 8192, 8), (8, 2, 6, 4096, 2), (512, 0, 512, 5000, 10), (60, 0, 30, 33, 3), (1, 0, 1, 40, 1)])
 def test_expert_plan_keeps_the_order_of_the_routes(E, e0, e1, routes, k):
     ids = torch.randint(0, E, (routes // k, k), device=DEV, dtype=torch.int32)
