@@ -784,9 +784,16 @@ static bool staged_epilogue_ok(const void* Y, const void* residual, int N, int l
 // step of 16 layers 2048 wide 766 -> 728 us, up to 24 MB one of 8 expert layers 672 -> 628; 33 MB and above lose it again (759 us, and
 // 912 -> 945 for 8 layers 4096 wide). Two tokens are twice the arithmetic on the CUDA cores: 3072 x 2048 5.7 -> 5.1 us, 5120 x 2048
 // 6.8 -> 7.8.
-static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K, int ldx, int ldw, int dual, int flags, int force_split) {
+// Its CTAs have to run in one round, two to an SM: of short rows a second round costs more than the tensor-core kernel (5120 x 512 4.3
+// us there, 4.8 here; 12288 x 512 5.5 and 8.1); one token with rows of 2048 still gains (5120 x 2048 7.1 -> 6.7). With sums of squares
+// clusters of eight leave part of a GPC empty: one round is 7/8 of that, three quarters for two tokens (4608 x 512 4.3 and 6.3, 4096 x 512 with
+// two tokens 4.2 and 4.5), unless rows are long enough to make up for it (4608 x 1024 9.0 and 6.8).
+static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K, int ldx, int ldw, int dual, int flags, int force_split, bool ssq,
+                              int sm_count) {
   if (force_split > 0 || dual || M > 2 || (flags & 1) || K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || N % kRowsOut != 0) return false;
   if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) != 0) return false;
+  const int ctas = N / kRowsOut, round = 2 * (sm_count > 0 ? sm_count : 148);
+  if (ssq ? ctas > round || (K < 1024 && ctas * 8 > round * (M == 1 ? 7 : 6)) : ctas > round && (M > 1 || K < 2048)) return false;
   return static_cast<long long>(N) * K * 2 <= (M == 1 ? 24LL : 13LL) << 20;
 }
 
@@ -870,7 +877,7 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   // the remaining tiles are prefetched into L2 as well (level 2). EREDU_GEMM_PREFETCH overrides the level.
   p.w_static = (flags & 1) ? 0 : prefetch_level(static_cast<long long>(w_rows) * K * 2);
   cudaError_t e;
-  if (rows_kernel_takes(X, W, M, N, K, ldx, ldw, dual, flags, force_split)) {
+  if (rows_kernel_takes(X, W, M, N, K, ldx, ldw, dual, flags, force_split, ssq_out != nullptr, sm_count)) {
     e = M == 1 ? launch_rows<1>(p, X, W, ldx, ldw, stream) : launch_rows<2>(p, X, W, ldx, ldw, stream);
     eredu_count_launches(1);
     return static_cast<int>(e);

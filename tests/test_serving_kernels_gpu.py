@@ -179,6 +179,12 @@ def test_rows_of_one_and_two_tokens(M, N, K):
     assert rel_l2(y, torch.relu(x.float() @ w.float().t()) ** 2) < 1e-5
 
 
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("N,K", [(4736, 64), (4752, 64), (4144, 1016), (4160, 1016), (4736, 1024), (3552, 512), (3568, 512)])
+def test_rows_of_one_and_two_tokens_at_the_borders_of_a_round(M, N, K):
+    test_rows_of_one_and_two_tokens(M, N, K)
+
+
 @pytest.mark.parametrize("M", [257, 2049, 2304, 4100])
 def test_prompt_gemm_bands(M):
     """Token tiles that do not fill a band, and a last one that is nearly empty."""
