@@ -1036,8 +1036,11 @@ extern "C" int eredu_gemm_bf16_grouped(const void* X, const void* W, void* Y, co
   if (rows_cap < n_work) n_work = rows_cap;
   // Items of at most 16 rows that give every SM two tiles or more: a step that reads most experts. The persistent form streams their weights
   // without a start and an end of a CTA per tile: both GEMMs of 128 experts (768 x 2048), 8 tokens 101 -> 93 us, 64 tokens 194 -> 188; in a
-  // decode step of 32 sequences, behind and in front of other kernels, 12.5 us a layer (8275 -> 7877 for 32 of them).
-  if (tile == 16 && bias == nullptr && act == 0 && act_limit <= 0.f && force_split <= 0 &&
+  // decode step of 32 sequences, behind and in front of other kernels, 12.5 us a layer (8275 -> 7877 for 32 of them). Few experts are
+  // streamed as fast by CTAs of their own (8 of 14336 x 4096, 4 tokens 268 us, persistent 278); and above twelve rows an expert, many have
+  // a second item, which meets the weights in L2 only where it runs beside the first (32 of 2880 x 2880, 16 rows each 283 us, persistent 342).
+  if (tile == 16 && bias == nullptr && act == 0 && act_limit <= 0.f && force_split <= 0 && n_work >= 32 &&
+      static_cast<long long>(rows_cap) * w_rows_per_expert <= 12LL * w_rows_total &&
       static_cast<long long>(n_work) * ((N + 127) / 128) >= 2LL * (sm_count > 0 ? sm_count : 148)) {
     const int pr = launch_gemm_persistent_grouped(X, W, Y, work, n_work, tile, rows_cap, N, K, ldx, ldw, ldy, w_rows_total, w_rows_per_expert, dual,
                                                   sm_count, status, stream);
