@@ -255,7 +255,9 @@ class QuantLinear:
         """silu(x Wgate^T) * (x Wup^T) for a weight that stacks gate rows over up rows: one kernel for decode-sized
         batches, the weight decoded once and the dense kernel with its SwiGLU epilogue for prompt-sized ones (70 B shape, 4096 tokens:
         137 us and a round trip of 470 MB less per layer than with the activation kernel), the projection followed by the activation
-        kernel otherwise."""
+        kernel otherwise. That includes prompts of many tokens where the sums are short: the epilogue of a gated tile takes longer than the
+        next tile's products (1000 tokens, us of the activation kernel and of the epilogue: 8192 x 1024 60 / 68, 2048 x 2048 29 / 32, 4096 x 2048
+        47 / 48, 8192 x 2048 86 / 83, 2048 x 4096 45 / 43; 400 tokens, 8192 x 1024 37 / 36)."""
         inter = self.out_features // 2
         if x.is_cuda:
             assert x.shape[1] == self.in_features and x.dtype == torch.bfloat16 and x.stride(1) == 1
@@ -263,7 +265,9 @@ class QuantLinear:
             return self._gemv(x, bias, None, None, torch.bfloat16, True, limit or 0.0)
         from .core import gated_linear, silu_mul
 
-        if x.is_cuda and x.shape[0] > self.DENSE_FALLBACK_TOKENS and not limit and inter % 8 == 0 and x.stride(0) % 8 == 0:
+        short = self.in_features <= 1024 or (self.in_features <= 2048 and inter <= 2048)
+        if (x.is_cuda and x.shape[0] > self.DENSE_FALLBACK_TOKENS and not (short and x.shape[0] > 512) and not limit and inter % 8 == 0
+                and x.stride(0) % 8 == 0):
             return gated_linear(x, self._dense(), inter, bias=bias, dynamic_weight=True)
 
         return silu_mul(self(x, bias=bias), inter, limit or 0.0)

@@ -92,6 +92,11 @@ def test_gated_projection_of_prompts(M, inter, K, bits):
         assert rel_l2(ql.gated(x, bias=bias, limit=limit), ref) < (BF16 if not limit else 3 * BF16)
 
 
+@pytest.mark.parametrize("M,inter,K", [(512, 2056, 1088), (513, 2048, 2048), (513, 136, 2112), (513, 2056, 1088)])
+def test_gated_projection_on_either_side_of_short_sums(M, inter, K):
+    test_gated_projection_of_prompts(M, inter, K, 4)
+
+
 @pytest.mark.parametrize("M", [1, 2, 7, 8])
 @pytest.mark.parametrize("N,K,group,gated", [(48, 64, 64, False), (208, 192, 64, False), (2 * 48, 8192, 64, True), (1040, 4096, 128, False),
                                              (2 * 4112, 2048, 32, True), (16, 320, 16, False)])
