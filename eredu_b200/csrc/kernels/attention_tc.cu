@@ -539,7 +539,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       float l = 0.f;
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
-        if (s < nsplit && v[s].x > -INFINITY) {
+        // a part without a maximum and with a sum saw only scores that are no numbers: it makes the row one, as in the unsplit form
+        if (s < nsplit && (v[s].x > -INFINITY || v[s].y != 0.f)) {
           const float a = ex2_approx(v[s].x - top);
           float4 o;
           asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(mapa_shared(at, s)));

@@ -355,3 +355,24 @@ def test_experts_at_the_borders_of_the_rule(E, k, T, H, inter):
     ids, w = moe_ops.route(torch.randn(T, E, device=DEV), k, "softmax", True, 1.0, None, 1, 1)
     # the product of gate and up and every expert's row are rounded to bf16 on both sides, the sum on this one
     assert rel_l2(moe_ops.experts_forward(x, ids, w, gu, dn), moe_ops.experts_ref(x, ids, w, gu, dn)) < 2 * BF16
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_what_is_no_number_stays_none_when_keys_are_split(D):
+    """A query that is no number, and a cached key that is none: the rows that meet them, and no others."""
+    n_q, n_kv, new, kv = 32, 8, 20, 2000
+    pages = (kv + 15) // 16
+    kc, vc = (torch.randn(pages, n_kv, 16, D, device=DEV).bfloat16() for _ in range(2))
+    bt = torch.arange(pages, device=DEV, dtype=torch.int32)[None]
+    q = torch.randn(new, n_q, D, device=DEV).bfloat16()
+    lens, cu = torch.tensor([kv], device=DEV, dtype=torch.int32), torch.tensor([0, new], device=DEV, dtype=torch.int32)
+    clean = ops.attention_prefill(q, kc, vc, bt, lens, cu, new, D ** -0.5, max_kv_len=kv)
+    q[7, 3] = float("nan")
+    kc[(kv - 5) // 16, 6, (kv - 5) % 16] = float("nan")       # seen by the last five tokens, heads 24 to 27
+    want = torch.zeros(new, n_q, dtype=torch.bool, device=DEV)
+    want[7, 3] = True
+    want[new - 5:, 24:28] = True
+    for split in (0, kv):
+        got = ops.attention_prefill(q, kc, vc, bt, lens, cu, new, D ** -0.5, max_kv_len=split)
+        assert torch.equal(got.isnan().any(-1), want) and torch.equal(got.isnan().all(-1), want)
+        assert not split or torch.equal(got[~want], clean[~want])
