@@ -6,10 +6,10 @@
 //     operand, the token tile the MMA N operand);
 //   * the fp32 accumulator is double-buffered in TMEM (2 x 256 columns): while the epilogue warps drain tile i,
 //     the MMA warp already accumulates tile i+1;
-//   * a 4-stage TMA ring (48 KB per stage) runs ahead across tile boundaries;
+//   * a TMA ring runs ahead across tile boundaries: four stages of 48 KB, or ten of 18 KB for the expert items of decode steps;
 //   * the epilogue transposes through a 16 KB staging buffer so that Y leaves the SM as 16-byte row chunks;
-//   * grouped (MoE) form: the tiles come from a work table {expert, first row, rows, -} built on the device, an item of at most 256 rows
-//     each; a short item shortens the MMA and its copies (64 rows apiece) instead of fetching and multiplying rows nobody stores;
+//   * grouped (MoE) form: the tiles come from a work table {expert, first row, rows, -} built on the device, an item of at most 256 (16) rows
+//     each; a short item shortens the MMA and its copies (64 or 16 rows apiece) instead of fetching and multiplying rows nobody stores;
 //   * SwiGLU ("dual") tiles load 64 gate rows and 64 up rows into ONE 128-row operand tile, so gate and up use the
 //     same single 128x256 MMA stream as a plain GEMM; silu(gate) * up is formed when the staged rows are combined.
 //

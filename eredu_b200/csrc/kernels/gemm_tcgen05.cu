@@ -797,7 +797,7 @@ static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K,
   return static_cast<long long>(N) * K * 2 <= (M == 1 ? 24LL : 13LL) << 20;
 }
 
-// Number of K splits the launcher would use (exposed for tests and tuning).
+// K splits of a launch of [128 weight rows x tn tokens] tiles of which an SM takes ctas_per_sm.
 static int pick_split(int M, int N, int K, int tn, int ctas_per_sm, int sm_count) {
   if (tn > 64) return 1;
   const int tiles = ((N + 127) / 128) * ((M + tn - 1) / tn);
@@ -809,6 +809,8 @@ static int pick_split(int M, int N, int K, int tn, int ctas_per_sm, int sm_count
   return s;
 }
 
+// K splits of a GEMM with a collective in its epilogue (eredu_gemm_bf16_comm), for tests and tuning. A plain launch goes by its own tile: gated
+// tiles of 64 tokens count one CTA an SM, routers of prompts are not split, and one or two tokens may take the rows kernel.
 extern "C" int eredu_gemm_pick_split(int M, int N, int K, int sm_count) {
   const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   return pick_split(M, N, K, tn, 2, sm_count);

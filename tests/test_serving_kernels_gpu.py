@@ -376,3 +376,24 @@ def test_what_is_no_number_stays_none_when_keys_are_split(D):
         got = ops.attention_prefill(q, kc, vc, bt, lens, cu, new, D ** -0.5, max_kv_len=split)
         assert torch.equal(got.isnan().any(-1), want) and torch.equal(got.isnan().all(-1), want)
         assert not split or torch.equal(got[~want], clean[~want])
+
+
+@pytest.mark.parametrize("V", [32002, 128256])
+def test_largest_logit_among_what_is_none(V):
+    """Whole parts of a row that are masked, minus infinity or no number, and a row of nothing else."""
+    from eredu_b200.ops.sampling import SamplingParams, pack_rows
+
+    inf, nan = float("inf"), float("nan")
+    logits = torch.randn(6, V, device=DEV)
+    logits[0, :V - 10] = -inf
+    logits[1, 10:] = nan
+    logits[2] = -inf
+    logits[3] = nan
+    logits[4, V // 3] = inf
+    allow = torch.ones(6, V, dtype=torch.bool, device=DEV)
+    allow[5, :V - 100] = False
+    rows = torch.from_numpy(pack_rows([SamplingParams(temperature=0.0)] * 6, [1] * 6, hist_lens=[0] * 6, stream_ids=[0] * 6).view("u1").copy()).view(6, -1).to(DEV)
+    masks = torch.stack([ops.pack_allow_mask(a) for a in allow])
+    want = logits.masked_fill(~allow | logits.isnan(), -inf).argmax(-1)
+    want[2:4] = 0                                              # nothing is larger than the start of the search
+    assert torch.equal(ops.sample(logits.clone(), rows, allow=masks, all_greedy=True).long(), want)
