@@ -617,7 +617,8 @@ static int attn_prefill_tc_impl(const void* q, const void* k_cache, const void* 
   CUtensorMap tmQ, tmK, tmV;
   // Short portions (see SPLIT above the kernel): heads of 64 or 128, no chunks or pooled blocks, a context that the host has stated.
   // Up to eight splits (a portable cluster) while they find SMs of their own and two key tiles each - eight only on half of the SMs:
-  // a GPC does not always have room for two such clusters, and then the rest waits (33.6 us with 16 clusters, 18.5 with eight). The estimates
+  // a GPC does not always have room for two such clusters, and then the rest waits (33.6 us with 16 clusters, 18.5 with eight) - and four
+  // on seven eighths (three portions of 65 behind 1024, 32 heads over 4: 28.3 us with 36 clusters of four, 20.5 whole). The estimates
   // in us are what either form measured: start and end of a CTA, and a key tile; and, split, the exchange of a second tile of rows (four
   // sequences of 128 tokens behind 1024, 32 heads over 8, whole and split: heads of 128 19.5 and 22.9, heads of 64 16.7 and 17.7).
   int gshift = 0, nsplit = 1;
@@ -630,7 +631,7 @@ static int attn_prefill_tc_impl(const void* q, const void* k_cache, const void* 
     const long ctas = static_cast<long>(n_q_heads >> gshift) * ((max_q_len + tokens - 1) / tokens) * batch;
     const int seen = window > 0 ? std::min(max_kv_len, window + tokens + kTcTile) : max_kv_len;
     const int tiles = (seen + kTcTile - 1) / kTcTile;
-    while (nsplit < 8 && ctas * nsplit * 2 <= (nsplit < 4 ? sm : sm / 2) && tiles >= nsplit * 2 * 2) nsplit *= 2;
+    while (nsplit < 8 && ctas * nsplit * 2 <= (nsplit == 1 ? sm : nsplit == 2 ? sm * 7 / 8 : sm / 2) && tiles >= nsplit * 2 * 2) nsplit *= 2;
     const long whole = static_cast<long>(n_q_heads) * ((max_q_len + kTcRows - 1) / kTcRows) * batch;
     const double second = std::min(max_q_len, tokens) << gshift > kTcTile ? (key_dim == 128 ? 5.0 : 1.0) : 0.0;
     const double t_whole = ((whole + sm - 1) / sm) * (5.0 + 1.75 * tiles), t_split = 9.0 + second + 2.0 * ((tiles + nsplit - 1) / nsplit);

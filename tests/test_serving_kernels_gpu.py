@@ -397,3 +397,18 @@ def test_largest_logit_among_what_is_none(V):
     want = logits.masked_fill(~allow | logits.isnan(), -inf).argmax(-1)
     want[2:4] = 0                                              # nothing is larger than the start of the search
     assert torch.equal(ops.sample(logits.clone(), rows, allow=masks, all_greedy=True).long(), want)
+
+
+@pytest.mark.parametrize("new", [64, 65])
+@pytest.mark.parametrize("kv", [1024 + 65, 4096 + 65])
+def test_short_portions_on_either_side_of_a_cluster(new, kv):
+    """Three portions of heads in groups of eight: 24 tiles of rows, which four CTAs share, and 36, for which clusters of four have no room."""
+    n_q, n_kv, D, B = 32, 4, 128, 3
+    pages = (kv + 15) // 16
+    kc, vc = (torch.randn(B * pages, n_kv, 16, D, device=DEV).bfloat16() for _ in range(2))
+    bt = torch.randperm(B * pages, device=DEV).int().view(B, pages)
+    q = torch.randn(B * new, n_q, D, device=DEV).bfloat16()
+    lens, cu = torch.full((B,), kv, device=DEV, dtype=torch.int32), torch.arange(B + 1, device=DEV, dtype=torch.int32) * new
+    whole = ops.attention_prefill(q, kc, vc, bt, lens, cu, new, D ** -0.5)
+    # probabilities are rounded to bf16 in front of the second product on both sides, against different maxima, and outputs once more
+    assert rel_l2(ops.attention_prefill(q, kc, vc, bt, lens, cu, new, D ** -0.5, max_kv_len=kv), whole) < 2 * BF16
