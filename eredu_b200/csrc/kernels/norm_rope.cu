@@ -488,11 +488,12 @@ extern "C" int eredu_rope_kv(const void* qkv, void* q_out, void* k_cache, void* 
   // 16-byte pieces: heads and rotated parts of whole pairs of pieces, rows and pages on 16-byte boundaries. Everything else (and
   // angles that do not fit the shared table) keeps the kernel with 2-byte accesses.
   // And few tokens: its CTAs, one per token and head, end before one CTA has walked all heads of a token. Its time goes with tokens times
-  // heads (0.7 us and 1.05 per 1000), that of 16-byte pieces with the width of a token (1.7 us and 0.02 per head of 128, 1.2 more
-  // with norms): one token of 80 heads 1.8 against 3.3 us, 64 tokens of 40 heads with norms 3.4 against 3.8, of 48 without 3.9 against 2.6.
+  // heads (0.7 us and 1.05 per 1000), that of 16-byte pieces with the width of a token (1.7 us and 0.02 per head of 128; with norms
+  // 1.2 and 0.01 per head more): one token of 80 heads 1.8 against 3.3 us, 48 of them with norms 4.7 against 5.2, 64 tokens of 40 heads with norms 3.4 against 3.8, of 48 without 3.9 against 2.6.
   const auto aligned = [](const void* t) { return (reinterpret_cast<uintptr_t>(t) & 15) == 0; };
   const int heads = n_q + 2 * n_kv;
-  const bool many = static_cast<long long>(M) * heads > 960 + 20 * heads * D / 128 + (q_norm_w != nullptr || k_norm_w != nullptr ? 1152 : 0);
+  const bool norms = q_norm_w != nullptr || k_norm_w != nullptr;
+  const bool many = static_cast<long long>(M) * heads > 960 + (norms ? 1152 : 0) + (norms ? 28 : 20) * heads * D / 128;
   if (many && (D == 64 || D == 128) && rot % 16 == 0 && ld % 8 == 0 && aligned(qkv) && aligned(q_out) && aligned(k_cache) &&
       aligned(v_cache))
     launch_pdl(rope_kv_rows_kernel, dim3(M), dim3(kRopeThreads), 0, stream, p, __builtin_ctz(static_cast<unsigned>(D)) - 4);

@@ -45,9 +45,9 @@ def test_rotation_and_append_rows(M, n_q, n_kv, D, rot, interleaved):
     assert torch.equal(vc, vr)
 
 
-@pytest.mark.parametrize("M", [125, 126])
+@pytest.mark.parametrize("M", [125, 126, 133, 134])
 def test_rotation_of_few_tokens(M):
-    """On either side of where a token has a CTA of its own (20 heads of 128 with norms: from 126 tokens on)."""
+    """On either side of where a token has a CTA of its own (20 heads of 128 with norms: from 134 tokens on)."""
     test_rotation_and_append_rows(M, 16, 2, 128, 128, False)
 
 
