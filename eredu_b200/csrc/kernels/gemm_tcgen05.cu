@@ -782,8 +782,8 @@ static bool staged_epilogue_ok(const void* Y, const void* residual, int N, int l
 // 2048 5.8 -> 4.5 us, 6144 x 4096 12.2 -> 10.9, 4096 x 14336 21.3 -> 20.4), but in a decode step, behind other kernels, the copy
 // rings of the tensor-core kernel start with 160 KB an SM where this one holds 64 KB a CTA: taking matrices up to 16 MB makes a
 // step of 16 layers 2048 wide 766 -> 728 us, up to 24 MB one of 8 expert layers 672 -> 628; 33 MB and above lose it again (759 us, and
-// 912 -> 945 for 8 layers 4096 wide). Two tokens are twice the arithmetic on the CUDA cores: 3072 x 2048 5.7 -> 5.1 us, 5120 x 2048
-// 6.8 -> 7.8.
+// 912 -> 945 for 8 layers 4096 wide). Two tokens are twice the arithmetic on the CUDA cores: 3072 x 2048 5.7 -> 5.1 us, 2560 x 2560
+// 6.2 -> 6.6, 5120 x 2048 6.8 -> 7.8.
 // Its CTAs have to run in one round, two to an SM: of short rows a second round costs more than the tensor-core kernel (5120 x 512 4.3
 // us there, 4.8 here; 12288 x 512 5.5 and 8.1); one token with rows of 2048 still gains (5120 x 2048 7.1 -> 6.7). With sums of squares
 // clusters of eight leave part of a GPC empty: one round is 7/8 of that, three quarters for two tokens (4608 x 512 4.3 and 6.3, 4096 x 512 with
@@ -794,7 +794,7 @@ static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K,
   if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) != 0) return false;
   const int ctas = N / kRowsOut, round = 2 * (sm_count > 0 ? sm_count : 148);
   if (ssq ? ctas > round || (K < 1024 && ctas * 8 > round * (M == 1 ? 7 : 6)) : ctas > round && (M > 1 || K < 2048)) return false;
-  return static_cast<long long>(N) * K * 2 <= (M == 1 ? 24LL : 13LL) << 20;
+  return static_cast<long long>(N) * K * 2 <= (M == 1 ? 24LL : 12LL) << 20;
 }
 
 // K splits of a launch of [128 weight rows x tn tokens] tiles of which an SM takes ctas_per_sm.

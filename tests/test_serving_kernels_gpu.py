@@ -185,7 +185,7 @@ def test_rows_of_one_and_two_tokens(M, N, K):
 
 
 @pytest.mark.parametrize("M", [1, 2])
-@pytest.mark.parametrize("N,K", [(4736, 64), (4752, 64), (4144, 1016), (4160, 1016), (4736, 1024), (3552, 512), (3568, 512)])
+@pytest.mark.parametrize("N,K", [(4736, 64), (4752, 64), (4144, 1016), (4160, 1016), (4736, 1024), (3552, 512), (3568, 512), (3072, 2048), (3088, 2048)])
 def test_rows_of_one_and_two_tokens_at_the_borders_of_a_round(M, N, K):
     test_rows_of_one_and_two_tokens(M, N, K)
 
