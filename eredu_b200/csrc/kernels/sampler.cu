@@ -194,13 +194,14 @@ __global__ void __launch_bounds__(kSampThreads) sampler_kernel(SamplerParams p) 
 
   pdl_launch_early();
   trace_mark(kTraceSampler, kTraceStart);
-  cluster_arrive_relaxed();         // waited for in front of the exchange below, when its result has long been there
-  pdl_wait();
-  trace_mark(kTraceSampler, kTraceAfterWait);
-  pdl_launch_dependents();
   uint32_t rank, nrank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(nrank));
+  // waited for in front of the exchange below, when its result has long been there; a row with one CTA has none of the cluster's barriers
+  if (nrank > 1) cluster_arrive_relaxed();
+  pdl_wait();
+  trace_mark(kTraceSampler, kTraceAfterWait);
+  pdl_launch_dependents();
   const int r = blockIdx.x / nrank;
   const int tid = threadIdx.x;
   SamplerRow cfg;
@@ -239,11 +240,15 @@ __global__ void __launch_bounds__(kSampThreads) sampler_kernel(SamplerParams p) 
         row[tok] = x;
       }
     }
-    __syncwarp();
-    cluster_wait_acquire();
-    cluster_arrive_release();
-    cluster_wait_acquire();
-    cluster_arrive_relaxed();
+    if (nrank > 1) {
+      __syncwarp();
+      cluster_wait_acquire();
+      cluster_arrive_release();
+      cluster_wait_acquire();
+      cluster_arrive_relaxed();
+    } else {
+      __syncthreads();
+    }
   }
 
   // ---- 2. max / argmax (the greedy answer; also the softmax shift)
@@ -274,14 +279,20 @@ __global__ void __launch_bounds__(kSampThreads) sampler_kernel(SamplerParams p) 
       }
     }
   } else {
-    for (int i = begin + tid; i < end; i += kSampThreads) {
-      const float x = load_logit(p, row, allow, i);
-      if (x > vmax) { vmax = x; imax = i; }
+    // eight loads on their way: 200 rows of 50257 14.3 us with a comparison behind every load, 10.7 with these
+    constexpr int kBatch = 8;
+    for (int i0 = begin + tid; i0 < end; i0 += kBatch * kSampThreads) {
+      float x[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) x[b] = i0 + b * kSampThreads < end ? load_logit(p, row, allow, i0 + b * kSampThreads) : -INFINITY;
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b)
+        if (x[b] > vmax) { vmax = x[b]; imax = i0 + b * kSampThreads; }
     }
   }
   block_argmax(vmax, imax, scr);
-  cluster_wait_acquire();           // every CTA of the cluster has started: its shared memory may be written
   if (nrank > 1) {
+    cluster_wait_acquire();           // every CTA of the cluster has started: its shared memory may be written
     if (tid == 0) {
       const uint32_t at = mapa_shared(smem_u32(&part[rank]), 0u);
       asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_int(vmax)), "r"(imax) : "memory");
