@@ -1,4 +1,5 @@
-// Decode-regime quantised linear layer: Y[M,N] = X[M,K] · dequant(Wq)[N,K]^T for M <= 8 tokens and 4-bit affine weights.
+// Decode-regime quantised linear layer: Y[M,N] = X[M,K] · dequant(Wq)[N,K]^T for M <= 8 tokens and 4-bit affine weights (one and two
+// tokens of larger matrices: qgemv_stream.cu).
 //
 // With so few tokens the layer is a stream over the packed weights (0.5 B per weight), and what matters is that nothing
 // but HBM sits on the critical path. This kernel therefore keeps the weights in registers from the load to the tensor
@@ -32,6 +33,7 @@
 #include "../common/peer.cuh"
 #include "../common/ptx.cuh"
 #include "../common/trace.cuh"
+#include "qgemv_stream.h"
 
 namespace eredu {
 
@@ -550,6 +552,28 @@ extern "C" int eredu_qgemv4(const void* X, const void* wq, const void* dq, void*
     if (static_cast<long long>((M + 1) / 2) * N * 4 > pc->lam_bytes) return -2;
     p.use_comm = 1;
     p.comm = *pc;
+  }
+  // One or two tokens of larger matrices: the persistent kernel on integer products (force_wk = -1, with force_ns: always; -2: never)
+  if (group >= 64 && force_exact_bf16 == 0 && comm == nullptr && M <= kQGemvStreamTokens && (force_wk == -1 || (force_wk == 0 && force_ns == 0))) {
+    QGemvStreamParams q = {};
+    q.x = p.x;
+    q.wq = p.wq;
+    q.dq = p.dq;
+    q.y = p.y;
+    q.residual = p.residual;
+    q.bias = p.bias;
+    q.M = p.M;
+    q.n_out = p.n_out;
+    q.ldx = p.ldx;
+    q.ldy = p.ldy;
+    q.ldr = p.ldr;
+    q.group_shift = p.group_shift;
+    q.kblocks = p.kblocks;
+    q.out_fp32 = p.out_fp32;
+    q.limit = p.limit;
+    q.status = p.status;
+    const int r = launch_qgemv_stream(q, gated != 0, force_wk == -1 ? std::max(1, force_ns) : 0, sm_count, stream);
+    if (r != kQGemvStreamUnsupported) return r;
   }
   // Row tiles of a warp and K splits. Four tiles take the fewest instructions per row and win wherever the kernel is bound by issue; a matrix
   // that gives the SMs only a round of CTAs, or less, is bound by the first copies and the end of each, and wants more and smaller ones:

@@ -121,6 +121,29 @@ def test_four_bit_rows_at_the_borders_of_the_plan(M, N, K, group, gated):
     test_four_bit_rows_of_few_tokens(M, N, K, group, gated)
 
 
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("N,K,group,gated", [(4752, 3072, 64, False), (4736, 3072, 64, False), (4744, 5120, 128, False), (2 * 4736, 3136, 64, True),
+                                             (2848, 10240, 64, False), (2848, 10496, 128, False), (2832, 10240, 64, False), (4752, 17600, 64, False), (2 * 2384, 17664, 64, True),
+                                             (71040, 128, 64, False), (35520, 960, 64, False)])
+@pytest.mark.parametrize("decades", [0, 6])
+def test_four_bit_rows_on_integer_products(M, N, K, group, gated, decades):
+    """On either side of where one or two tokens take the persistent kernel, with and without a split of K; row tiles that are no whole rounds,
+    K blocks that leave warps without any; activations of one size and over six decades; rows that are part of wider ones."""
+    ql = QuantLinear.from_dense((torch.randn(N, K, device=DEV) * 0.05).bfloat16(), 4, group)
+    x = torch.randn(M, K + 8, device=DEV) * 10.0 ** (torch.rand(M, K + 8, device=DEV) * decades - decades / 2)
+    x = x.bfloat16()[:, :K]
+    y = x.double() @ ql.dequantize(torch.float32).double().t()
+    res = torch.randn(M, N, device=DEV).bfloat16()
+    ref = moe_ops.gated_act_ref(y[:, :N // 2].float(), y[:, N // 2:].float()) if gated else (y + res.double()).float()
+    got = ql.gated(x) if gated else ql(x, residual=res)
+    assert rel_l2(got, ref) < BF16
+    if not gated:
+        # fp32 results: a block's numbers are kept to 2^-21 of its largest, and 64 of them times at most 15 steps around zero are summed in fp32
+        assert rel_l2(ql(x, out_dtype=torch.float32), y) < 2.0 ** -18
+    x[0, K - 5] = float("inf")
+    assert bool(torch.isnan(ql.gated(x) if gated else ql(x)).all(-1)[0]) and (M == 1 or bool(torch.isfinite(ql(x)[1]).all()))
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 5, 64])
 @pytest.mark.parametrize("H,inter", [(256, 96), (2048, 768)])
 def test_experts_of_few_tokens(T, H, inter):
