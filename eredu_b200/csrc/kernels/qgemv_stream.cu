@@ -16,7 +16,7 @@
 // A block that holds an infinity or a NaN makes its token's results NaN, as the bf16 form does (128 + code and its correction cancel there).
 // Errors against 64 bits (2-norm): 1.1e-7 of normal activations (bf16 form 1.3e-6), 1.3e-6 of activations over nine decades (1.9e-6).
 //
-// One CTA of sixteen warps per SM (eight left the chains of a warp exposed: gate_up 69 us instead of 56 before the loops were trimmed), or a
+// One CTA of sixteen warps per SM (eight left the chains of a warp exposed: gate_up 69 us instead of 56 before the loops were trimmed, 45 now), or a
 // cluster of ns that splits K, walks a run of 16-row tiles. The activations are turned into bytes once per CTA, in shared memory, in the
 // order in which lanes meet them; every warp has a K range of its own and a private ring of bulk copies that runs on across the rounds of
 // four tiles (of a gated matrix two gate and two up tiles), so that HBM does not wait for the sum over warps and CTAs at the end of a round.
@@ -31,7 +31,6 @@
 #include "../common/launch.h"
 #include "../common/launch_count.h"
 #include "../common/ptx.cuh"
-#include "../common/trace.cuh"
 
 namespace eredu {
 
@@ -39,6 +38,7 @@ namespace {
 
 constexpr int kWarps = 16, kThreads = 32 * kWarps;
 constexpr int kTiles = 4;                 // row tiles of a round
+constexpr int kChunk = 2;                 // K blocks of a slot
 constexpr int kMaxSlots = 4;
 constexpr float kMagic = 12582912.f;      // 1.5 * 2^23
 constexpr uint32_t kMagicBits = 0x4B400000u;
@@ -47,10 +47,8 @@ constexpr int kCtrlBytes = 1024;          // [16 warps][kMaxSlots] ring barriers
 
 // of a K block: three pieces of M tokens, then four float4 {X, X, sum, sum}
 __host__ __device__ constexpr int x_block_bytes(int M) { return 3 * 64 * M + 64; }
-__host__ __device__ constexpr int dq_slot_bytes(int chunk, int group_shift) {
-  return ((chunk * 64 >> group_shift) > 0 ? (chunk * 64 >> group_shift) : 1) * 64;
-}
-__host__ __device__ constexpr int slot_bytes(int chunk, int group_shift) { return kTiles * (chunk * 512 + dq_slot_bytes(chunk, group_shift)); }
+__host__ __device__ constexpr int dq_slot_bytes(int group_shift) { return (kChunk * 64 >> group_shift) * 64; }
+__host__ __device__ constexpr int slot_bytes(int group_shift) { return kTiles * (kChunk * 512 + dq_slot_bytes(group_shift)); }
 __host__ __device__ constexpr int round_rows(bool gated) { return (gated ? kTiles / 2 : kTiles) * 16; }
 __host__ __device__ constexpr int red_plane(bool gated, int tokens) { return (gated ? 2 : 1) * tokens * (round_rows(gated) + 4); }   // floats of a warp
 __host__ __device__ constexpr int recv_floats(bool gated, int tokens) { return (gated ? 2 : 1) * tokens * round_rows(gated); }       // of a round, all ranks
@@ -115,12 +113,11 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
   uint64_t* xbars = bars + kWarps * kMaxSlots;                         // [2]
   float* red = reinterpret_cast<float*>(smem + kCtrlBytes);            // [2][16 warps][PLANE]
   float* recv = red + 2 * kWarps * PLANE;                              // [2][ns ranks][S][TOK][cols] (clusters)
-  const int slot_size = slot_bytes(p.chunk, p.group_shift);
+  const int slot_size = slot_bytes(p.group_shift);
   uint8_t* ring = reinterpret_cast<uint8_t*>(recv + (p.ns > 1 ? 2 * recv_floats(GATED, TOK) : 0));   // [16 warps][slots]
   uint8_t* xs = ring + kWarps * p.slots * slot_size;                   // [kb_cta][XSTRIDE]
 
   pdl_launch_early();
-  trace_mark(kTraceQGemm, kTraceStart);
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -132,7 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
   const int rounds = (u1 - u0 + RT - 1) / RT;
   const int kbc0 = min(static_cast<int>(crank) * p.kb_cta, p.kblocks), kbc1 = min(kbc0 + p.kb_cta, p.kblocks);
   const int kb0 = min(kbc0 + warp * p.kb_warp, kbc1), kb1 = min(kb0 + p.kb_warp, kbc1);
-  const int C = p.chunk;
+  constexpr int C = kChunk;
   const int cols = ROWS / p.ns;                                        // output columns of a round that this CTA finishes
 
   uint8_t* my_ring = ring + warp * p.slots * slot_size;
@@ -152,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
   // lane s < T copies the codes of tile s of a round, lane T + s its (scale, bias) words; the copies run on across rounds
   const bool copies_dq = lane >= T;
   const int cs = lane % T;
-  const int dq_slot = dq_slot_bytes(C, p.group_shift);                 // of a tile
+  const int dq_slot = dq_slot_bytes(p.group_shift);                 // of a tile
   const size_t tile_bytes = copies_dq ? (static_cast<size_t>(p.kblocks) * 64 >> p.group_shift) * 64 : static_cast<size_t>(p.kblocks) * 512;
   const uint8_t* csrc = (copies_dq ? reinterpret_cast<const uint8_t*>(p.dq) : p.wq) +
                         static_cast<size_t>(u0 + cs % RT + (cs / RT) * p.units) * tile_bytes;       // GATED: the up tiles follow the gate tiles
@@ -185,7 +182,6 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
   for (int i = 0; i < p.slots; ++i) issue();
 
   pdl_wait();
-  trace_mark(kTraceQGemm, kTraceAfterWait);
   pdl_launch_dependents();
 
   // ---- activations of this CTA's K blocks: four lanes per token and block, 16 values each
@@ -326,8 +322,9 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
       const uint8_t* slot = my_ring + slot_i * slot_size;
       const uint32_t* dqs = reinterpret_cast<const uint32_t*>(slot + T * C * 512) + g;
       const int nb = min(C, kb1 - kb);
-#pragma unroll 1
-      for (int j = 0; j < nb; ++j, xb += XSTRIDE) block(slot + j * 512 + code_off, dqs + ((j * 64) >> p.group_shift) * 16, xb);
+      block(slot + code_off, dqs, xb);
+      if (nb == 2) block(slot + 512 + code_off, dqs + (64 >> p.group_shift) * 16, xb + XSTRIDE);
+      xb += 2 * XSTRIDE;
       __syncwarp();                                 // every lane has read this slot
       issue();
       if (++slot_i == p.slots) {
@@ -388,12 +385,11 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
     cluster_arrive_release();
     cluster_wait_acquire();
   }
-  trace_mark(kTraceQGemm, kTraceEnd);
 }
 
-int smem_bytes(const QGemvStreamParams& p, bool gated, int ns, int kb_cta, int chunk, int slots) {
+int smem_bytes(const QGemvStreamParams& p, bool gated, int ns, int kb_cta, int slots) {
   return kCtrlBytes + 2 * kWarps * red_plane(gated, p.M) * 4 + (ns > 1 ? 2 * recv_floats(gated, p.M) * 4 : 0) +
-         kWarps * slots * slot_bytes(chunk, p.group_shift) + kb_cta * x_block_bytes(p.M);
+         kWarps * slots * slot_bytes(p.group_shift) + kb_cta * x_block_bytes(p.M);
 }
 
 template <bool GATED, int TOK>
@@ -436,21 +432,20 @@ cudaError_t launch(const QGemvStreamParams& p, int clusters, int smem, cudaStrea
 
 // Where this kernel takes a matrix, and over how many CTAs it splits K; 0: the register kernel. Turning the activations into bytes, the larger
 // CTAs and their barriers cost about a microsecond, so that it takes several row tiles an SM and long rows to pay. Microseconds of one token,
-// register kernel -> this one (K blocks x row tiles an SM): 57344 x 8192 gated (128 x 24) 67.5 -> 47.9, 10240 x 8192 19.3 -> 14.9, 8192 x 8192
-// 11.4 -> 9.8, 28672 x 4096 gated (64 x 12) 19.7 -> 16.6, 14336 x 4096 gated (64 x 6) 10.7 -> 10.4, 8192 x 3584 (56 x 3.5) 6.6 -> 6.3, 5120 x 5120
-// (80 x 2.2) 8.6 -> 7.3, 4864 x 3072 (48 x 2.1) 6.1 -> 5.2, 36864 x 2048 (32 x 16) 11.6 -> 11.3, 128256 x 2048 43 -> 31; but 4096 x 4096 (64 x 1.7)
-// 4.7 / 5.7, 4736 x 5120 (80 x 2.0) 6.1 / 7.1, 16384 x 2048 gated (32 x 7) 6.6 / 6.9, 35520 x 1024 (16 x 15) 6.8 / 7.9.
-// Two CTAs that split K: where one has no room for the activations (8192 x 28672: 35.2 -> 28.0), and where the row tiles are between one and two an
-// SM and long (4096 x 11008: 10.8 -> 9.3, 2848 x 16384: 13.4 -> 10.3; 2848 x 8192 7.5 / 7.3, 2048 x 8192 6.4 / 7.0).
-// Two tokens take more fmas: 28672 x 4096 gated 19.7 -> 18.3, 10240 x 8192 19.4 -> 16.6, 5120 x 5120 8.7 -> 8.3, 4096 x 14336 12.9 -> 11.8; but 16384 x
-// 4096 (64 x 7) 10.8 / 11.2, 36864 x 2048 11.9 / 12.8, 8192 x 3584 7.1 / 7.1, 8192 x 28672 (two CTAs, 3.5 tiles) 35.5 / 35.5.
+// register kernel -> this one (K blocks x row tiles an SM): 57344 x 8192 gated (128 x 24) 67.5 -> 44.8, 10240 x 8192 19.3 -> 13.4, 8192 x 8192
+// 11.4 -> 9.0, 28672 x 4096 gated (64 x 12) 19.7 -> 15.4, 14336 x 4096 gated (64 x 6) 10.7 -> 9.7, 8192 x 3584 (56 x 3.5) 6.6 -> 5.9, 5120 x 5120
+// (80 x 2.2) 8.6 -> 6.6, 4864 x 3072 (48 x 2.1) 6.2 -> 4.8, 36864 x 2048 (32 x 16) 11.6 -> 10.5, 128256 x 2048 43 -> 29; but 4096 x 4096 (64 x 1.7)
+// 4.7 / 5.2, 4736 x 5120 (80 x 2.0) 6.1 / 6.5, 12288 x 2048 (32 x 5) 6.0 / 6.1, 35520 x 1024 (16 x 15) 6.8 / 7.5.
+// Two CTAs that split K: where one has no room for the activations (8192 x 28672: 35.2 -> 25.7), and where the row tiles are between one and two an
+// SM and long (4096 x 11008: 10.8 -> 8.6, 2848 x 16384: 13.4 -> 9.4, 3072 x 8192: 8.0 -> 6.7; 2048 x 8192 6.4 / 6.4).
+// Two tokens take more fmas: 28672 x 4096 gated 19.7 -> 17.7, 10240 x 8192 19.4 -> 15.8, 5120 x 5120 8.7 -> 7.7, 4096 x 14336 12.9 -> 11.2, 16384 x
+// 4096 (64 x 7) 10.8 -> 10.6; but 14336 x 4096 gated (64 x 6) 10.7 / 11.0, 36864 x 2048 11.9 / 12.2.
 static int pick_splits(const QGemvStreamParams& p, bool gated, int sms) {
   const double tiles = static_cast<double>(p.units) * (gated ? 2 : 1) / sms;
-  const bool room = smem_bytes(p, gated, 1, (p.kblocks + 1) / 2 * 2, 2, 2) <= kMaxSmem;
-  if (tiles <= 2) return tiles >= 1.2 && p.kblocks >= 160 ? 2 : 0;
-  if (!room) return p.M == 1 || tiles >= 6 ? 2 : 0;
-  if (p.M == 1) return p.kblocks >= 48 || p.kblocks * tiles >= 480 ? 1 : 0;
-  return p.kblocks >= 80 || p.kblocks * tiles >= (p.kblocks >= 48 ? 480 : 1000) ? 1 : 0;
+  if (tiles <= 2) return tiles >= 1.2 && p.kblocks >= 128 ? 2 : 0;
+  if (smem_bytes(p, gated, 1, (p.kblocks + 1) / 2 * 2, 2) > kMaxSmem) return 2;
+  if (p.kblocks >= (p.M == 1 ? 48 : 80)) return 1;
+  return p.kblocks * tiles >= (p.M == 1 ? 480 : p.kblocks >= 48 ? 440 : 1000) ? 1 : 0;
 }
 
 int launch_qgemv_stream(QGemvStreamParams p, bool gated, int force_ns, int sm_count, cudaStream_t stream) {
@@ -459,14 +454,13 @@ int launch_qgemv_stream(QGemvStreamParams p, bool gated, int force_ns, int sm_co
   p.units = (p.n_out + 15) / 16;
   p.ns = force_ns > 0 ? force_ns : pick_splits(p, gated, sms);
   if (p.ns == 0) return kQGemvStreamUnsupported;
-  p.chunk = 2;
-  p.kb_cta = ((p.kblocks + p.ns - 1) / p.ns + p.chunk - 1) / p.chunk * p.chunk;          // starts on a group
-  if (p.ns > 8 || (p.ns & (p.ns - 1)) != 0 || smem_bytes(p, gated, p.ns, p.kb_cta, p.chunk, 2) > kMaxSmem) return kQGemvStreamUnsupported;
+  p.kb_cta = ((p.kblocks + p.ns - 1) / p.ns + kChunk - 1) / kChunk * kChunk;          // starts on a group
+  if (p.ns > 8 || (p.ns & (p.ns - 1)) != 0 || smem_bytes(p, gated, p.ns, p.kb_cta, 2) > kMaxSmem) return kQGemvStreamUnsupported;
   const int clusters = std::min(p.units, std::max(1, (p.ns > 2 ? sms * 7 / 8 : sms) / p.ns));     // clusters of more than two find seven eighths of the SMs
-  p.kb_warp = ((p.kb_cta + kWarps - 1) / kWarps + p.chunk - 1) / p.chunk * p.chunk;   // a warp's slots start on a group
+  p.kb_warp = ((p.kb_cta + kWarps - 1) / kWarps + kChunk - 1) / kChunk * kChunk;   // a warp's slots start on a group
   p.slots = 2;
-  while (p.slots < kMaxSlots && smem_bytes(p, gated, p.ns, p.kb_cta, p.chunk, p.slots + 1) <= kMaxSmem) ++p.slots;
-  const int smem = smem_bytes(p, gated, p.ns, p.kb_cta, p.chunk, p.slots);
+  while (p.slots < kMaxSlots && smem_bytes(p, gated, p.ns, p.kb_cta, p.slots + 1) <= kMaxSmem) ++p.slots;
+  const int smem = smem_bytes(p, gated, p.ns, p.kb_cta, p.slots);
   cudaError_t e;
   if (p.M == 1) e = gated ? launch<true, 1>(p, clusters, smem, stream) : launch<false, 1>(p, clusters, smem, stream);
   else e = gated ? launch<true, 2>(p, clusters, smem, stream) : launch<false, 2>(p, clusters, smem, stream);
@@ -475,5 +469,3 @@ int launch_qgemv_stream(QGemvStreamParams p, bool gated, int force_ns, int sm_co
 }
 
 }  // namespace eredu
-
-EREDU_TRACE_INSTALLER(qgemv_stream)

@@ -28,7 +28,7 @@ struct QGemvStreamParams {
   int units;            // tiles of 16 output rows
   int kb_cta, kb_warp;  // K blocks of a CTA of the cluster, and of a warp
   int ns;               // CTAs of a cluster, which split K
-  int chunk, slots;     // K blocks of a slot of a warp's ring, and slots
+  int slots;            // of a warp's ring
 };
 
 int launch_qgemv_stream(QGemvStreamParams p, bool gated, int force_ns, int sm_count, cudaStream_t stream);

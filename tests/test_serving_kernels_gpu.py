@@ -123,7 +123,7 @@ def test_four_bit_rows_at_the_borders_of_the_plan(M, N, K, group, gated):
 
 @pytest.mark.parametrize("M", [1, 2])
 @pytest.mark.parametrize("N,K,group,gated", [(4752, 3072, 64, False), (4736, 3072, 64, False), (4744, 5120, 128, False), (2 * 4736, 3136, 64, True),
-                                             (2848, 10240, 64, False), (2848, 10496, 128, False), (2832, 10240, 64, False), (4752, 17600, 64, False), (2 * 2384, 17664, 64, True),
+                                             (2848, 8192, 64, False), (2848, 8448, 128, False), (2832, 8192, 64, False), (4752, 17600, 64, False), (2 * 2384, 17664, 64, True),
                                              (71040, 128, 64, False), (35520, 960, 64, False)])
 @pytest.mark.parametrize("decades", [0, 6])
 def test_four_bit_rows_on_integer_products(M, N, K, group, gated, decades):
