@@ -3,10 +3,14 @@
 // next norm), built so that the tensor cores never wait for an epilogue:
 //
 //   * one CTA per SM walks a list of [128 weight rows x up to 256 tokens] tiles (swap-AB: the weight tile is the MMA M
-//     operand, the token tile the MMA N operand);
+//     operand, the token tile the MMA N operand); dense matrices with sums of some length go to pairs of CTAs (cta_group::2), which share
+//     [256 x up to 256] tiles: a CTA fetches its 128 weight rows and half of the tokens, 32 KB a stage instead of 48, and has six stages;
+//   * the warps that fetch and multiply run their loops whole, and one elected lane issues (see elect_one in ptx.cuh). 2048 tokens, one
+//     CTA with a lane of its own / elected / pairs: 4096 x 14336 210 / 210 / 174 us, 2 x 14336 x 4096 404 / 402 / 326, 300 tokens, 8192 x 8192
+//     55.7 / 55.1 / 46;
 //   * the fp32 accumulator is double-buffered in TMEM (2 x 256 columns): while the epilogue warps drain tile i,
 //     the MMA warp already accumulates tile i+1;
-//   * a TMA ring runs ahead across tile boundaries: four stages of 48 KB, or ten of 18 KB for the expert items of decode steps;
+//   * a TMA ring runs ahead across tile boundaries: six stages of 32 KB, four of 48 KB, or ten of 18 KB for the expert items of decode steps;
 //   * the epilogue transposes through a 16 KB staging buffer so that Y leaves the SM as 16-byte row chunks;
 //   * grouped (MoE) form: the tiles come from a work table {expert, first row, rows, -} built on the device, an item of at most 256 (16) rows
 //     each; a short item shortens the MMA and its copies (64 or 16 rows apiece) instead of fetching and multiplying rows nobody stores;
@@ -33,15 +37,16 @@ namespace {
 constexpr int kTN = 256;                         // tokens per tile (MMA N)
 constexpr int kATile = 128 * 64 * 2;             // 16 KB: 128 weight rows x 64 k
 constexpr int kBTile = kTN * 64 * 2;             // 32 KB: 256 tokens x 64 k
-constexpr int kTileFixed = 268;                  // of a tile's time, in token rows
 constexpr int kBand = 8;                         // token tiles that vary fastest
 // Stages of the ring. BOX: grouped form, token rows of one copy - 64, or 16 for the items of a decode step (at most 16 rows): such a step
 // streams the weights of nearly all experts, and what counts are the bytes on their way, 160 KB an SM with ten small stages.
+// kPair: two CTAs share a tile, half of its tokens in the shared memory of each.
+constexpr int kPair = 128;
 template <int BOX>
 struct Ring {
   static constexpr int kBoxBytes = BOX * 64 * 2;
-  static constexpr int kStageBytes = kATile + (BOX == 16 ? kBoxBytes : kBTile);    // 18 or 48 KB
-  static constexpr int kStages = BOX == 16 ? 10 : 4;
+  static constexpr int kStageBytes = kATile + (BOX == 16 ? kBoxBytes : BOX == kPair ? kBTile / 2 : kBTile);    // 18, 32 or 48 KB
+  static constexpr int kStages = BOX == 16 ? 10 : BOX == kPair ? 6 : 4;
 };
 constexpr int kStagingBytes = 16 * 1024;
 constexpr int kCtrlBytes = 1024;
@@ -65,6 +70,7 @@ struct PGemmParams {
   float act_a, act_b;  // xIELU
   int act;  // plain tiles: 2 = squared ReLU before the residual, 4 = xIELU; dual tiles: 0 = silu(g) * u, 3 = relu(g) * u
   int n_tiles, m_tiles;
+  int ssq_stride;  // tiles of 128 output columns
   int tn;  // token rows of a tile: 256, or fewer where that saves a round of tiles
   // grouped form: m_tiles work items, used ones first (the rest have no rows); the expert's weights start at row expert * w_rows_per_expert
   const int4* work;
@@ -76,8 +82,8 @@ struct PTile {
 };
 
 // Tile t of the list; false behind the last one.
-template <bool GROUPED, int ROWS>
-__device__ __forceinline__ bool tile_at(const PGemmParams& p, int t, PTile& o) {
+template <bool GROUPED, int ROWS, bool PAIR>
+__device__ __forceinline__ bool tile_at(const PGemmParams& p, int t, uint32_t crank, PTile& o) {
   int tile_m = t / p.n_tiles;
   o.tile_n = t % p.n_tiles;
   if (!GROUPED) {
@@ -90,6 +96,7 @@ __device__ __forceinline__ bool tile_at(const PGemmParams& p, int t, PTile& o) {
     tile_m = band * kBand + in % height;
     o.tile_n = in / height;
   }
+  if (PAIR) o.tile_n = 2 * o.tile_n + static_cast<int>(crank);
   o.w_row0 = o.tile_n * ROWS;
   if (GROUPED) {
     const int4 item = p.work[tile_m];
@@ -124,11 +131,15 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   __shared__ float s_scale[kTN];
   __shared__ int s_fail;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int kblocks = (p.K + 63) >> 6;
   const int total = p.n_tiles * p.m_tiles;
-  constexpr int kRowsPerTile = DUAL ? 64 : 128;  // output columns (weight rows of the result) per tile
+  constexpr int kRowsPerTile = DUAL ? 64 : 128;  // output columns (weight rows of the result) per tile and CTA
+  // A pair walks the list together: first CTA's rows, then the second's. The first one's MMA warp issues for both.
+  constexpr bool PAIR = BOX == kPair;
+  const uint32_t crank = PAIR ? blockIdx.x & 1 : 0;
+  const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmW);
@@ -139,93 +150,124 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 128);
+      mbar_init(&tempty_bar[b], PAIR ? 256 : 128);
     }
     s_fail = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
     __syncwarp();
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(tmem_slot, 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (PAIR) {   // the other CTA's barriers and tensor memory are ready too
+    cluster_arrive_release();
+    cluster_wait_acquire();
+  }
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   pdl_wait();
   trace_mark(kTraceGemmPersistent, kTraceAfterWait);
   pdl_launch_dependents();
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      // both operands are re-read by other CTAs from L2; the weights of a decode step are not
-      const uint64_t pol_w = BOX == 16 ? l2_policy_evict_first() : l2_policy_evict_last();
-      const uint64_t pol_x = l2_policy_evict_last();
-      int it = 0, issued = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        PTile tl;
-        if (!tile_at<GROUPED, kRowsPerTile>(p, t, tl)) break;
-        const int w_row0 = tl.w_row0, m_base = tl.m_base;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          ok = mbar_wait(&empty_bar[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
-          if (!ok) break;
-          uint8_t* a = stages + s * kStageBytes;
-          const int boxes = (tl.m_cnt + BOX - 1) / BOX;
-          mbar_arrive_expect_tx(&full_bar[s], kATile + (GROUPED ? boxes * kBoxBytes : p.tn * 128));
-          if (DUAL) {
-            tma_load_2d_hint(a, &tmW, kb * 64, w_row0, &full_bar[s], pol_w);
-            tma_load_2d_hint(a + kATile / 2, &tmW, kb * 64, p.dual_row_offset + w_row0, &full_bar[s], pol_w);
+    // ------------------------------------------------------------ TMA producer (the warp waits, one lane issues)
+    // both operands are re-read by other CTAs from L2; the weights of a decode step are not
+    const uint64_t pol_w = BOX == 16 ? l2_policy_evict_first() : l2_policy_evict_last();
+    const uint64_t pol_x = l2_policy_evict_last();
+    const bool one = elect_one();
+    int s = 0, issued = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int t = first; t < total && ok; t += step) {
+      PTile tl;
+      if (!tile_at<GROUPED, kRowsPerTile, PAIR>(p, t, crank, tl)) break;
+      const int w_row0 = tl.w_row0;
+      const int half = PAIR ? ((tl.m_cnt + 31) & ~31) >> 1 : 0;     // tokens that the MMA takes from either CTA
+      const int m_base = tl.m_base + static_cast<int>(crank) * half;
+      const int boxes = GROUPED ? (tl.m_cnt + BOX - 1) / BOX : 1;
+      const uint32_t bytes = PAIR ? 2 * (kATile + p.tn * 64) : kATile + (GROUPED ? boxes * kBoxBytes : p.tn * 128);
+      for (int kb = 0; kb < kblocks; ++kb) {
+        ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
+        if (!ok) break;
+        uint8_t* a = stages + s * kStageBytes;
+        if (one) {
+          if (PAIR) {
+            const uint32_t full = mapa_shared(smem_u32(&full_bar[s]), 0);
+            if (crank == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
+            tma_load_2d_pair_hint(a, &tmW, kb * 64, w_row0, full, pol_w);
+            if (DUAL) tma_load_2d_pair_hint(a + kATile / 2, &tmW, kb * 64, p.dual_row_offset + w_row0, full, pol_w);
+            tma_load_2d_pair_hint(a + kATile, &tmX, kb * 64, m_base, full, pol_x);
           } else {
+            mbar_arrive_expect_tx(&full_bar[s], bytes);
             tma_load_2d_hint(a, &tmW, kb * 64, w_row0, &full_bar[s], pol_w);
+            if (DUAL) tma_load_2d_hint(a + kATile / 2, &tmW, kb * 64, p.dual_row_offset + w_row0, &full_bar[s], pol_w);
+            for (int i = 0; i < boxes; ++i) tma_load_2d_hint(a + kATile + i * kBoxBytes, &tmX, kb * 64, m_base + i * BOX, &full_bar[s], pol_x);
           }
-          if (GROUPED) {
-            for (int i = 0; i < boxes; ++i)
-              tma_load_2d_hint(a + kATile + i * kBoxBytes, &tmX, kb * 64, m_base + i * BOX, &full_bar[s], pol_x);
-          } else {
-            tma_load_2d_hint(a + kATile, &tmX, kb * 64, m_base, &full_bar[s], pol_x);
-          }
-          issued = it + 1;
+        }
+        ++issued;
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1;
         }
       }
-      if (!ok) {  // wait (bounded) for the copies still in flight before shared memory goes away
-        for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait(&full_bar[j % kStages], (j / kStages) & 1, nullptr, 0);
-      }
+    }
+    if (PAIR && ok) {  // until the MMA warp has given back every stage: it arrives on this CTA's barriers
+      for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait(&empty_bar[j % kStages], (j / kStages) & 1, p.status, kStatusSmemEmptyTimeout);
+    }
+    if (!ok) {  // wait (bounded) for the copies still in flight before shared memory goes away
+      for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait(&full_bar[j % kStages], (j / kStages) & 1, nullptr, 0);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      uint32_t idesc = 0;
-      int it = 0, lt = 0;
+    // ------------------------------------------------------------ MMA issuer (of a pair, the first CTA's)
+    if (crank == 0) {
+      const bool one = elect_one();
+      int s = 0, lt = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++lt) {
+      for (int t = first; t < total && ok; t += step, ++lt) {
         PTile tl;
-        if (!tile_at<GROUPED, kRowsPerTile>(p, t, tl)) break;
-        idesc = umma_idesc_bf16(128, (tl.m_cnt + 15) & ~15);   // the last token tile may be a short one
+        if (!tile_at<GROUPED, kRowsPerTile, PAIR>(p, t, crank, tl)) break;
+        // the last token tile may be a short one
+        const uint32_t idesc = PAIR ? umma_idesc_bf16(256, (tl.m_cnt + 31) & ~31) : umma_idesc_bf16(128, (tl.m_cnt + 15) & ~15);
         const int buf = lt & 1;
         const uint32_t bph = (lt >> 1) & 1;
-        ok = mbar_wait(&tempty_bar[buf], bph ^ 1, p.status, kStatusAccumTimeout);
+        ok = mbar_wait_warp(&tempty_bar[buf], bph ^ 1, p.status, kStatusAccumTimeout);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t acc_addr = tmem_base + buf * kTN;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          ok = mbar_wait(&full_bar[s], ph, p.status, kStatusTmaFullTimeout);
+        for (int kb = 0; kb < kblocks; ++kb) {
+          ok = mbar_wait_warp(&full_bar[s], ph, p.status, kStatusTmaFullTimeout);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t a_addr = smem_u32(stages + s * kStageBytes);
           const uint64_t da = umma_desc_k_sw128(a_addr);
           const uint64_t db = umma_desc_k_sw128(a_addr + kATile);
+          if (one) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16(acc_addr, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(&empty_bar[s]);
+            for (int k = 0; k < 4; ++k) {
+              if (PAIR) umma_f16_pair(acc_addr, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              else umma_f16(acc_addr, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            }
+            if (PAIR) umma_commit_pair(&empty_bar[s]);
+            else umma_commit(&empty_bar[s]);
+          }
+          if (++s == kStages) {
+            s = 0;
+            ph ^= 1;
+          }
         }
-        if (ok) umma_commit(&tfull_bar[buf]);
+        if (ok && one) {
+          if (PAIR) umma_commit_pair(&tfull_bar[buf]);
+          else umma_commit(&tfull_bar[buf]);
+        }
       }
     }
   } else {
@@ -237,9 +279,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     const __nv_bfloat16* bias = static_cast<const __nv_bfloat16*>(p.bias);
     __nv_bfloat16* yout = static_cast<__nv_bfloat16*>(p.y);
     int lt = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
+    for (int t = first; t < total; t += step, ++lt) {
       PTile tl;
-      if (!tile_at<GROUPED, kRowsPerTile>(p, t, tl)) break;
+      if (!tile_at<GROUPED, kRowsPerTile, PAIR>(p, t, crank, tl)) break;
       const int tile_n = tl.tile_n, m_base = tl.m_base, m_cnt = tl.m_cnt;
       const int buf = lt & 1;
       const uint32_t bph = (lt >> 1) & 1;
@@ -295,7 +337,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
         if (cc == last_cc) {
           // this thread has read everything it needs from TMEM: hand the accumulator back to the MMA warp
           tc_fence_before_sync();
-          mbar_arrive(&tempty_bar[buf]);
+          if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
+          else mbar_arrive(&tempty_bar[buf]);
         }
         epi_bar();
         const float* st = reinterpret_cast<const float*>(staging);
@@ -351,7 +394,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
             }
 #pragma unroll
             for (int o2 = 8; o2 > 0; o2 >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o2);
-            if ((lane & 15) == 0 && cc + c < m_cnt) p.ssq_out[static_cast<size_t>(m) * p.n_tiles + tile_n] = sq;
+            if ((lane & 15) == 0 && cc + c < m_cnt && tile_n < p.ssq_stride) p.ssq_out[static_cast<size_t>(m) * p.ssq_stride + tile_n] = sq;
           }
         }
         epi_bar();  // staging may be overwritten
@@ -361,31 +404,65 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
+  if (PAIR) {   // neither leaves while the other's products read its shared memory, or its barriers are arrived on
+    cluster_arrive_release();
+    cluster_wait_acquire();
+  }
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tmem_base, 512);
+    if (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
   trace_mark(kTraceGemmPersistent, kTraceEnd);
 }
 
 }  // namespace
 
-// Token rows of a tile. A CTA walks ceil(tiles / SMs) tiles, and with 256 rows the last of these walks is often nearly empty (1250 x 4096:
-// 160 tiles on 148 SMs). A round of smaller tiles is shorter, but by much less than its rows: weights have to be fetched and read all
-// the same. Rounds of 256, 160, 128 and 96 rows at K = 4096 took 29.4, 24.4, 22.6 and 21.5 us, which is kTileFixed rows and the tile's own;
-// 1250 x 4096 x 14336 165 -> 157 us, 300 x 2 x 28672 x 8192 368 -> 317.
-static int pick_token_tile(int M, int n_tiles, int sms) {
+// Token rows of a tile. A CTA (pair) walks ceil(tiles / CTAs) tiles, and with 256 rows the last of these walks is often nearly empty (1250 x 4096:
+// 80 tiles on 74 pairs). Microseconds of a pair per 64 of K with 256, 224, 192, 160, 128, 96 and 64 rows: 0.40, 0.34, 0.30, 0.26, 0.25, 0.25
+// and 0.24 (what it takes to fetch and issue a stage); of one CTA with 256, 128 and 64: 0.49, 0.33, 0.29 (it fetches 128 weight rows and all tokens).
+// 1250 x 4096 x 14336 157 us -> 114, 1024 x 4096 x 4096 32.9 -> 28.5, 300 x 8192 x 8192 55 -> 46.
+static int pick_token_tile(int M, int n_tiles, int workers, bool pair) {
   int best = kTN;
   long cost = -1;
-  for (int tn = kTN; tn >= 96; tn -= 16) {
+  for (int tn = kTN; tn >= 64; tn -= pair ? 32 : 16) {
     const long tiles = static_cast<long>(n_tiles) * ((M + tn - 1) / tn);
-    const long c = (tiles + sms - 1) / sms * (std::min(tn, M) + kTileFixed);
+    const int rows = std::min(tn, M);
+    const long c = (tiles + workers - 1) / workers * (pair ? std::max(rows + 22, 172) : std::max(rows + 128, 220));
     if (cost < 0 || c < cost) {
       cost = c;
       best = tn;
     }
   }
   return best;
+}
+
+template <bool DUAL>
+static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const PGemmParams& p, int grid, cudaStream_t stream) {
+  static bool configured[64] = {};  // the attribute is a per-device setting
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(gemm_persistent_kernel<DUAL, false, kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<kPair>);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = kSmemBytes<kPair>;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, gemm_persistent_kernel<DUAL, false, kPair>, tmW, tmX, p);
 }
 
 int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* residual, const void* bias, int M, int N,
@@ -401,8 +478,12 @@ int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* re
   if (r != 0) return -100 + r;
   const int sms = sm_count > 0 ? sm_count : 148;
   const int n_tiles = dual ? (N + 63) / 64 : (N + 127) / 128;
-  const int tn = pick_token_tile(M, n_tiles, sms);
-  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, ldx, tn, 64);
+  // Two CTAs to a tile: 1.1 to 1.3 times the speed wherever the products count. Sums of less than sixteen blocks are bound by the epilogue, and a
+  // second CTA without rows does not help a single row tile (8192 x 2 x 768 x 768: 22.8 us with one CTA, 23.6 with two).
+  const bool pair = K >= 1024 && n_tiles > 1 && sms > 1;
+  const int workers = pair ? sms / 2 : sms, row_tiles = pair ? (n_tiles + 1) / 2 : n_tiles;
+  const int tn = pick_token_tile(M, row_tiles, workers, pair);
+  r = make_tma_2d(&tmX, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, ldx, pair ? tn / 2 : tn, 64);
   if (r != 0) return -200 + r;
   PGemmParams p = {};
   p.y = Y;
@@ -424,13 +505,19 @@ int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* re
   p.act_a = act_a;
   p.act_b = act_b;
   p.out_fp32 = out_fp32;
-  p.n_tiles = n_tiles;
+  p.n_tiles = row_tiles;
+  p.ssq_stride = n_tiles;
   p.tn = tn;
   p.m_tiles = (M + tn - 1) / tn;
   const int total = p.n_tiles * p.m_tiles;
   // equal rounds for every CTA where possible: ceil(total / rounds) CTAs, never more than the SM count
-  const int rounds = (total + sms - 1) / sms;
-  const int grid = (total + rounds - 1) / rounds;
+  const int rounds = (total + workers - 1) / workers;
+  const int grid = (total + rounds - 1) / rounds * (pair ? 2 : 1);
+  if (pair) {
+    const cudaError_t e = dual ? launch_pair<true>(tmW, tmX, p, grid, stream) : launch_pair<false>(tmW, tmX, p, grid, stream);
+    eredu_count_launches(1);
+    return static_cast<int>(e);
+  }
   auto launch = [&](auto kern) -> cudaError_t {
     static bool configured_plain = false, configured_dual = false;
     bool& configured = dual ? configured_dual : configured_plain;

@@ -121,6 +121,23 @@ def test_four_bit_rows_at_the_borders_of_the_plan(M, N, K, group, gated):
     test_four_bit_rows_of_few_tokens(M, N, K, group, gated)
 
 
+@pytest.mark.parametrize("M", [129, 161, 300, 777])
+@pytest.mark.parametrize("N,K", [(128, 1024), (136, 1024), (264, 1016), (392, 1088), (3848, 4096)])
+def test_projections_of_prompts_on_pairs_of_ctas(M, N, K):
+    """One row tile, a second tile that only one CTA of a pair has rows of, sums on either side of where pairs start; last token tiles of which a
+    CTA's half is short."""
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = (torch.randn(2 * N, K, device=DEV) * K ** -0.5).bfloat16()
+    res = torch.randn(M, N, device=DEV).bfloat16()
+    y = x.double() @ w.double().t()
+    # products of bf16 are exact in fp32, and the sums are a thousandth of the result's rounding
+    assert rel_l2(ops.linear(x, w[:N], residual=res), y[:, :N] + res.double()) < BF16
+    assert rel_l2(ops.linear(x, w[:N], out_dtype=torch.float32), y[:, :N]) < BF16 / 256
+    got, ssq = ops.linear(x, w[:N], residual=res, want_ssq=True)
+    assert rel_l2(ssq.sum(-1), got.double().square().sum(-1)) < 1e-5
+    assert rel_l2(ops.gated_linear(x, w, N), moe_ops.gated_act_ref(y[:, :N].float(), y[:, N:].float())) < BF16
+
+
 @pytest.mark.parametrize("M", [1, 2])
 @pytest.mark.parametrize("N,K,group,gated", [(4752, 3072, 64, False), (4736, 3072, 64, False), (4744, 5120, 128, False), (2 * 4736, 3136, 64, True),
                                              (2848, 8192, 64, False), (2848, 8448, 128, False), (2832, 8192, 64, False), (4752, 17600, 64, False), (2 * 2384, 17664, 64, True),
