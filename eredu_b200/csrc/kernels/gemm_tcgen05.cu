@@ -177,7 +177,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);  // [1]
   uint8_t* stages = smem + Cfg::kCtrlBytes;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int tile_n = blockIdx.x;
   const int tile_m = blockIdx.y;
@@ -221,23 +221,30 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   // Weight tiles do not depend on the producer kernels: start them before the wait.
   int n_pre = 0;
   if (p.w_static && p.work == nullptr) {
     n_pre = min(niter, Cfg::kStages);
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
       const uint64_t pol_w = l2_policy_evict_first();
-      for (int it = 0; it < niter; ++it) {
+      const bool one = elect_one();
+      for (int it = 0; it < n_pre; ++it) {
         const int kx = (kb0 + it) * 64;
-        if (it < n_pre) {
-          uint8_t* a = stages + it * Cfg::kStageBytes;
+        uint8_t* a = stages + it * Cfg::kStageBytes;
+        if (one) {
           mbar_arrive_expect_tx(&full_bar[it], Cfg::kStageBytes);
           tma_load_2d_hint(a, &tmW, kx, w_row0, &full_bar[it], pol_w);
           if (DUAL) tma_load_2d_hint(a + Cfg::kATile, &tmW, kx, p.dual_row_offset + w_row0, &full_bar[it], pol_w);
-        } else if (p.w_static > 1) {
-          tma_prefetch_l2_2d(&tmW, kx, w_row0);
-          if (DUAL) tma_prefetch_l2_2d(&tmW, kx, p.dual_row_offset + w_row0);
+        }
+      }
+      if (p.w_static > 1) {
+        for (int it = n_pre; it < niter; ++it) {
+          const int kx = (kb0 + it) * 64;
+          if (one) {
+            tma_prefetch_l2_2d(&tmW, kx, w_row0);
+            if (DUAL) tma_prefetch_l2_2d(&tmW, kx, p.dual_row_offset + w_row0);
+          }
         }
       }
     }
@@ -251,52 +258,57 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   const int parity = static_cast<int>(seq & 1u);
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const uint64_t pol_w = l2_policy_evict_first();
-      const uint64_t pol_x = l2_policy_evict_last();
-      int issued = n_pre;
-      bool ok = true;
-      for (int it = 0; it < niter && ok; ++it) {
-        const int s = it % Cfg::kStages;
-        const uint32_t ph = (it / Cfg::kStages) & 1;
-        uint8_t* a = stages + s * Cfg::kStageBytes;
-        const int kx = (kb0 + it) * 64;
-        if (it >= n_pre) {  // the first n_pre stages already hold (or are receiving) their weight tiles
-          ok = mbar_wait(&empty_bar[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
-          if (!ok) break;
+    // ------------------------------------------------------------ TMA producer (the warp waits, one lane issues)
+    const uint64_t pol_w = l2_policy_evict_first();
+    const uint64_t pol_x = l2_policy_evict_last();
+    const bool one = elect_one();
+    int issued = n_pre, s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int it = 0; it < niter; ++it) {
+      uint8_t* a = stages + s * Cfg::kStageBytes;
+      const int kx = (kb0 + it) * 64;
+      if (it >= n_pre) {  // the first n_pre stages already hold (or are receiving) their weight tiles
+        ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
+        if (!ok) break;
+        if (one) {
           mbar_arrive_expect_tx(&full_bar[s], Cfg::kStageBytes);
           tma_load_2d_hint(a, &tmW, kx, w_row0, &full_bar[s], pol_w);
           if (DUAL) tma_load_2d_hint(a + Cfg::kATile, &tmW, kx, p.dual_row_offset + w_row0, &full_bar[s], pol_w);
         }
-        tma_load_2d_hint(a + Cfg::kATile * (DUAL ? 2 : 1), &tmX, kx, m_base, &full_bar[s], pol_x);
-        issued = it + 1;
       }
-      if (!ok) {
-        // Give up cleanly: wait (bounded) for the copies still in flight before shared memory dies.
-        const int first = max(0, issued - Cfg::kStages);
-        for (int it = first; it < issued; ++it) {
-          mbar_wait(&full_bar[it % Cfg::kStages], (it / Cfg::kStages) & 1, nullptr, 0);
-        }
+      if (one) tma_load_2d_hint(a + Cfg::kATile * (DUAL ? 2 : 1), &tmX, kx, m_base, &full_bar[s], pol_x);
+      issued = it + 1;
+      if (++s == Cfg::kStages) {
+        s = 0;
+        ph ^= 1;
+      }
+    }
+    if (!ok) {
+      // Give up cleanly: wait (bounded) for the copies still in flight before shared memory dies.
+      const int first = max(0, issued - Cfg::kStages);
+      for (int it = first; it < issued; ++it) {
+        mbar_wait(&full_bar[it % Cfg::kStages], (it / Cfg::kStages) & 1, nullptr, 0);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, TN);
-      bool ok = true;
-      for (int it = 0; it < niter; ++it) {
-        const int s = it % Cfg::kStages;
-        const uint32_t ph = (it / Cfg::kStages) & 1;
-        ok = mbar_wait(&full_bar[s], ph, p.status, kStatusTmaFullTimeout);
-        if (!ok) break;
-        if (it == 0) trace_mark_thread(kTraceGemm, 3, 32);       // first operands landed
-        if (it == niter - 1) trace_mark_thread(kTraceGemm, 4, 32);  // last operands landed
-        tc_fence_after_sync();
-        const uint32_t a_addr = smem_u32(stages + s * Cfg::kStageBytes);
-        const uint64_t da = umma_desc_k_sw128(a_addr);
-        const uint64_t da2 = umma_desc_k_sw128(a_addr + Cfg::kATile);
-        const uint64_t db = umma_desc_k_sw128(a_addr + Cfg::kATile * (DUAL ? 2 : 1));
+    constexpr uint32_t idesc = umma_idesc_bf16(128, TN);
+    const bool one = elect_one();
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int it = 0; it < niter; ++it) {
+      ok = mbar_wait_warp(&full_bar[s], ph, p.status, kStatusTmaFullTimeout);
+      if (!ok) break;
+      if (it == 0) trace_mark_thread(kTraceGemm, 3, 32);       // first operands landed
+      if (it == niter - 1) trace_mark_thread(kTraceGemm, 4, 32);  // last operands landed
+      tc_fence_after_sync();
+      const uint32_t a_addr = smem_u32(stages + s * Cfg::kStageBytes);
+      const uint64_t da = umma_desc_k_sw128(a_addr);
+      const uint64_t da2 = umma_desc_k_sw128(a_addr + Cfg::kATile);
+      const uint64_t db = umma_desc_k_sw128(a_addr + Cfg::kATile * (DUAL ? 2 : 1));
+      if (one) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
@@ -305,10 +317,14 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         }
         umma_commit(&empty_bar[s]);
       }
-      if (ok) umma_commit(accum_bar);
+      if (++s == Cfg::kStages) {
+        s = 0;
+        ph ^= 1;
+      }
     }
+    if (ok && one) umma_commit(accum_bar);
   }
-  __syncwarp();  // lanes 1..31 of the producer / MMA warps rejoin lane 0 before any block or cluster barrier
+  __syncwarp();  // the producer / MMA warps are whole again before any block or cluster barrier
 
   // ------------------------------------------------------------ epilogue (warps 2..5)
   const int q = warp & 3;  // TMEM lane quarter this warp may read
