@@ -154,7 +154,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   pdl_launch_early();
   trace_mark(kTraceAttnPrefill, kTraceStart);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   // heads vary fastest: the first wave holds the longest query tiles of every head (longest-first balances the causal
   // triangle), and neighbouring CTAs are query heads of one key / value head reading the same pages
   const int gs = SPLIT ? p.gshift : 0;
@@ -163,10 +163,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   if (SPLIT) {
     asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(nsplit));
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    nsplit = static_cast<int>(warp_uniform(nsplit));
+    rank = static_cast<int>(warp_uniform(rank));
   }
   const int b = blockIdx.z, head = SPLIT ? static_cast<int>(blockIdx.x) / nsplit << gs : blockIdx.x, qt = tc_query_tile(p, gridDim.y, blockIdx.y);
   const int4 seq = ROWS ? p.table[b] : make_int4(p.cu_q[b], p.cu_q[b + 1] - p.cu_q[b], 0, p.seq_lens[b]);
-  const int q0 = seq.x, q_len = seq.y, kv_len = seq.w;
+  // (the same in all lanes for the compiler too: loops of the issuing warps hang on them)
+  const int q0 = static_cast<int>(warp_uniform(seq.x)), q_len = static_cast<int>(warp_uniform(seq.y)), kv_len = static_cast<int>(warp_uniform(seq.w));
   const int row0 = qt * 2 * tile_tokens;
   if (row0 >= q_len) return;                                            // uniform: before any barrier or allocation
   const int kv_head = head / (p.n_q_heads / p.n_kv_heads);
@@ -224,7 +227,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
   pdl_wait();
   trace_mark(kTraceAttnPrefill, kTraceAfterWait);
   pdl_launch_dependents();
@@ -233,16 +236,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   float m_row = -INFINITY, l_row = 0.f;      // SPLIT: a softmax thread's row
   bool live_row = false;
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && (!SPLIT || total > 0)) {
-      mbar_arrive_expect_tx(q_full, 2 * NK * kTcHalf);
-      for (int w = 0; w < 2; ++w)
-        for (int h = 0; h < NK; ++h)
-          // ROWS: the last half starts where the shared part does; a box that reaches beyond the per-head part meets zeros on the key side
-          tma_load_3d(q_s + (w * NK + h) * kTcHalf, &tmQ, ROWS && h == NK - 1 ? p.dk - p.rot : h * 64, head, q0 + row0 + w * tile_tokens, q_full);
+    // ------------------------------------------------------------------ TMA producer (the warp waits, one lane issues)
+    if (!SPLIT || total > 0) {
+      const bool one = elect_one();
+      if (one) {
+        mbar_arrive_expect_tx(q_full, 2 * NK * kTcHalf);
+        for (int w = 0; w < 2; ++w)
+          for (int h = 0; h < NK; ++h)
+            // ROWS: the last half starts where the shared part does; a box that reaches beyond the per-head part meets zeros on the key side
+            tma_load_3d(q_s + (w * NK + h) * kTcHalf, &tmQ, ROWS && h == NK - 1 ? p.dk - p.rot : h * 64, head, q0 + row0 + w * tile_tokens, q_full);
+      }
       const int* pages = p.block_table + static_cast<size_t>(b) * p.max_pages;
-      const int pool_row = POOL ? p.pool_first[b] : 0;
-      for (int jj = 0; jj < total && ok; ++jj) {
+      const int pool_row = POOL ? static_cast<int>(warp_uniform(p.pool_first[b])) : 0;
+      const int first_row = static_cast<int>(warp_uniform(seq.z));
+      for (int jj = 0; jj < total; ++jj) {
         const bool means = POOL && jj < pooled;
         const int j = means ? jj : j0 + jj - pooled;                     // key tile; jj counts this CTA's iterations
         const int s = jj & 1;
@@ -250,43 +257,47 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const int sv = VST == 2 ? s : 0;
         int page[8];
         if (!ROWS && !means) {
+          // lane pg reads page pg; beyond the table: the reserved page (masked)
+          const int mine = lane < 8 && j * 8 + lane < p.max_pages ? pages[j * 8 + lane] : 0;
 #pragma unroll
-          for (int pg = 0; pg < 8; ++pg) {
-            const int page_index = j * 8 + pg;
-            page[pg] = page_index < p.max_pages ? pages[page_index] : 0;            // beyond the table: the reserved page (masked)
+          for (int pg = 0; pg < 8; ++pg) page[pg] = __shfl_sync(0xffffffffu, mine, pg);
+        }
+        if (jj >= 2) ok = mbar_wait_warp(&k_empty[s], reuse_parity, p.status, kStatusSmemEmptyTimeout);
+        if (!ok) break;
+        if (one) {
+          mbar_arrive_expect_tx(&k_full[s], NK * kTcHalf);
+          if (ROWS) {
+            for (int h = 0; h + 1 < NK; ++h) tma_load_3d(k_s + (s * NK + h) * kTcHalf, &tmK, h * 64, head, first_row + j * kTcTile, &k_full[s]);
+            tma_load_2d(k_s + (s * NK + NK - 1) * kTcHalf, &tmR, 0, first_row + j * kTcTile, &k_full[s]);
+          }
+          if (means) {
+            for (int h = 0; h < NK; ++h) tma_load_3d(k_s + (s * NK + h) * kTcHalf, &tmR, h * 64, kv_head, pool_row + j * kTcTile, &k_full[s]);
+          } else {
+#pragma unroll
+            for (int pg = 0; pg < (ROWS ? 0 : 8); ++pg)
+              for (int h = 0; h < NK; ++h) tma_load_4d(k_s + (s * NK + h) * kTcHalf + pg * 2048, &tmK, h * 64, 0, kv_head, page[pg], &k_full[s]);
           }
         }
-        if (jj >= 2) ok = mbar_wait(&k_empty[s], reuse_parity, p.status, kStatusSmemEmptyTimeout);
+        if (jj >= VST) ok = mbar_wait_warp(&v_empty[sv], VST == 2 ? reuse_parity : (jj - 1) & 1, p.status, kStatusSmemEmptyTimeout);
         if (!ok) break;
-        mbar_arrive_expect_tx(&k_full[s], NK * kTcHalf);
-        if (ROWS) {
-          for (int h = 0; h + 1 < NK; ++h) tma_load_3d(k_s + (s * NK + h) * kTcHalf, &tmK, h * 64, head, seq.z + j * kTcTile, &k_full[s]);
-          tma_load_2d(k_s + (s * NK + NK - 1) * kTcHalf, &tmR, 0, seq.z + j * kTcTile, &k_full[s]);
-        }
-        if (means) {
-          for (int h = 0; h < NK; ++h) tma_load_3d(k_s + (s * NK + h) * kTcHalf, &tmR, h * 64, kv_head, pool_row + j * kTcTile, &k_full[s]);
-        } else {
+        if (one) {
+          mbar_arrive_expect_tx(&v_full[sv], NV * kTcHalf);
+          if (ROWS)
+            for (int h = 0; h < NV; ++h) tma_load_3d(v_s + (sv * NV + h) * kTcHalf, &tmV, h * 64, head, first_row + j * kTcTile, &v_full[sv]);
+          if (means) {
+            for (int h = 0; h < NV; ++h) tma_load_3d(v_s + (sv * NV + h) * kTcHalf, &tmS, h * 64, kv_head, pool_row + j * kTcTile, &v_full[sv]);
+          } else {
 #pragma unroll
-          for (int pg = 0; pg < (ROWS ? 0 : 8); ++pg)
-            for (int h = 0; h < NK; ++h) tma_load_4d(k_s + (s * NK + h) * kTcHalf + pg * 2048, &tmK, h * 64, 0, kv_head, page[pg], &k_full[s]);
-        }
-        if (jj >= VST) ok = mbar_wait(&v_empty[sv], VST == 2 ? reuse_parity : (jj - 1) & 1, p.status, kStatusSmemEmptyTimeout);
-        if (!ok) break;
-        mbar_arrive_expect_tx(&v_full[sv], NV * kTcHalf);
-        if (ROWS)
-          for (int h = 0; h < NV; ++h) tma_load_3d(v_s + (sv * NV + h) * kTcHalf, &tmV, h * 64, head, seq.z + j * kTcTile, &v_full[sv]);
-        if (means) {
-          for (int h = 0; h < NV; ++h) tma_load_3d(v_s + (sv * NV + h) * kTcHalf, &tmS, h * 64, kv_head, pool_row + j * kTcTile, &v_full[sv]);
-        } else {
-#pragma unroll
-          for (int pg = 0; pg < (ROWS ? 0 : 8); ++pg)
-            for (int h = 0; h < NV; ++h) tma_load_4d(v_s + (sv * NV + h) * kTcHalf + pg * 2048, &tmV, h * 64, 0, kv_head, page[pg], &v_full[sv]);
+            for (int pg = 0; pg < (ROWS ? 0 : 8); ++pg)
+              for (int h = 0; h < NV; ++h) tma_load_4d(v_s + (sv * NV + h) * kTcHalf + pg * 2048, &tmV, h * 64, 0, kv_head, page[pg], &v_full[sv]);
+          }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && (!SPLIT || total > 0)) {
+    if (!SPLIT || total > 0) {
+      const bool one = elect_one();
       const uint32_t q_addr = smem_u32(q_s);
       // jj: this CTA's iteration (selects the K / V stage); tile w is active on key tiles [first_w, n_w)
       const int first[2] = {j0_a, j0_b}, last[2] = {n_a, n_b};
@@ -294,6 +305,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const uint32_t qa = q_addr + w * NK * kTcHalf;
         const uint32_t ka = smem_u32(k_s + (jj & 1) * NK * kTcHalf);
         const uint32_t d = tmem + w * 128;
+        if (!one) return;
 #pragma unroll
         for (int kk = 0; kk < NK * 4; ++kk) {      // K = key width: four 16-steps per 64-wide half
           if (ROWS ? (kk & 3) * 16 >= (kk >> 2 == NK - 1 ? p.rot : p.dk - p.rot - (kk >> 2) * 64) : kk >= k_steps) continue;
@@ -304,6 +316,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       };
       auto issue_pv = [&](int w, int jj, bool fresh) {
         const uint32_t va = smem_u32(v_s + (VST == 2 ? jj & 1 : 0) * NV * kTcHalf);
+        if (!one) return;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)             // K = keys: P from tensor memory (8 columns per step), V MN-major (2048 bytes per step)
           umma_f16_ts(tmem + 256 + w * 128, tmem + w * 128 + kk * 8, umma_desc_mn_sw128(va + kk * 2048, kTcHalf), kIdescPV,
@@ -312,41 +325,41 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const int seen[2] = {np_a, np_b};
       // u counts this CTA's iterations; a query tile's last one is a token tile
       auto active = [&](int w, int u) { return POOL && u < pooled ? u < seen[w] : u >= pooled + first[w] - j0 && u < pooled + last[w] - j0; };
-      ok = mbar_wait(q_full, 0, p.status, kStatusTmaFullTimeout);
-      if (ok) ok = mbar_wait(&k_full[0], 0, p.status, kStatusTmaFullTimeout);
+      ok = mbar_wait_warp(q_full, 0, p.status, kStatusTmaFullTimeout);
+      if (ok) ok = mbar_wait_warp(&k_full[0], 0, p.status, kStatusTmaFullTimeout);
       if (ok) {
         tc_fence_after_sync();
         if (active(0, 0)) issue_s(0, 0);
         if (active(1, 0)) issue_s(1, 0);
-        umma_commit(&k_empty[0]);
+        if (one) umma_commit(&k_empty[0]);
       }
       int done[2] = {0, 0};                        // softmax rounds completed per tile: parity of p_full
       for (int jj = 0; jj < total && ok; ++jj) {
         const bool next = jj + 1 < total;
         bool k_ready = false;
-        ok = mbar_wait(&v_full[VST == 2 ? jj & 1 : 0], (VST == 2 ? jj >> 1 : jj) & 1, p.status, kStatusTmaFullTimeout);
+        ok = mbar_wait_warp(&v_full[VST == 2 ? jj & 1 : 0], (VST == 2 ? jj >> 1 : jj) & 1, p.status, kStatusTmaFullTimeout);
         for (int w = 0; w < 2 && ok; ++w) {
           if (active(w, jj)) {
-            ok = mbar_wait(&p_full[w], done[w] & 1, p.status, kStatusAccumTimeout);   // P_w(j) is in tensor memory, O_w is rescaled
+            ok = mbar_wait_warp(&p_full[w], done[w] & 1, p.status, kStatusAccumTimeout);   // P_w(j) is in tensor memory, O_w is rescaled
             if (!ok) break;
             tc_fence_after_sync();
             issue_pv(w, jj, done[w] == 0);
             ++done[w];
           }
-          if (w == 1) umma_commit(&v_empty[VST == 2 ? jj & 1 : 0]);
+          if (w == 1 && one) umma_commit(&v_empty[VST == 2 ? jj & 1 : 0]);
           if (active(w, jj + 1)) {
             if (!k_ready) {
-              ok = mbar_wait(&k_full[(jj + 1) & 1], ((jj + 1) >> 1) & 1, p.status, kStatusTmaFullTimeout);
+              ok = mbar_wait_warp(&k_full[(jj + 1) & 1], ((jj + 1) >> 1) & 1, p.status, kStatusTmaFullTimeout);
               if (!ok) break;
               tc_fence_after_sync();
               k_ready = true;
             }
             issue_s(w, jj + 1);
           } else if (jj + 1 == pooled + last[w] - j0) {
-            umma_commit(&o_final[w]);
+            if (one) umma_commit(&o_final[w]);
           }
         }
-        if (ok && next) umma_commit(&k_empty[(jj + 1) & 1]);
+        if (ok && next && one) umma_commit(&k_empty[(jj + 1) & 1]);
       }
     }
   } else {
