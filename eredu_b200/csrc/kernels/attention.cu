@@ -77,28 +77,72 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t cluster_addr) {
 // rotation of the first `rot` dims by the token's position. Executed by one warp; lane l owns the pairs l, l + 32, ...
 // `store(i0, a, i1, b)` receives the finished element pairs.
 // `whole_inv` > 0: the projection's own 1 / rms, instead of the head's. Heads may be narrower than D (p.dk).
-template <int D, bool EXT, typename Store>
-__device__ __forceinline__ void rope_head_row(const AttnParams& p, const __nv_bfloat16* src, const float* nw, float whole_inv,
-                                              int pos, int lane, Store store) {
-  constexpr int PER = D / 64;  // pairs per lane
-  const int dk = EXT ? p.dk : D;
+// The parts are called on their own where a row's numbers, or what goes with its position, are known earlier than the rest.
+template <int D>
+struct HeadRow {
+  static constexpr int PER = D / 64;  // pairs per lane
+  float a[PER], b[PER];
+};
+template <int D>
+struct Turn {
+  float cs[D / 64], sn[D / 64];
+};
+
+__device__ __forceinline__ void pair_index(const AttnParams& p, int i, int& i0, int& i1) {
   const int rh = p.rot >> 1;
+  if (i < rh) {
+    i0 = p.interleaved ? 2 * i : i;
+    i1 = p.interleaved ? 2 * i + 1 : i + rh;
+  } else {  // pass-through tail beyond the rotary dims
+    i0 = p.rot + 2 * (i - rh);
+    i1 = i0 + 1;
+  }
+}
+
+template <int D, bool EXT>
+__device__ __forceinline__ HeadRow<D> load_head_row(const AttnParams& p, const __nv_bfloat16* src, int lane) {
+  HeadRow<D> r;
+#pragma unroll
+  for (int j = 0; j < D / 64; ++j) {
+    int i0, i1;
+    pair_index(p, lane + 32 * j, i0, i1);
+    const bool in = 2 * (lane + 32 * j) < (EXT ? p.dk : D);
+    r.a[j] = in ? __bfloat162float(src[i0]) : 0.f;
+    r.b[j] = in ? __bfloat162float(src[i1]) : 0.f;
+  }
+  return r;
+}
+
+template <int D>
+__device__ __forceinline__ Turn<D> turn_at(const AttnParams& p, int pos, int lane) {
+  Turn<D> t;
+#pragma unroll
+  for (int j = 0; j < D / 64; ++j) {
+    const int i = lane + 32 * j;
+    t.cs[j] = 1.f;
+    t.sn[j] = 0.f;
+    if (i < p.rot >> 1) {
+      sincosf(static_cast<float>(pos) * p.inv_freq[i], &t.sn[j], &t.cs[j]);
+      t.sn[j] *= p.attn_factor;
+      t.cs[j] *= p.attn_factor;
+    }
+  }
+  return t;
+}
+
+template <int D, bool EXT, typename Store>
+__device__ __forceinline__ void rope_head_row(const AttnParams& p, const HeadRow<D>& row, const float* nw, float whole_inv,
+                                              const Turn<D>& turn, int lane, Store store) {
+  constexpr int PER = D / 64;
+  const int dk = EXT ? p.dk : D;
   float a[PER], b[PER];
   int i0[PER], i1[PER];
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
-    const int i = lane + 32 * j;
-    if (i < rh) {
-      i0[j] = p.interleaved ? 2 * i : i;
-      i1[j] = p.interleaved ? 2 * i + 1 : i + rh;
-    } else {  // pass-through tail beyond the rotary dims
-      i0[j] = p.rot + 2 * (i - rh);
-      i1[j] = i0[j] + 1;
-    }
-    const bool in = 2 * i < dk;
-    a[j] = in ? __bfloat162float(src[i0[j]]) : 0.f;
-    b[j] = in ? __bfloat162float(src[i1[j]]) : 0.f;
+    pair_index(p, lane + 32 * j, i0[j], i1[j]);
+    a[j] = row.a[j];
+    b[j] = row.b[j];
     ss += a[j] * a[j] + b[j] * b[j];
   }
   if (nw != nullptr && (EXT && p.norm_whole)) {
@@ -122,13 +166,9 @@ __device__ __forceinline__ void rope_head_row(const AttnParams& p, const __nv_bf
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     const int i = lane + 32 * j;
-    if (i < rh) {
-      float sn, cs;
-      sincosf(static_cast<float>(pos) * p.inv_freq[i], &sn, &cs);
-      sn *= p.attn_factor;
-      cs *= p.attn_factor;
-      const float ra = a[j] * cs - b[j] * sn;
-      const float rb = b[j] * cs + a[j] * sn;
+    if (i < p.rot >> 1) {
+      const float ra = a[j] * turn.cs[j] - b[j] * turn.sn[j];
+      const float rb = b[j] * turn.cs[j] + a[j] * turn.sn[j];
       a[j] = ra;
       b[j] = rb;
     }
@@ -352,35 +392,36 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(AttnParams p) {
 
 // ============================================================================ decode (split-KV)
 // grid (splits, n_kv_heads, B). The MT*16 MMA rows hold (query token t, head-in-group g) pairs,
-// row = (t - t0) * group + g. Each of the 4 warps streams every 4th page through its own 3-stage
+// row = (t - t0) * group + g. Each of the NW warps streams every NWth page through its own 3-stage
 // cp.async ring and keeps private (m, l, O); the warps are merged through shared memory at the end.
 // Keys and values may differ in width: tiles are DK / DV wide (64 or 128), rows of the cache dk / dv (the rest of a
 // tile row is zero-filled, which adds nothing to scores or outputs). EXT = false is the common case with everything beyond
 // it folded away: one head size that fills the tile, no chunks, the preparation of rope_kv. POOL: sixteen pooled blocks at a time are
 // walked like a page, in front of the pages of the window.
-// A step of one sequence is bound by a chain of latencies: length, table, first pages, rows of the projection, then little arithmetic and the
-// exchange of the splits. With p.settled only the projection comes from the kernel before this one - what the lengths, tables and pages
-// hold was written by kernels that had ended when that one passed its own dependency wait - so the first three links run ahead of the
+// A step of one sequence is bound by a chain of latencies: length, table, first pages, rows of the projection and their turn, then little
+// arithmetic and the exchange of the splits. The turn of a single new token and its slot are taken, and three pages asked for, before the rows
+// are waited for (one sequence of 2048, 32 heads of 128 over 8: 10.0 -> 8.8 us, 7.5 with eight warps). With p.settled only the projection comes from the kernel before this one - what the lengths, tables and pages
+// hold was written by kernels that had ended when that one passed its own dependency wait - so the first links run ahead of the
 // wait, under the tail of the projection. That holds because a kernel releases the next one behind its own wait; a build that releases at
 // entry (EREDU_PDL_EARLY=1) waits first. Measured over whole decode steps: one sequence, 16 layers of 64-wide heads, three draft passes
 // 2917 -> 2870 us; one sequence, 32 layers of 128-wide heads 3687 -> 3660 us; 32 sequences of the same 5499 -> 5475 us.
-template <int DK, int DV, int MT, bool EXT, bool POOL>
-__global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) attn_decode_kernel(AttnParams p) {
+template <int DK, int DV, int MT, bool EXT, bool POOL, int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 4 && MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) attn_decode_kernel(AttnParams p) {
   const int dk = EXT ? p.dk : DK, dv = EXT ? p.dv : DV;
   const bool norm_whole = EXT && p.norm_whole, value_norm = EXT && p.value_norm;
   constexpr int CHK = DK / 8, CHV = DV / 8;
   constexpr int KS = DK / 16;
-  constexpr int NSTAGE = 3;
+  constexpr int NSTAGE = 3, NT = 32 * NW;
   constexpr int ROWS = 16 * MT;
   constexpr int KPAGE_BYTES = kPage * DK * 2;
   constexpr int STAGE_BYTES = kPage * (DK + DV) * 2;
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t* q_s = smem;                   // [ROWS][DK] bf16
   uint8_t* newkv_s = smem + ROWS * DK * 2;                   // [kMaxFusedNew][K row, V row] bf16 (fused path)
-  uint8_t* ring = newkv_s + kMaxFusedNew * (DK + DV) * 2;    // [4 warps][NSTAGE][K page, V page]
+  uint8_t* ring = newkv_s + kMaxFusedNew * (DK + DV) * 2;    // [NW warps][NSTAGE][K page, V page]
 
   __shared__ int s_last;
-  __shared__ float s_part[2][4], s_inv[2][kMaxFusedNew];   // fused path with norms over whole projections
+  __shared__ float s_part[2][NW], s_inv[2][kMaxFusedNew];   // fused path with norms over whole projections
   pdl_launch_early();
   trace_mark(kTraceAttnDecode, kTraceStart);
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
@@ -404,7 +445,7 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
   const int blocks = POOL ? pooled_seen(first_pos + p.t_count - 1, p.window, p.pool) : 0;
   const int base_page = first_page - (POOL ? (blocks + kPage - 1) / kPage : 0);
   int pps = (npages - base_page + p.splits - 1) / p.splits;
-  pps = (pps + 3) & ~3;
+  if (NW == 4) pps = (pps + 3) & ~3;
   const int page0 = base_page + split * pps;
   const int page1 = min(npages, page0 + pps);
 
@@ -416,7 +457,7 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
   const int new_pos0 = kv_len - p.q_per_seq;
   const int first_new_page = appending ? new_pos0 / kPage : 0x7fffffff;
   if (!fused) {
-    for (int i = threadIdx.x; i < ROWS * CHK; i += 128) {
+    for (int i = threadIdx.x; i < ROWS * CHK; i += NT) {
       const int r = i / CHK, c = i % CHK;
       const bool ok = r < rows && c * 8 < dk;
       const int t = p.t0 + (r < rows ? r / group : 0), hg = r < rows ? r % group : 0;
@@ -475,10 +516,21 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
   }
 
   const int first = page0 + warp;
-  load_page(first, 0, settled);
-  cp_async_commit();
-  load_page(first + 4, 1, settled);
-  cp_async_commit();
+#pragma unroll
+  for (int i = 0; i < NSTAGE; ++i) {
+    load_page(first + i * NW, i, settled);
+    cp_async_commit();
+  }
+  // What goes with the one new token of a sequence, its place and the turn of its position, is known ahead of the projection as well.
+  const bool single = fused && p.q_per_seq == 1;
+  Turn<DK> turn;
+  long long slot = -1;
+  if (single) {
+    turn = turn_at<DK>(p, settled ? __ldcg(p.positions + b) : p.positions[b], lane);
+    if (appending) slot = settled ? __ldcg(p.slots + b) : p.slots[b];
+  }
+  // the last warp appends the new key and value; it reads them along with its query row
+  const bool brings = single && appending && slot >= 0 && warp == NW - 1 && new_pos0 / kPage >= page0 && new_pos0 / kPage < page1;
   if (settled) {
     pdl_wait();
     trace_mark(kTraceAttnDecode, kTraceAfterWait);
@@ -491,8 +543,8 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
         const uint4* row = reinterpret_cast<const uint4*>(p.qkv + (static_cast<size_t>(b) * p.q_per_seq + t) * p.ld_qkv);
         const int nq = p.n_q_heads * dk / 8, nk = appending ? p.n_kv_heads * dk / 8 : 0;
         float sq = 0.f, sk = 0.f;
-        for (int i = threadIdx.x; i < nq; i += 128) sq += sum_squares8(row[i]);
-        for (int i = threadIdx.x; i < nk; i += 128) sk += sum_squares8(row[nq + i]);
+        for (int i = threadIdx.x; i < nq; i += NT) sq += sum_squares8(row[i]);
+        for (int i = threadIdx.x; i < nk; i += NT) sk += sum_squares8(row[nq + i]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
           sq += __shfl_xor_sync(0xffffffffu, sq, o);
@@ -506,13 +558,27 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
         if (threadIdx.x < 2) {
           const float* r = s_part[threadIdx.x];
           const float n = static_cast<float>((threadIdx.x == 0 ? p.n_q_heads : p.n_kv_heads) * dk);
-          s_inv[threadIdx.x][t] = rsqrtf((r[0] + r[1] + r[2] + r[3]) / n + p.norm_eps);
+          float sum = 0.f;
+          for (int w = 0; w < NW; ++w) sum += r[w];
+          s_inv[threadIdx.x][t] = rsqrtf(sum / n + p.norm_eps);
         }
         __syncthreads();
       }
     }
+    const __nv_bfloat16* new_row = p.qkv + static_cast<size_t>(b) * p.q_per_seq * p.ld_qkv;
+    HeadRow<DK> new_key;
+    uint32_t new_value[DV / 64];
+    if (brings) {
+      new_key = load_head_row<DK, EXT>(p, new_row + static_cast<size_t>(p.n_q_heads + kvh) * dk, lane);
+#pragma unroll
+      for (int j = 0; j < DV / 64; ++j) {
+        const int i = lane + 32 * j;
+        new_value[j] = 2 * i < dv ? reinterpret_cast<const uint32_t*>(new_row + static_cast<size_t>(p.n_q_heads + p.n_kv_heads) * dk +
+                                                                       static_cast<size_t>(kvh) * dv)[i] : 0u;
+      }
+    }
     // ---- q rows: norm + RoPE straight into the swizzled tile (rows beyond `rows` are zero)
-    for (int r = warp; r < ROWS; r += 4) {
+    for (int r = warp; r < ROWS; r += NW) {
       auto put = [&](int i0, float a, int i1, float bb) {
         *reinterpret_cast<__nv_bfloat16*>(q_s + swz<DK>(r, i0 >> 3) + (i0 & 7) * 2) = __float2bfloat16(a);
         *reinterpret_cast<__nv_bfloat16*>(q_s + swz<DK>(r, i1 >> 3) + (i1 & 7) * 2) = __float2bfloat16(bb);
@@ -522,8 +588,8 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
         const size_t m = static_cast<size_t>(b) * p.q_per_seq + t;
         const int head = kvh * group + hg;
         const float* nw = p.q_norm_w == nullptr ? nullptr : p.q_norm_w + (norm_whole ? head * dk : 0);
-        rope_head_row<DK, EXT>(p, p.qkv + m * p.ld_qkv + static_cast<size_t>(head) * dk, nw, norm_whole ? s_inv[0][t] : 0.f,
-                          p.positions[m], lane, put);
+        rope_head_row<DK, EXT>(p, load_head_row<DK, EXT>(p, p.qkv + m * p.ld_qkv + static_cast<size_t>(head) * dk, lane), nw,
+                               norm_whole ? s_inv[0][t] : 0.f, single ? turn : turn_at<DK>(p, p.positions[m], lane), lane, put);
         for (int i = dk / 2 + lane; i < DK / 2; i += 32) put(2 * i, 0.f, 2 * i + 1, 0.f);
       } else {
         for (int i = lane; i < DK / 2; i += 32) put(2 * i, 0.f, 2 * i + 1, 0.f);
@@ -532,12 +598,13 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
     // ---- new K / V rows whose page lies in this CTA's range: norm + RoPE on K; both go to the cache (for later
     // steps) and to `newkv_s` (for this step's own use)
     if (appending) {
-      for (int t = warp; t < p.q_per_seq; t += 4) {
+      for (int t = single ? 0 : warp; t < p.q_per_seq; t += NW) {
+        if (single && !brings) break;
         const int pg = (new_pos0 + t) / kPage;
         const size_t m = static_cast<size_t>(b) * p.q_per_seq + t;
-        const long long slot = p.slots[m];
-        if (pg < page0 || pg >= page1 || slot < 0) continue;  // warp-uniform
-        const size_t cell = (static_cast<size_t>(slot >> 4) * p.n_kv_heads + kvh) * kPage + static_cast<size_t>(slot & 15);
+        const long long at = single ? slot : p.slots[m];
+        if (pg < page0 || pg >= page1 || at < 0) continue;  // warp-uniform
+        const size_t cell = (static_cast<size_t>(at >> 4) * p.n_kv_heads + kvh) * kPage + static_cast<size_t>(at & 15);
         __nv_bfloat16* kd = const_cast<__nv_bfloat16*>(p.k_cache) + cell * dk;
         __nv_bfloat16* vd = const_cast<__nv_bfloat16*>(p.v_cache) + cell * dv;
         __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(newkv_s) + static_cast<size_t>(t) * (DK + DV);
@@ -545,7 +612,8 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
         const __nv_bfloat16* vrow = p.qkv + m * p.ld_qkv + static_cast<size_t>(p.n_q_heads + p.n_kv_heads) * dk +
                                     static_cast<size_t>(kvh) * dv;
         const float* nw = p.k_norm_w == nullptr ? nullptr : p.k_norm_w + (norm_whole ? kvh * dk : 0);
-        rope_head_row<DK, EXT>(p, krow, nw, norm_whole ? s_inv[1][t] : 0.f, p.positions[m], lane, [&](int i0, float a, int i1, float bb) {
+        rope_head_row<DK, EXT>(p, single ? new_key : load_head_row<DK, EXT>(p, krow, lane), nw, norm_whole ? s_inv[1][t] : 0.f,
+                               single ? turn : turn_at<DK>(p, p.positions[m], lane), lane, [&](int i0, float a, int i1, float bb) {
           const __nv_bfloat16 ha = __float2bfloat16(a), hb = __float2bfloat16(bb);
           kd[i0] = ha;
           kd[i1] = hb;
@@ -564,8 +632,10 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
           for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
           v_inv = rsqrtf(ss / static_cast<float>(dv) + p.norm_eps);
         }
-        for (int i = lane; i < DV / 2; i += 32) {
-          uint32_t vv = 2 * i < dv ? reinterpret_cast<const uint32_t*>(vrow)[i] : 0u;
+#pragma unroll
+        for (int j = 0; j < DV / 64; ++j) {
+          const int i = lane + 32 * j;
+          uint32_t vv = single ? new_value[j] : 2 * i < dv ? reinterpret_cast<const uint32_t*>(vrow)[i] : 0u;
           if (value_norm) vv = pack_bf16x2(bf16_lo(vv) * v_inv, bf16_hi(vv) * v_inv);
           if (2 * i < dv) reinterpret_cast<uint32_t*>(vd)[i] = vv;
           reinterpret_cast<uint32_t*>(ks + DK)[i] = vv;
@@ -573,15 +643,13 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
       }
     }
   }
-  cp_async_wait<2>();  // the Q tile (the oldest group)
+  cp_async_wait<NSTAGE>();  // the Q tile (the oldest group)
   __syncthreads();     // Q tile and new rows visible to every warp
 
   const uint32_t q_base = smem_u32(q_s);
   int it = 0;
-  for (int pg = first; pg < page1; pg += 4, ++it) {
-    load_page(pg + 8, (it + 2) % NSTAGE);
-    cp_async_commit();
-    cp_async_wait<2>();
+  for (int pg = first; pg < page1; pg += NW, ++it) {
+    cp_async_wait<NSTAGE - 1>();
     __syncwarp();
     if (pg >= first_new_page) {
       // this page holds rows appended in this step: overwrite them in the landed copy (16-byte chunks, lanes 0-15 the
@@ -678,15 +746,17 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
       }
     }
     __syncwarp();
+    load_page(pg + NSTAGE * NW, it % NSTAGE);
+    cp_async_commit();
   }
   cp_async_wait<0>();
   __syncthreads();  // every warp is done with its ring: reuse it for the merge
 
-  // ---- merge the 4 warps: mo[w][row][DV] fp32, mm/ml[w][row]; then this CTA's merged partial (cluster mode)
+  // ---- merge the warps: mo[w][row][DV] fp32, mm/ml[w][row]; then this CTA's merged partial (cluster mode)
   float* mo = reinterpret_cast<float*>(ring);
-  float* mm = mo + 4 * ROWS * DV;
-  float* ml = mm + 4 * ROWS;
-  float* part_s = ml + 4 * ROWS;   // [ROWS][DV]
+  float* mm = mo + NW * ROWS * DV;
+  float* ml = mm + NW * ROWS;
+  float* part_s = ml + NW * ROWS;   // [ROWS][DV]
   float* part_m = part_s + ROWS * DV;
   float* part_l = part_m + ROWS;
 #pragma unroll
@@ -697,6 +767,7 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
       l += __shfl_xor_sync(0xffffffffu, l, 1);
       l += __shfl_xor_sync(0xffffffffu, l, 2);
       const int row = mt * 16 + g + r * 8;
+      if (row >= rows) continue;
       if (tig == 0) {
         mm[warp * ROWS + row] = m_run[mt][r];
         ml[warp * ROWS + row] = l;
@@ -709,16 +780,16 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < rows * DV; i += 128) {
+  for (int i = threadIdx.x; i < rows * DV; i += NT) {
     const int row = i / DV, d = i % DV;
     if (d >= dv) continue;
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) M = fmaxf(M, mm[w * ROWS + row]);
+    for (int w = 0; w < NW; ++w) M = fmaxf(M, mm[w * ROWS + row]);
     const float Ms = (M == -INFINITY) ? 0.f : M;
     float L = 0.f, acc = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < NW; ++w) {
       const float e = exp2f(mm[w * ROWS + row] - Ms);
       L += ml[w * ROWS + row] * e;
       acc += mo[(w * ROWS + row) * DV + d] * e;
@@ -750,7 +821,7 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
     cluster_arrive_release();
     cluster_wait_acquire();
     const uint32_t a_s = smem_u32(part_s), a_m = smem_u32(part_m), a_l = smem_u32(part_l);
-    for (int i = threadIdx.x + split * 128; i < rows * DV; i += 128 * p.splits) {  // row-major: a warp stays in one row
+    for (int i = threadIdx.x + split * NT; i < rows * DV; i += NT * p.splits) {  // row-major: a warp stays in one row
       const int row = i / DV, d = i % DV;
       if (d >= dv) continue;
       float M = -INFINITY;
@@ -798,7 +869,7 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
       float* wgt = mo;                       // [rows][splits]  exp2(m_s - M)
       float* linv = mo + ROWS * 64;          // [rows]          1 / L
       __syncthreads();
-      for (int row = threadIdx.x; row < rows; row += 128) {
+      for (int row = threadIdx.x; row < rows; row += NT) {
         const int t = p.t0 + row / group, hg = row % group;
         const int head = kvh * group + hg;
         const size_t qrow = static_cast<size_t>(b * p.q_per_seq + t) * p.n_q_heads + head;
@@ -816,7 +887,7 @@ __global__ void __launch_bounds__(128, MT == 1 ? (DK + DV <= 128 ? 5 : 4) : 1) a
         linv[row] = L > 0.f ? 1.f / L : 0.f;
       }
       __syncthreads();
-      for (int i = threadIdx.x; i < rows * DV; i += 128) {
+      for (int i = threadIdx.x; i < rows * DV; i += NT) {
         const int row = i / DV, d = i % DV;
         if (d >= dv) continue;
         const int t = p.t0 + row / group, hg = row % group;
@@ -842,10 +913,10 @@ template <int D>
 static size_t prefill_smem() {
   return 64 * D * 2 + 4 * 64 * D * 2;
 }
-template <int DK, int DV, int MT>
+template <int DK, int DV, int MT, int NW>
 static size_t decode_smem() {
-  const size_t ring = 4 * 3 * kPage * (DK + DV) * 2;
-  const size_t merge = (4 * 16 * MT * DV + 2 * 4 * 16 * MT + 16 * MT * DV + 2 * 16 * MT) * sizeof(float);
+  const size_t ring = NW * 3 * kPage * (DK + DV) * 2;
+  const size_t merge = (NW * 16 * MT * DV + 2 * NW * 16 * MT + 16 * MT * DV + 2 * 16 * MT) * sizeof(float);
   return 16 * MT * DK * 2 + kMaxFusedNew * (DK + DV) * 2 + (ring > merge ? ring : merge);
 }
 
@@ -912,14 +983,22 @@ extern "C" int eredu_attn_prefill(const void* q, const void* k_cache, const void
   return static_cast<int>(e);
 }
 
-template <int DK, int DV, int MT, bool EXT, bool POOL = false>
+static int multiprocessors() {
+  static int count[kMaxDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  if (count[dev] == 0) cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev);
+  return count[dev];
+}
+
+template <int DK, int DV, int MT, bool EXT, bool POOL = false, int NW = 4>
 static cudaError_t launch_decode(const AttnParams& p, dim3 grid, cudaStream_t stream) {
   static bool cfg[kMaxDevices] = {};
-  if (!configure_once(cfg, attn_decode_kernel<DK, DV, MT, EXT, POOL>, decode_smem<DK, DV, MT>())) return cudaErrorInvalidValue;
+  if (!configure_once(cfg, attn_decode_kernel<DK, DV, MT, EXT, POOL, NW>, decode_smem<DK, DV, MT, NW>())) return cudaErrorInvalidValue;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = grid;
-  lc.blockDim = dim3(128);
-  lc.dynamicSmemBytes = decode_smem<DK, DV, MT>();
+  lc.blockDim = dim3(32 * NW);
+  lc.dynamicSmemBytes = decode_smem<DK, DV, MT, NW>();
   lc.stream = stream;
   cudaLaunchAttribute attr[2];
   int nattr = 0;
@@ -937,7 +1016,7 @@ static cudaError_t launch_decode(const AttnParams& p, dim3 grid, cudaStream_t st
   }
   lc.attrs = attr;
   lc.numAttrs = nattr;
-  const cudaError_t e = cudaLaunchKernelEx(&lc, attn_decode_kernel<DK, DV, MT, EXT, POOL>, p);
+  const cudaError_t e = cudaLaunchKernelEx(&lc, attn_decode_kernel<DK, DV, MT, EXT, POOL, NW>, p);
   eredu_count_launches(1);
   return e;
 }
@@ -961,6 +1040,13 @@ static int launch_decode_all(AttnParams p, int batch, int q_per_seq, int n_q_hea
   p.cluster_reduce = (p.splits > 1 && p.splits <= kMaxClusterSplits && !force_scratch) ? 1 : 0;
   if (p.splits > 1 && !p.cluster_reduce && (p.part_o == nullptr || p.part_ml == nullptr || p.counters == nullptr)) return -1;
   dim3 grid(p.splits, n_kv_heads, batch);
+  // CTAs of eight warps, one to an SM, where they run in one round: a warp then walks half the pages one after the other. One sequence of
+  // 2048, 32 heads of 128 over 8: 8.8 us with four warps, 7.5 with eight; 32 sequences of 1024, 32 heads over 4: 21.6 and 16.9. A
+  // second round costs more (32 of 2048 over 8 heads: 47 and 51), and clusters leave parts of a GPC empty (two of 2048 with eight splits
+  // 10.2 and 14.9, with six 11.2 and 9.5).
+  const int sms = multiprocessors();
+  const int round = !p.cluster_reduce || p.splits <= 2 ? sms : p.splits <= 4 ? sms * 7 / 8 : sms * 2 / 3;
+  const bool wide = p.splits * n_kv_heads * batch <= round;
   const int settled = p.settled;
   for (int t0 = 0; t0 < q_per_seq; t0 += t_per) {
     p.t0 = t0;
@@ -989,7 +1075,9 @@ static int launch_decode_all(AttnParams p, int batch, int q_per_seq, int n_q_hea
         ER_POOLED(64, 64);
       }
 #undef ER_POOLED
-    } else if (plain && key_dim == 128) ER_DECODE(128, 128, false);
+    } else if (plain && one && wide) e = key_dim == 128 ? launch_decode<128, 128, 1, false, false, 8>(p, grid, stream)
+                                                       : launch_decode<64, 64, 1, false, false, 8>(p, grid, stream);
+    else if (plain && key_dim == 128) ER_DECODE(128, 128, false);
     else if (plain) ER_DECODE(64, 64, false);
     else if (key_dim > 64 && value_dim > 64) ER_DECODE(128, 128, true);
     else if (key_dim > 64) ER_DECODE(128, 64, true);

@@ -180,6 +180,13 @@ class CausalLM:
         self.residency = None  # set by runtime.weight_residency when the layers live in host memory
         self.observer = None   # runtime.inspection.ActivationObserver for observed (eager) passes
 
+    @property
+    def decode_rows(self) -> int:
+        """Query heads that share a key / value head where decode attention is the plain kernel's in every layer, else 0 (see ops.decode_splits)."""
+        plain = (self.family is None and not self.cfg.is_mla and self.cfg.head_dim in (64, 128) and getattr(self, "g4", None) is None
+                 and getattr(self, "mg", None) is None)
+        return self.n_q_local // self.n_kv_local if plain else 0
+
     # ------------------------------------------------------------------------------------------ layer
     def _linear(self, lw: LayerWeights, role: str, x, w, bias=None, residual=None):
         q = lw.qlin.get(role)

@@ -620,11 +620,19 @@ CLUSTER_SPLITS = 8      # splits the decode kernel combines through distributed 
 FUSED_ROPE_MAX_NEW = 8  # new tokens per sequence the fused RoPE + append decode path takes
 
 
-def decode_splits(batch, n_kv, max_kv_len, sm_count=148):
+def decode_splits(batch, n_kv, max_kv_len, sm_count=148, rows=0):
     """Split-KV factor: enough CTAs to fill the GPU once (a second wave costs more than it returns: the CTAs of the
-    following kernel are already resident under programmatic dependent launch), at least 8 pages per split."""
+    following kernel are already resident under programmatic dependent launch), at least 8 pages per split.
+    ``rows``: query rows that share a key / value head where the caller knows that the plain kernel takes them (head sizes 64 and 128, at
+    most 16 rows), else 0. Its CTAs of eight warps run one to an SM, and as many splits as that allows are the best there are (us with the
+    splits of either rule: one sequence of 4096, 32 heads over 8, 13.8 with 32 and 10.2 with 8; eight of 1024, 64 heads over 8, 15.2 with 4 and
+    13.3 with 2; 32 of 1024, 32 heads over 4, 21.6 with 2 and 16.9 with 1)."""
     ctas = max(1, batch * n_kv)
     pages = max(1, (max_kv_len + PAGE - 1) // PAGE)
+    if 0 < rows <= 16 and ctas <= sm_count:
+        # clusters of more than two CTAs, and of more than four, leave parts of a GPC empty
+        want = max(s for s in range(1, CLUSTER_SPLITS + 1) if ctas * s <= (sm_count if s <= 2 else sm_count * 7 // 8 if s <= 4 else sm_count * 2 // 3) or s == 1)
+        return max(1, min(want, pages // 8))
     want = max(1, (_SPLIT_WAVES * sm_count) // ctas)
     splits = int(max(1, min(want, pages // 8 if pages >= 8 else 1, 32)))
     # up to CLUSTER_SPLITS splits combine inside a thread-block cluster (no scratch, no second pass over global memory):

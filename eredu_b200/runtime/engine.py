@@ -361,7 +361,7 @@ class Engine:
                 h[i, :len(tail)] = tail
             hist = self._t(h, torch.int32)
         max_len = int(pos.max()) + 1 + max(s.max_new_tokens for s in seqs)
-        splits = ops.decode_splits(B, self.model.n_kv_local, max_len, self.sm_count) if self.cuda else 1
+        splits = ops.decode_splits(B, self.model.n_kv_local, max_len, self.sm_count, self.model.decode_rows) if self.cuda else 1
         st = {
             "B": B,
             "seqs": list(seqs),
@@ -405,7 +405,7 @@ class Engine:
             logit_rows=self._t(np.asarray(logit_rows, dtype=np.int64), torch.int64))
         if decode_form and max(counts) == 1:
             longest = int(lens.max())
-            splits = ops.decode_splits(len(seqs), self.model.n_kv_local, longest, self.sm_count) if self.cuda else 1
+            splits = ops.decode_splits(len(seqs), self.model.n_kv_local, longest, self.sm_count, self.model.decode_rows) if self.cuda else 1
             return ForwardBatch(**common, is_prefill=False, q_per_seq=1, max_kv_len=longest, splits=splits)
         cu = np.concatenate(([0], np.cumsum(counts))).astype(np.int32)
         return ForwardBatch(**common, is_prefill=True, cu_q=self._t(cu, torch.int32), max_q_len=max(counts),
@@ -482,7 +482,7 @@ class Engine:
         dev = self.device
         rows = pack_rows([SamplingParams(temperature=0.0)] * B, [1] * B, hist_lens=[0] * B, stream_ids=[0] * B)
         max_len = max_context or self.max_seq_len
-        splits = ops.decode_splits(B, self.model.n_kv_local, max_len, self.sm_count) if self.cuda else 1
+        splits = ops.decode_splits(B, self.model.n_kv_local, max_len, self.sm_count, self.model.decode_rows) if self.cuda else 1
         st = {
             "B": B, "seqs": [None] * B, "slotted": True,
             "token_ids": torch.zeros(B, dtype=torch.int32, device=dev),

@@ -121,6 +121,33 @@ def test_four_bit_rows_at_the_borders_of_the_plan(M, N, K, group, gated):
     test_four_bit_rows_of_few_tokens(M, N, K, group, gated)
 
 
+@pytest.mark.parametrize("B,n_q,n_kv,D,splits", [(1, 32, 8, 128, 8), (1, 4, 4, 64, 5), (2, 32, 8, 128, 6), (2, 32, 8, 128, 8), (32, 32, 4, 128, 1),
+                                                 (37, 64, 4, 128, 1), (38, 64, 4, 128, 1), (3, 16, 1, 64, 3)])
+@pytest.mark.parametrize("length", [1, 16, 17, 128, 129, 1025])
+def test_decode_attention_of_one_new_token(B, n_q, n_kv, D, splits, length):
+    """Grids on either side of where CTAs have eight warps; contexts that leave splits or warps without a page, new tokens that open a page; one
+    sequence whose token is not kept; pages, tables and lengths read ahead of the projection."""
+    n_pages = length // 16 + 1
+    qkv = torch.randn(B, (n_q + 2 * n_kv) * D, device=DEV).bfloat16()
+    kc, vc = (torch.randn(B * n_pages + 1, n_kv, 16, D, device=DEV).bfloat16() for _ in range(2))
+    table = (torch.randperm(B * n_pages, device=DEV) + 1).int().view(B, n_pages)
+    lens = torch.full((B,), length, device=DEV, dtype=torch.int32)
+    lens[B // 2:] = max(1, length - 5)
+    slots = table.gather(1, ((lens - 1) // 16).long()[:, None])[:, 0].long() * 16 + (lens - 1) % 16
+    if B > 1:
+        slots[1] = -1
+    inv = 1.0 / (10000.0 ** (torch.arange(0, D, 2, device=DEV).float() / D))
+    norm = torch.rand(D, device=DEV) + 0.5
+    kr, vr = kc.clone(), vc.clone()
+    got = ops.attention_decode_rope(qkv, kc, vc, table, lens, 1, D ** -0.5, lens - 1, slots, inv, n_q, n_kv, D, attn_factor=1.25, q_norm_w=norm,
+                                    splits=splits, settled=True)
+    q = ops.rope_kv_ref(qkv, lens - 1, slots, inv, kr, vr, n_q, n_kv, D, attn_factor=1.25, q_norm_w=norm)
+    ref = ops.attention_ref(q, kr, vr, table, lens, [1] * B, D ** -0.5)
+    assert torch.equal(vc, vr) and rel_l2(kc, kr) < BF16
+    # queries, probabilities and the result are rounded
+    assert rel_l2(got.view(B, -1), ref.view(B, -1)) < 3 * BF16
+
+
 @pytest.mark.parametrize("M", [129, 161, 300, 777])
 @pytest.mark.parametrize("N,K", [(128, 1024), (136, 1024), (264, 1016), (392, 1088), (3848, 4096)])
 def test_projections_of_prompts_on_pairs_of_ctas(M, N, K):
