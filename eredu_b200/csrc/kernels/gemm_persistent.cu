@@ -179,8 +179,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (the warp waits, one lane issues)
-    // both operands are re-read by other CTAs from L2; the weights of a decode step are not
-    const uint64_t pol_w = BOX == 16 ? l2_policy_evict_first() : l2_policy_evict_last();
+    // both operands are re-read by other CTAs from L2; the weights of experts, and of a single token tile, are not
+    const uint64_t pol_w = GROUPED || p.m_tiles == 1 ? l2_policy_evict_first() : l2_policy_evict_last();
     const uint64_t pol_x = l2_policy_evict_last();
     const bool one = elect_one();
     int s = 0, issued = 0;

@@ -131,7 +131,7 @@ __device__ __forceinline__ float residual_at(const GemmParams& p, int m, int n) 
 // `rv`: the residual value of the element (0 when there is none), loaded by the caller ahead of time so that
 // the load does not sit between two dependent stores.
 template <bool DUAL>
-__device__ __forceinline__ float epilogue_store(const GemmParams& p, float g, float u, int m, int n, float scale, float rv) {
+__device__ __forceinline__ float epilogue_value(const GemmParams& p, float g, float u, int n, float scale, float rv) {
   g *= scale;
   if (DUAL) u *= scale;
   if (p.bias != nullptr) {
@@ -139,7 +139,12 @@ __device__ __forceinline__ float epilogue_store(const GemmParams& p, float g, fl
     g += __bfloat162float(b[n]);
     if (DUAL) u += __bfloat162float(b[p.N + n]);
   }
-  float v = (DUAL ? gated_act(p, g, u) : plain_act(p, g)) + rv;
+  return (DUAL ? gated_act(p, g, u) : plain_act(p, g)) + rv;
+}
+
+template <bool DUAL>
+__device__ __forceinline__ float epilogue_store(const GemmParams& p, float g, float u, int m, int n, float scale, float rv) {
+  const float v = epilogue_value<DUAL>(p, g, u, n, scale, rv);
   if (p.out_fp32) {
     static_cast<float*>(p.y)[static_cast<size_t>(m) * p.ldy + n] = v;
     return v;
@@ -376,13 +381,47 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     }
   };
 
+  // Split sums without a collective: a warp finishes a column at a time, a lane four of its rows (16 bytes of every CTA's partial sums, 8 of
+  // the residual and of the result). With a row a thread and a column after the other, each of them waited for its remote loads: 0.4 us a
+  // column (4096 x 14336: 23.5 us with 45 tokens, 20.9 now; 6144 x 4096 with 64 18.4 and 13.1).
+  constexpr bool kQuads = SPLIT && COMM == COMM_NONE;
+  constexpr int kAhead = 4;
+  const int qn = tile_n * 128 + lane * 4;      // first of the lane's rows
+  const bool whole = (p.N & 3) == 0 && (p.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 &&
+                     (p.residual == nullptr || ((p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0));
+  uint2 quad_res[kAhead];
+  auto quad_residual = [&](int c) {
+    uint2 r = make_uint2(0u, 0u);
+    if (p.residual == nullptr || c >= m_end || qn >= p.N) return r;
+    const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(p.residual) + static_cast<size_t>(m_base + c) * p.ldr + qn;
+    if (whole) return *reinterpret_cast<const uint2*>(src);
+    const unsigned short* bits = reinterpret_cast<const unsigned short*>(src);
+    uint32_t e[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = qn + i < p.N ? bits[i] : 0u;
+    r.x = e[0] | e[1] << 16;
+    r.y = e[2] | e[3] << 16;
+    return r;
+  };
+
   if (warp >= 2) {
     if (p.ssq_in != nullptr) {
       for (int c = et; c < TN; c += 128) {
         float t = 0.f;
         if (m_base + c < m_limit) {
           const float* src = p.ssq_in + static_cast<size_t>(m_base + c) * p.ssq_parts;
-          for (int j = 0; j < p.ssq_parts; ++j) t += src[j];
+          int j = 0;
+          if ((p.ssq_parts & 3) == 0) {     // the same sum with eight 16-byte loads on their way
+#pragma unroll 8
+            for (; j < p.ssq_parts; j += 4) {
+              const float4 v = *reinterpret_cast<const float4*>(src + j);
+              t += v.x;
+              t += v.y;
+              t += v.z;
+              t += v.w;
+            }
+          }
+          for (; j < p.ssq_parts; ++j) t += src[j];
         }
         s_scale[c] = rsqrtf(t * p.norm_inv_dim + p.norm_eps);
       }
@@ -397,11 +436,15 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           const int c = 2 * (own_first + j * own_step);
           if (c < m_end) rpre[2 * j] = residual_at(p, m_base + c, n);
           if (c + 1 < m_end) rpre[2 * j + 1] = residual_at(p, m_base + c + 1, n);
-        } else if (SPLIT) {
+        } else if (SPLIT && COMM != COMM_NONE) {
           const int c = own_first + j * own_step;
           if (c < m_end) rpre[j] = residual_at(p, m_base + c, n);
         }
       }
+    }
+    if (kQuads) {
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) quad_res[j] = quad_residual(split + (q + 4 * j) * nsplit);
     }
     acc_ok = (niter > 0) && mbar_wait(accum_bar, 0, p.status, kStatusAccumTimeout);
     acc_ok = __all_sync(0xffffffffu, acc_ok);
@@ -410,7 +453,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     if (acc_ok) {
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
-      for (int c0 = 0; c0 < TN; c0 += 16) {
+      for (int c0 = 0; c0 < (kQuads ? m_end : TN); c0 += 16) {
         uint32_t g[16];
         uint32_t u[16];
         tmem_ld16(taddr + c0, g);
@@ -540,6 +583,82 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           }
         }
       }
+    }
+  } else if (kQuads) {
+    if (warp >= 2) {
+      const uint32_t red_addr = smem_u32(red) + lane * 16u;
+      uint32_t peers[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) peers[r] = mapa_shared(red_addr, static_cast<uint32_t>(r < nsplit ? r : 0));
+      auto remote = [](uint32_t addr) {
+        float4 v;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+        return v;
+      };
+      // all remote loads of a column are issued together; the sum runs in cluster-rank order (deterministic)
+      auto sum_of = [&](int c) {
+        float4 part[8], t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (r < nsplit) part[r] = remote(peers[r] + c * 512u);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (r < nsplit) {
+            t.x += part[r].x;
+            t.y += part[r].y;
+            t.z += part[r].z;
+            t.w += part[r].w;
+          }
+        return t;
+      };
+      auto finish_quad = [&](int c, const float4& g4, const float4& u4, const uint2& res) {
+        const float g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+        const float rv[4] = {bf16_lo(res.x), bf16_hi(res.x), bf16_lo(res.y), bf16_hi(res.y)};
+        const float sc = p.ssq_in != nullptr ? s_scale[c] : 1.f;
+        const size_t at = static_cast<size_t>(m_base + c) * p.ldy + qn;
+        float v[4], sq = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = qn + i < p.N ? epilogue_value<DUAL>(p, g[i], u[i], qn + i, sc, rv[i]) : 0.f;
+        if (p.out_fp32) {
+          float* dst = static_cast<float*>(p.y) + at;
+          if (whole && qn < p.N) {
+            *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (qn + i < p.N) dst[i] = v[i];
+          }
+        } else {
+          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.y) + at;
+          const uint2 o = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+          if (whole && qn < p.N) {
+            *reinterpret_cast<uint2*>(dst) = o;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (qn + i < p.N) dst[i] = __float2bfloat16(v[i]);
+          }
+          v[0] = bf16_lo(o.x);
+          v[1] = bf16_hi(o.x);
+          v[2] = bf16_lo(o.y);
+          v[3] = bf16_hi(o.y);
+        }
+        if (p.ssq_out != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sq += v[i] * v[i];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+          if (lane == 0) p.ssq_out[static_cast<size_t>(m_base + c) * gridDim.x + tile_n] = sq;
+        }
+      };
+      const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        const int c = split + (q + 4 * j) * nsplit;
+        if (c < m_end) finish_quad(c, sum_of(c), DUAL ? sum_of(TN + c) : none, quad_res[j]);   // warp-uniform
+      }
+      for (int c = split + (q + 4 * kAhead) * nsplit; c < m_end; c += 4 * nsplit)
+        finish_quad(c, sum_of(c), DUAL ? sum_of(TN + c) : none, quad_residual(c));
     }
   } else if (SPLIT) {
     if (warp >= 2) {
@@ -754,7 +873,7 @@ template <int TN, bool DUAL, int COMM = COMM_NONE>
 static cudaError_t launch_gemm_split(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p,
                                      int n_tiles, int m_tiles, int nsplit, cudaStream_t stream) {
   if (nsplit > 1) {
-    if constexpr (TN <= 64) return launch_gemm<TN, DUAL, true, COMM>(tmW, tmX, p, n_tiles, m_tiles, nsplit, stream);
+    if constexpr (TN <= 64 || COMM == COMM_NONE) if constexpr (TN <= 128) return launch_gemm<TN, DUAL, true, COMM>(tmW, tmX, p, n_tiles, m_tiles, nsplit, stream);
   }
   return launch_gemm<TN, DUAL, false, COMM>(tmW, tmX, p, n_tiles, m_tiles, 1, stream);
 }
@@ -815,9 +934,15 @@ static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K,
 
 // K splits of a launch of [128 weight rows x tn tokens] tiles of which an SM takes ctas_per_sm.
 static int pick_split(int M, int N, int K, int tn, int ctas_per_sm, int sm_count) {
-  if (tn > 64) return 1;
+  if (tn > 128) return 1;
   const int tiles = ((N + 127) / 128) * ((M + tn - 1) / tn);
   const int kblocks = (K + 63) / 64;
+  if (tn == 128) {
+    // One CTA to an SM: clusters of eight find two thirds of the SMs and of four seven eighths; what splits less goes to the persistent kernel.
+    // 100 tokens: 4096 x 4096 22.6 us unsplit, 19.3 there, 14.3 split four times, 4096 x 14336 52.9, 52.5 and 26.3, 2048 x 4096 21.9, 18.6 and 12.4
+    // (eight times 16.3); 6144 x 4096 23.5 and 20.3, split twice 21.1, 2 x 14336 x 4096 59 and 52, 2 x 8192 x 2048 34 and 20.8, split twice 26.4.
+    return kblocks < 16 ? 1 : tiles * 8 <= sm_count / 2 ? 8 : tiles * 4 <= sm_count * 7 / 8 ? 4 : 1;
+  }
   int s = 1;
   // Split while the grid still fits the CTAs an SM takes: besides streaming the weights in parallel, a split CTA
   // finishes only every s-th token column, and the serial per-column epilogue is what a small GEMM pays for.
@@ -829,7 +954,7 @@ static int pick_split(int M, int N, int K, int tn, int ctas_per_sm, int sm_count
 // tiles of 64 tokens count one CTA an SM, routers of prompts are not split, and one or two tokens may take the rows kernel.
 extern "C" int eredu_gemm_pick_split(int M, int N, int K, int sm_count) {
   const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-  return pick_split(M, N, K, tn, 2, sm_count);
+  return tn > 64 ? 1 : pick_split(M, N, K, tn, 2, sm_count);
 }
 
 // Y = X W^T (+bias) (+residual), or with dual != 0: Y = silu(X Wg^T) * (X Wu^T) where Wg = W[0:N],
@@ -857,7 +982,8 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
     tn = 64;
     while (tn > 16 && ((N + 127) / 128) * ((M + tn / 2 - 1) / (tn / 2)) <= ctas) tn >>= 1;
   }
-  if (tn == 256 && force_split <= 1 && persistent_enabled()) {
+  const bool unsplit = tn == 128 && force_split <= 0 && pick_split(M, N, K, tn, 1, sm_count > 0 ? sm_count : 148) == 1;
+  if (((tn == 256 && force_split <= 1) || unsplit) && persistent_enabled()) {
     // prefill-sized: persistent kernel with double-buffered accumulators
     const int pr = launch_gemm_persistent(X, W, Y, residual, bias, M, N, K, ldx, ldw, ldy, ldr, w_rows, dual, dual_row_offset,
                                           sm_count, status, ssq_in, ssq_parts, norm_eps, norm_dim, ssq_out, act, act_a, act_b, out_fp32,

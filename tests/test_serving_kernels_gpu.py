@@ -148,6 +148,28 @@ def test_decode_attention_of_one_new_token(B, n_q, n_kv, D, splits, length):
     assert rel_l2(got.view(B, -1), ref.view(B, -1)) < 3 * BF16
 
 
+@pytest.mark.parametrize("M", [5, 33, 64, 65, 100, 128])
+@pytest.mark.parametrize("N,K", [(130, 1024), (131, 2048), (512, 1088), (2176, 1024), (4128, 1024), (4736, 1024)])
+@pytest.mark.parametrize("odd", [False, True])
+def test_split_sums_of_several_tokens(M, N, K, odd):
+    """Rows that are no whole quads of columns, residuals whose rows start anywhere, columns beyond the tokens, one CTA and clusters of two, four and
+    eight, and the kernel that takes over where K is not split."""
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = (torch.randn(2 * N, K, device=DEV) * K ** -0.5).bfloat16()
+    bias = torch.randn(N, device=DEV).bfloat16()
+    res = torch.randn(M, N + 8, device=DEV).bfloat16()[:, 1:N + 1] if odd else torch.randn(M, N, device=DEV).bfloat16()
+    y = x.double() @ w.double().t()
+    got, ssq = ops.linear(x, w[:N], bias=bias, residual=res, want_ssq=True)
+    assert rel_l2(got, y[:, :N] + bias.double() + res.double()) < BF16
+    assert rel_l2(ssq.sum(-1), got.double().square().sum(-1)) < 1e-5
+    assert rel_l2(ops.linear(x, w[:N], out_dtype=torch.float32), y[:, :N]) < BF16 / 256
+    scale = (got.double().square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    if N % 8 == 0:
+        w2 = (torch.randn(2 * 264, N, device=DEV) * N ** -0.5).bfloat16()
+        z = (got.double() * scale) @ w2.double().t()
+        assert rel_l2(ops.gated_linear(got, w2, 264, row_ssq=ssq, norm_eps=1e-6), moe_ops.gated_act_ref(z[:, :264].float(), z[:, 264:].float())) < BF16
+
+
 @pytest.mark.parametrize("M", [129, 161, 300, 777])
 @pytest.mark.parametrize("N,K", [(128, 1024), (136, 1024), (264, 1016), (392, 1088), (3848, 4096)])
 def test_projections_of_prompts_on_pairs_of_ctas(M, N, K):
