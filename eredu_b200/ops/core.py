@@ -102,28 +102,45 @@ def linear(x, w, bias=None, residual=None, out_dtype=None, out=None, force_split
             x = x.float() * torch.rsqrt(row_ssq.sum(-1, keepdim=True) / x.shape[1] + norm_eps)
         y = linear_ref(x, w, bias, residual, out_dtype or w.dtype, activation)
         return (y, y.float().pow(2).sum(-1, keepdim=True)) if want_ssq else y
-    if x.dtype == torch.float32 or not (_tma_rows(x) and _tma_rows(w)):
+    at = _tma_operands(x, w)
+    if at is None:
         assert residual is None and row_ssq is None and not want_ssq, "the CUDA-core linear has no norm or residual fusion"
         return _linear_simt(x, w, bias, out_dtype or x.dtype, activation, out)
-    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16, "CUDA linear is bf16"
     M, K = x.shape
     N = w.shape[0]
+    dev = x.device
     out_dtype = out_dtype or torch.bfloat16
     assert out_dtype in (torch.bfloat16, torch.float32)
-    assert x.stride(1) == 1 and w.stride(1) == 1
     if out is None:
-        out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+        out = torch.empty((M, N), dtype=out_dtype, device=dev)
     ssq_in, parts, eps, dim, ssq_out = _norm_args(x, row_ssq, norm_eps, want_ssq, N)
     if M == 0:
         return (out, ssq_out) if want_ssq else out
+    flags = 1 if dynamic_weight else 0
+    above = below = 0.0
+    if activation is not None:
+        flags |= 8 if xielu else 2
+        if xielu:
+            above, below = xielu.above, xielu.below
     code = lib().eredu_gemm_bf16(
-        ptr(x), ptr(w), ptr(out), ptr(residual), ptr(bias), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-        residual.stride(0) if residual is not None else 0, w.shape[0], 0, 0, 1 if out_dtype == torch.float32 else 0,
-        force_split, _sm_count(x.device), ptr(status_word(x.device)), ptr(ssq_in), parts, eps, dim, ptr(ssq_out),
-        (1 if dynamic_weight else 0) | (2 if activation == "relu2" else 8 if xielu else 0), xielu.above if xielu else 0.0,
-        xielu.below if xielu else 0.0, stream_ptr(x.device))
+        at[0], at[1], out.data_ptr(), None if residual is None else residual.data_ptr(), None if bias is None else bias.data_ptr(), M, N, K, at[2], at[3],
+        out.stride(0), 0 if residual is None else residual.stride(0), N, 0, 0, 1 if out_dtype == torch.float32 else 0, force_split, _sm_count(dev),
+        status_word(dev).data_ptr(), None if ssq_in is None else ssq_in.data_ptr(), parts, eps, dim, None if ssq_out is None else ssq_out.data_ptr(),
+        flags, above, below, stream_ptr(dev))
     check(code, "eredu_gemm_bf16")
     return (out, ssq_out) if want_ssq else out
+
+
+def _tma_operands(x, w):
+    """(address of x, of w, row pitch of x, of w) of bf16 matrices whose rows TMA descriptors can describe; None for fp32 operands and other rows."""
+    if x.dtype == torch.float32:
+        return None
+    (x0, x1), (w0, w1) = x.stride(), w.stride()
+    xp, wp, size = x.data_ptr(), w.data_ptr(), w.element_size()
+    if x1 != 1 or w1 != 1 or (x0 * 2) % 16 or (w0 * size) % 16 or (xp | wp) % 16:
+        return None
+    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16, "CUDA linear is bf16"
+    return xp, wp, x0, w0
 
 
 def _tma_rows(t) -> bool:
@@ -162,21 +179,21 @@ def gated_linear(x, w_gate_up, inter, bias=None, out=None, force_split=0, row_ss
         if row_ssq is not None:
             x = x.float() * torch.rsqrt(row_ssq.sum(-1, keepdim=True) / x.shape[1] + norm_eps)
         return gated_linear_ref(x, w_gate_up, inter, bias, w_gate_up.dtype, activation)
-    if x.dtype == torch.float32 or not (_tma_rows(x) and _tma_rows(w_gate_up)):
+    at = _tma_operands(x, w_gate_up)
+    if at is None:
         assert row_ssq is None, "the CUDA-core linear has no norm fusion"
         return _linear_simt(x, w_gate_up, bias, x.dtype, "gated_" + activation, out)
-    assert x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16
     M, K = x.shape
+    dev = x.device
     if out is None:
-        out = torch.empty((M, inter), dtype=torch.bfloat16, device=x.device)
+        out = torch.empty((M, inter), dtype=torch.bfloat16, device=dev)
     if M == 0:
         return out
     ssq_in, parts, eps, dim, _ = _norm_args(x, row_ssq, norm_eps, False, inter)
     code = lib().eredu_gemm_bf16(
-        ptr(x), ptr(w_gate_up), ptr(out), None, ptr(bias), M, inter, K, x.stride(0), w_gate_up.stride(0),
-        out.stride(0), 0, w_gate_up.shape[0], 1, inter, 0, force_split, _sm_count(x.device),
-        ptr(status_word(x.device)), ptr(ssq_in), parts, eps, dim, None,
-        (1 if dynamic_weight else 0) | (4 if activation == "relu" else 0), 0.0, 0.0, stream_ptr(x.device))
+        at[0], at[1], out.data_ptr(), None, None if bias is None else bias.data_ptr(), M, inter, K, at[2], at[3], out.stride(0), 0, w_gate_up.shape[0], 1,
+        inter, 0, force_split, _sm_count(dev), status_word(dev).data_ptr(), None if ssq_in is None else ssq_in.data_ptr(), parts, eps, dim, None,
+        (1 if dynamic_weight else 0) | (4 if activation == "relu" else 0), 0.0, 0.0, stream_ptr(dev))
     check(code, "eredu_gemm_bf16(dual)")
     return out
 
