@@ -352,6 +352,21 @@ def test_expert_plan_keeps_the_order_of_the_routes(E, e0, e1, routes, k):
     assert plan.seg.tolist() == [int(((flat >= e0) & (flat < e0 + i)).sum()) for i in range(e1 - e0 + 1)]
 
 
+@pytest.mark.parametrize("T,E,e0,n_local,k", [(1, 128, 0, 128, 8), (4, 128, 0, 128, 8), (5, 128, 0, 128, 8), (1, 512, 128, 256, 10), (3, 8, 2, 4, 2),
+                                              (16, 4, 0, 4, 2), (17, 4, 0, 4, 1), (32, 64, 0, 64, 1), (1, 16, 12, 4, 1)])
+def test_routes_of_few_tokens_are_planned_alike(T, E, e0, n_local, k):
+    """Up to 32 routes, compared by the lanes of a warp, against the general plan of the same routes; experts elsewhere, and none at all."""
+    logits, x = torch.randn(T, E, device=DEV), torch.randn(T, 256, device=DEV).bfloat16()
+    if T == 1 and E == 16:
+        logits[0, 3] = 9.0
+    ids, _, plan, xp = moe_ops.route_plan_gather(logits, x, k, "softmax", True, 1.0, None, e0, n_local)
+    want = moe_ops.ExpertPlan(ids, k, e0, e0 + n_local, plan.tile, T * k)
+    rows = int(want.counts[0])
+    assert torch.equal(plan.counts, want.counts) and torch.equal(plan.work, want.work) and torch.equal(plan.seg, want.seg)
+    assert torch.equal(plan.route_pos, want.route_pos) and torch.equal(plan.row_token[:rows], want.row_token[:rows])
+    assert torch.equal(xp[:rows], x[want.row_token[:rows].long()])
+
+
 @pytest.mark.parametrize("E,e0,e1,routes,k", [(8, 0, 8, 3000, 2), (9, 0, 9, 3000, 3), (20, 4, 20, 130, 2)])
 def test_expert_plan_of_few_experts(E, e0, e1, routes, k):
     """On either side of where lanes find their like by values instead of bits; batches of routes that end early."""
