@@ -82,6 +82,9 @@ struct GemmParams {
 //            output at the rank's column offset.
 enum { COMM_NONE = 0, COMM_AR = 1, COMM_AG = 2 };
 
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 template <int TN, bool DUAL>
@@ -97,7 +100,9 @@ struct GemmCfg {
   static constexpr int kAccCols = TN * (DUAL ? 2 : 1);
   static constexpr int kTmemCols = kAccCols <= 32 ? 32 : kAccCols <= 64 ? 64 : kAccCols <= 128 ? 128 : kAccCols <= 256 ? 256 : 512;
   static constexpr int kCtrlBytes = 1024;
-  static constexpr int kSmemBytes = 1024 + kCtrlBytes + kStages * kStageBytes;
+  // partial sums that the other CTAs of a split send for the one column this CTA finishes
+  static constexpr int kSentBytes = TN == 16 ? 8 * 128 * 4 * (DUAL ? 2 : 1) : 0;
+  static constexpr int kSmemBytes = 1024 + kCtrlBytes + kStages * kStageBytes + kSentBytes;
   static_assert(kStages >= 2, "pipeline too shallow");
 };
 
@@ -179,8 +184,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);            // [kStages]
   uint64_t* empty_bar = full_bar + Cfg::kStages;                     // [kStages]
   uint64_t* accum_bar = empty_bar + Cfg::kStages;                    // [1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);  // [1]
+  uint64_t* sent_bar = accum_bar + 1;                                // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sent_bar + 1);   // [1]
   uint8_t* stages = smem + Cfg::kCtrlBytes;
+  float* sent = reinterpret_cast<float*>(stages + Cfg::kStages * Cfg::kStageBytes);   // [8 ranks][gate, up][128 rows]
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -207,6 +214,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   const int kb0 = split * kb_per;
   const int kb1 = min(kblocks, kb0 + kb_per);
   const int niter = max(0, kb1 - kb0);
+  const int m_end = min(TN, m_limit - m_base);
+  // Split sums without a collective (kQuads). Of no more columns than CTAs every CTA finishes one at the most: the others send it their
+  // partial sums (st.async) and are done. That spares the barrier before the sums are read, their way back and the barrier that kept
+  // everybody until they were: 6144 x 4096 with one token 11.5 -> 10.7 us, 2048 x 8192 10.1 -> 9.0, 2 x 8192 x 2048 12.0 -> 11.1, a decode step of 8B
+  // 3429 -> 3316 (four, eight layers). Expert items lost by it (2152 -> 2171 a step): the CTAs that leave early make room for some of the next GEMM's.
+  constexpr bool kQuads = SPLIT && COMM == COMM_NONE;
+  const bool pushed = kQuads && TN == 16 && m_end <= nsplit && p.work == nullptr;
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmW);
@@ -216,6 +230,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(accum_bar, 1);
+    if (pushed) {
+      mbar_init(sent_bar, 1);
+      if (split < m_end) mbar_arrive_expect_tx(sent_bar, static_cast<uint32_t>((nsplit - 1) * 128 * 4 * (DUAL ? 2 : 1)));
+    }
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -227,6 +245,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  if (pushed) cluster_arrive_release();      // the other half: in front of the first store into another CTA
   // Weight tiles do not depend on the producer kernels: start them before the wait.
   int n_pre = 0;
   if (p.w_static && p.work == nullptr) {
@@ -345,7 +364,6 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   constexpr bool kCanStage = (TN >= 64) && !SPLIT && COMM == COMM_NONE;
   // Columns (tokens) of the tile whose final value this CTA produces: all of them, or with cluster split-K
   // every nsplit-th one (COMM_AR: every nsplit-th PAIR of columns, because partials travel as bf16x2).
-  const int m_end = min(TN, m_limit - m_base);
   const int own_first = SPLIT ? split : 0, own_step = SPLIT ? nsplit : 1;
   constexpr int kPre = 8;
   float rpre[2 * kPre];
@@ -384,7 +402,6 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // Split sums without a collective: a warp finishes a column at a time, a lane four of its rows (16 bytes of every CTA's partial sums, 8 of
   // the residual and of the result). With a row a thread and a column after the other, each of them waited for its remote loads: 0.4 us a
   // column (4096 x 14336: 23.5 us with 45 tokens, 20.9 now; 6144 x 4096 with 64 18.4 and 13.1).
-  constexpr bool kQuads = SPLIT && COMM == COMM_NONE;
   constexpr int kAhead = 4;
   const int qn = tile_n * 128 + lane * 4;      // first of the lane's rows
   const bool whole = (p.N & 3) == 0 && (p.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 &&
@@ -444,13 +461,35 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     }
     if (kQuads) {
 #pragma unroll
-      for (int j = 0; j < kAhead; ++j) quad_res[j] = quad_residual(split + (q + 4 * j) * nsplit);
+      for (int j = 0; j < kAhead; ++j) quad_res[j] = quad_residual(pushed ? (j == 0 ? split : TN) : split + (q + 4 * j) * nsplit);
     }
     acc_ok = (niter > 0) && mbar_wait(accum_bar, 0, p.status, kStatusAccumTimeout);
     acc_ok = __all_sync(0xffffffffu, acc_ok);
     trace_mark_thread(kTraceGemm, 5, 64);  // accumulator complete
     tc_fence_after_sync();
-    if (acc_ok) {
+    if (pushed) {
+      cluster_wait_acquire();
+      if (acc_ok) {
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+        uint32_t g[16], u[16];
+        tmem_ld16(taddr, g);
+        if (DUAL) tmem_ld16(taddr + TN, u);
+        tmem_wait_ld();
+        const uint32_t at = smem_u32(sent) + static_cast<uint32_t>(split * (DUAL ? 2 : 1) * 128 + row) * 4u, bar = smem_u32(sent_bar);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          if (c >= m_end) break;
+          if (c == split) {
+            sent[split * (DUAL ? 2 : 1) * 128 + row] = __uint_as_float(g[c]);
+            if (DUAL) sent[(split * 2 + 1) * 128 + row] = __uint_as_float(u[c]);
+          } else {
+            const uint32_t to = mapa_shared(at, static_cast<uint32_t>(c)), done = mapa_shared(bar, static_cast<uint32_t>(c));
+            st_async(to, g[c], done);
+            if (DUAL) st_async(to + 512u, u[c], done);
+          }
+        }
+      }
+    } else if (acc_ok) {
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
       for (int c0 = 0; c0 < (kQuads ? m_end : TN); c0 += 16) {
@@ -540,7 +579,9 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     }
   }
 
-  if (SPLIT) {
+  if (pushed) {
+    if (warp < 2) cluster_wait_acquire();    // arrived at the start
+  } else if (SPLIT) {
     // Every thread of every CTA of the cluster reaches both barriers, whatever happened above.
     cg::cluster_group cluster = cg::this_cluster();
     trace_mark_thread(kTraceGemm, 6, 64);  // partials staged
@@ -588,6 +629,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     if (warp >= 2) {
       const uint32_t red_addr = smem_u32(red) + lane * 16u;
       uint32_t peers[8];
+      if (pushed) epi_barrier();             // this CTA's own part is in place
 #pragma unroll
       for (int r = 0; r < 8; ++r) peers[r] = mapa_shared(red_addr, static_cast<uint32_t>(r < nsplit ? r : 0));
       auto remote = [](uint32_t addr) {
@@ -652,6 +694,28 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         }
       };
       const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (pushed) {
+        if (q == 2 && split < m_end && mbar_wait_warp(sent_bar, 0, p.status, kStatusAccumTimeout)) {     // the first epilogue warp
+          float4 g = none, u = none;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            if (r >= nsplit) break;
+            const float4 v = reinterpret_cast<const float4*>(sent + r * (DUAL ? 2 : 1) * 128)[lane];
+            g.x += v.x;
+            g.y += v.y;
+            g.z += v.z;
+            g.w += v.w;
+            if (DUAL) {
+              const float4 w = reinterpret_cast<const float4*>(sent + (r * 2 + 1) * 128)[lane];
+              u.x += w.x;
+              u.y += w.y;
+              u.z += w.z;
+              u.w += w.w;
+            }
+          }
+          finish_quad(split, g, u, quad_res[0]);
+        }
+      } else {
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
         const int c = split + (q + 4 * j) * nsplit;
@@ -659,6 +723,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
       for (int c = split + (q + 4 * kAhead) * nsplit; c < m_end; c += 4 * nsplit)
         finish_quad(c, sum_of(c), DUAL ? sum_of(TN + c) : none, quad_residual(c));
+      }
     }
   } else if (SPLIT) {
     if (warp >= 2) {
@@ -699,7 +764,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       if (COMM == COMM_NONE) publish_ssq(split, nsplit);
     }
   }
-  if (SPLIT) {
+  if (SPLIT && !pushed) {
     cg::cluster_group cluster = cg::this_cluster();
     trace_mark_thread(kTraceGemm, 8, 64);  // reduced and stored
     cluster.sync();
@@ -913,23 +978,22 @@ static bool staged_epilogue_ok(const void* Y, const void* residual, int N, int l
 }
 
 // Whether the call runs on gemv_rows_kernel: one or two tokens, whole 16-byte pieces of rows, whole CTAs of columns, weights that no
-// kernel just before this one writes - and few enough of them. With one token the kernel alone is the faster one at any size (2048 x
-// 2048 5.8 -> 4.5 us, 6144 x 4096 12.2 -> 10.9, 4096 x 14336 21.3 -> 20.4), but in a decode step, behind other kernels, the copy
-// rings of the tensor-core kernel start with 160 KB an SM where this one holds 64 KB a CTA: taking matrices up to 16 MB makes a
-// step of 16 layers 2048 wide 766 -> 728 us, up to 24 MB one of 8 expert layers 672 -> 628; 33 MB and above lose it again (759 us, and
-// 912 -> 945 for 8 layers 4096 wide). Two tokens are twice the arithmetic on the CUDA cores: 3072 x 2048 5.7 -> 5.1 us, 2560 x 2560
-// 6.2 -> 6.6, 5120 x 2048 6.8 -> 7.8.
+// kernel just before this one writes - and few enough of them. Microseconds of one token there and on the tensor-core kernel, which
+// splits K: 128 x 2048 2.4 / 3.3, 1024 x 1024 2.4 / 3.0, 2048 x 2048 3.7 / 3.8, 4096 x 1024 3.9 / 4.4, 4736 x 1024 4.1 / 6.4, 2048 x 4096 5.6 / 4.7, 3072 x 2048
+// 4.7 / 4.3; with sums of squares 512 x 2048 3.2 / 3.4, 1536 x 1536 3.7 / 3.5, 2048 x 2048 4.6 / 4.0. Two tokens: 1024 x 1024 2.7 / 3.0, 2048 x 1024
+// 3.4 / 3.4, 3072 x 2048 5.2 / 4.5. Behind other kernels the copy rings of the tensor-core kernel hold more than the registers here: with matrices
+// of 24 MB and less a step of 16 layers 2048 wide takes 2604 us, with these lines 2556, one of 8 expert layers 2112 and 2068.
 // Its CTAs have to run in one round, two to an SM: of short rows a second round costs more than the tensor-core kernel (5120 x 512 4.3
-// us there, 4.8 here; 12288 x 512 5.5 and 8.1); one token with rows of 2048 still gains (5120 x 2048 7.1 -> 6.7). With sums of squares
-// clusters of eight leave part of a GPC empty: one round is 7/8 of that, three quarters for two tokens (4608 x 512 4.3 and 6.3, 4096 x 512 with
-// two tokens 4.2 and 4.5), unless rows are long enough to make up for it (4608 x 1024 9.0 and 6.8).
+// us there, 4.8 here; 12288 x 512 5.5 and 8.1). With sums of squares clusters of eight leave part of a GPC empty: one round is 7/8 of that
+// (4608 x 512 4.3 and 6.3), unless rows are long enough to make up for it.
 static bool rows_kernel_takes(const void* X, const void* W, int M, int N, int K, int ldx, int ldw, int dual, int flags, int force_split, bool ssq,
                               int sm_count) {
   if (force_split > 0 || dual || M > 2 || (flags & 1) || K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || N % kRowsOut != 0) return false;
   if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) != 0) return false;
   const int ctas = N / kRowsOut, round = 2 * (sm_count > 0 ? sm_count : 148);
-  if (ssq ? ctas > round || (K < 1024 && ctas * 8 > round * (M == 1 ? 7 : 6)) : ctas > round && (M > 1 || K < 2048)) return false;
-  return static_cast<long long>(N) * K * 2 <= (M == 1 ? 24LL : 12LL) << 20;
+  if (ctas > round || (ssq && K < 1024 && ctas * 8 > round * 7)) return false;
+  const long long most = ssq ? (M == 1 ? 2 : 0) : K <= 1024 ? 12 : M == 1 ? 8 : 4;
+  return static_cast<long long>(N) * K * 2 <= most << 20;
 }
 
 // K splits of a launch of [128 weight rows x tn tokens] tiles of which an SM takes ctas_per_sm.
