@@ -268,7 +268,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
   uint8_t* raw_ring = a_ring + A * Cfg::kATile;            // [R][X tile | packed weights]
   constexpr int kRawOff = Cfg::kBTile, kScaleOff = Cfg::kBTile + Cfg::kRaw, kBiasOff = kScaleOff + Cfg::kSbBytes;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int tile_n = blockIdx.x, tile_m = blockIdx.y;
   const int nsplit = SPLIT ? gridDim.z : 1;
   const int split = SPLIT ? blockIdx.z : 0;
@@ -299,24 +299,25 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   pdl_launch_early();
   pdl_wait();
   pdl_launch_dependents();
 
   if (warp == 0) {
-    if (lane == 0) {
-      const uint64_t pol_w = l2_policy_evict_first();
-      const uint64_t pol_x = l2_policy_evict_last();
-      int issued = 0;
-      bool ok = true;
-      for (int it = 0; it < niter; ++it) {
-        const int s = it % R;
-        const uint32_t ph = (it / R) & 1;
-        ok = mbar_wait(&raw_empty[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
-        if (!ok) break;
-        uint8_t* st = raw_ring + s * Cfg::kRawSlot;
-        const int kb = kb0 + it;
+    // the warps that fetch and multiply run whole, one elected lane issues (see elect_one)
+    const uint64_t pol_w = l2_policy_evict_first();
+    const uint64_t pol_x = l2_policy_evict_last();
+    const bool one = elect_one();
+    int issued = 0, s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int it = 0; it < niter; ++it) {
+      ok = mbar_wait_warp(&raw_empty[s], ph ^ 1, p.status, kStatusSmemEmptyTimeout);
+      if (!ok) break;
+      uint8_t* st = raw_ring + s * Cfg::kRawSlot;
+      const int kb = kb0 + it;
+      if (one) {
         mbar_arrive_expect_tx(&raw_full[s], Cfg::kRaw + Cfg::kBTile + (FMT == QF_FP8 ? p.sb_rows * 512 : 2 * p.sb_rows * 256));
         // packed weights: byte tensor [N, row_bytes]; x coordinate in bytes (a multiple of 32)
         if (FMT == QF_AFFINE4) tma_load_3d_hint(st + kRawOff, &tmQ, 0, kb, tile_n * 8, &raw_full[s], pol_w);  // 8 tiles of 16 rows
@@ -327,31 +328,44 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
           tma_load_2d_hint(st + kScaleOff, &tmS, tile_n * 128, grow, &raw_full[s], pol_w);
           if (FMT != QF_FP8) tma_load_2d_hint(st + kBiasOff, &tmB, tile_n * 128, grow, &raw_full[s], pol_w);
         }
-        issued = it + 1;
       }
-      if (!ok) {
-        for (int it = max(0, issued - R); it < issued; ++it) mbar_wait(&raw_full[it % R], (it / R) & 1, nullptr, 0);
+      issued = it + 1;
+      if (++s == R) {
+        s = 0;
+        ph ^= 1;
       }
     }
+    if (!ok) {
+      for (int it = max(0, issued - R); it < issued; ++it) mbar_wait(&raw_full[it % R], (it / R) & 1, nullptr, 0);
+    }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, TN);
-      bool ok = true;
-      for (int it = 0; it < niter; ++it) {
-        const int rs = it % R, as = it % A;
-        ok = mbar_wait(&raw_full[rs], (it / R) & 1, p.status, kStatusTmaFullTimeout) &&
-             mbar_wait(&a_full[as], (it / A) & 1, p.status, kStatusTmaFullTimeout);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint64_t da = umma_desc_k_sw128(smem_u32(a_ring + as * Cfg::kATile));
-        const uint64_t db = umma_desc_k_sw128(smem_u32(raw_ring + rs * Cfg::kRawSlot));
+    constexpr uint32_t idesc = umma_idesc_bf16(128, TN);
+    const bool one = elect_one();
+    int rs = 0, as = 0;
+    uint32_t rph = 0, aph = 0;
+    bool ok = true;
+    for (int it = 0; it < niter; ++it) {
+      ok = mbar_wait_warp(&raw_full[rs], rph, p.status, kStatusTmaFullTimeout) && mbar_wait_warp(&a_full[as], aph, p.status, kStatusTmaFullTimeout);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint64_t da = umma_desc_k_sw128(smem_u32(a_ring + as * Cfg::kATile));
+      const uint64_t db = umma_desc_k_sw128(smem_u32(raw_ring + rs * Cfg::kRawSlot));
+      if (one) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_f16(tmem_base, da + 2 * k, db + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
         umma_commit(&a_empty[as]);
         umma_commit(&raw_empty[rs]);
       }
-      if (ok) umma_commit(accum_bar);
+      if (++rs == R) {
+        rs = 0;
+        rph ^= 1;
+      }
+      if (++as == A) {
+        as = 0;
+        aph ^= 1;
+      }
     }
+    if (ok && one) umma_commit(accum_bar);
   } else if (warp >= 6) {
     // ------------------------------------------------------------ dequant warps
     // 256 threads: thread t converts the 32-weight half t&1 of row t>>1 of every K block. (Giving each warp whole
