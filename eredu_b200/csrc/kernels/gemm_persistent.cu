@@ -11,7 +11,7 @@
 //   * the fp32 accumulator is double-buffered in TMEM (2 x 256 columns): while the epilogue warps drain tile i,
 //     the MMA warp already accumulates tile i+1;
 //   * a TMA ring runs ahead across tile boundaries: six stages of 32 KB, four of 48 KB, or ten of 18 KB for the expert items of decode steps;
-//   * the epilogue transposes through a 16 KB staging buffer so that Y leaves the SM as 16-byte row chunks;
+//   * two groups of four epilogue warps transpose through an 8 KB staging buffer each so that Y leaves the SM as 16-byte row chunks;
 //   * grouped (MoE) form: the tiles come from a work table {expert, first row, rows, -} built on the device, an item of at most 256 (16) rows
 //     each; a short item shortens the MMA and its copies (64 or 16 rows apiece) instead of fetching and multiplying rows nobody stores;
 //   * SwiGLU ("dual") tiles load 64 gate rows and 64 up rows into ONE 128-row operand tile, so gate and up use the
@@ -48,10 +48,16 @@ struct Ring {
   static constexpr int kStageBytes = kATile + (BOX == 16 ? kBoxBytes : BOX == kPair ? kBTile / 2 : kBTile);    // 18, 32 or 48 KB
   static constexpr int kStages = BOX == 16 ? 10 : BOX == kPair ? 6 : 4;
 };
-constexpr int kStagingBytes = 16 * 1024;
+constexpr int kChunkCols = 16;                    // tokens of a staging pass: 16 x 128 fp32 = 8 KB
+constexpr int kStagingBytes = kChunkCols * 128 * 4;
+// Epilogue groups of four warps, which take every second chunk of tokens. With one, a tile of 256 tokens took ten microseconds to store: about as
+// long as the products of short sums, and the end of every launch (2 x 8192 x 2048, 4096 tokens 258 -> 192 us, 300 tokens 31.0 -> 24.9; 4096 x 512,
+// 2048 tokens 21.4 -> 15.2; 4096 x 4096, 300 tokens 19.2 -> 18.2).
+constexpr int kGroups = 2;
+constexpr int kThreads = 64 + 128 * kGroups;
 constexpr int kCtrlBytes = 1024;
 template <int BOX>
-constexpr int kSmemBytes = 1024 + kCtrlBytes + Ring<BOX>::kStages * Ring<BOX>::kStageBytes + kStagingBytes;
+constexpr int kSmemBytes = 1024 + kCtrlBytes + Ring<BOX>::kStages * Ring<BOX>::kStageBytes + kGroups * kStagingBytes;
 
 struct PGemmParams {
   void* y;
@@ -110,11 +116,20 @@ __device__ __forceinline__ bool tile_at(const PGemmParams& p, int t, uint32_t cr
   return true;
 }
 
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void epi_bar(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+// Barrier of all groups; whether any of their threads says so.
+__device__ __forceinline__ bool epi_bar_any(bool said) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any)
+               : "r"(static_cast<uint32_t>(said)), "n"(1 + kGroups), "n"(128 * kGroups)
+               : "memory");
+  return any != 0;
+}
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
 template <bool DUAL, bool GROUPED, int BOX>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, PGemmParams p) {
   constexpr int kStages = Ring<BOX>::kStages, kStageBytes = Ring<BOX>::kStageBytes, kBoxBytes = Ring<BOX>::kBoxBytes;
   pdl_launch_early();
@@ -128,8 +143,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   uint8_t* stages = smem + kCtrlBytes;
   uint8_t* staging = stages + kStages * kStageBytes;
-  __shared__ float s_scale[kTN];
-  __shared__ int s_fail;
+  __shared__ float s_scales[2][kTN];     // of this tile and the next: a group may be a tile ahead
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -150,9 +164,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], PAIR ? 256 : 128);
+      mbar_init(&tempty_bar[b], (PAIR ? 2 : 1) * 128 * kGroups);
     }
-    s_fail = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -271,10 +284,12 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..5 and 6..9)
+    const int group = (warp - 2) >> 2;
     const int q = warp & 3;          // TMEM lane quarter this warp may read
     const int row = q * 32 + lane;   // accumulator lane = weight row inside the tile
-    const int et = threadIdx.x - 64;
+    const int et = (threadIdx.x - 64) & 127;
+    uint8_t* my_staging = staging + group * kStagingBytes;
     const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(p.residual);
     const __nv_bfloat16* bias = static_cast<const __nv_bfloat16*>(p.bias);
     __nv_bfloat16* yout = static_cast<__nv_bfloat16*>(p.y);
@@ -285,8 +300,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       const int tile_n = tl.tile_n, m_base = tl.m_base, m_cnt = tl.m_cnt;
       const int buf = lt & 1;
       const uint32_t bph = (lt >> 1) & 1;
+      float* s_scale = s_scales[buf];
       if (p.ssq_in != nullptr) {
-        for (int c = et; c < kTN; c += 128) {
+        for (int c = threadIdx.x - 64; c < kTN; c += 128 * kGroups) {
           float s = 0.f;
           if (c < m_cnt) {
             const float* src = p.ssq_in + static_cast<size_t>(m_base + c) * p.ssq_parts;
@@ -295,9 +311,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           s_scale[c] = rsqrtf(s * p.norm_inv_dim + p.norm_eps);
         }
       }
-      if (!mbar_wait(&tfull_bar[buf], bph, p.status, kStatusAccumTimeout)) s_fail = 1;
-      epi_bar();  // s_scale is complete; the failure flag is agreed on by all epilogue threads
-      if (s_fail) break;
+      // s_scale is complete behind this; all epilogue threads agree on a failure
+      if (epi_bar_any(!mbar_wait(&tfull_bar[buf], bph, p.status, kStatusAccumTimeout))) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + buf * kTN + (static_cast<uint32_t>(q * 32) << 16);
       // this thread's weight row: output column n (DUAL: gate rows are lanes 0..63, up rows lanes 64..127)
@@ -305,12 +320,16 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       const bool in_n = n < p.N;
       float b_row = 0.f;
       if (bias != nullptr && in_n) b_row = __bfloat162float(bias[DUAL && row >= 64 ? p.N + n : n]);
-      constexpr int kChunkCols = 32;  // tokens per staging pass: 32 x 128 fp32 = 16 KB
-      const int last_cc = ((m_cnt - 1) / kChunkCols) * kChunkCols;  // chunks past the last token are skipped
-      for (int cc = 0; cc <= last_cc; cc += kChunkCols) {
+      const int chunks = (m_cnt + kChunkCols - 1) / kChunkCols;       // chunks past the last token are skipped
+      const int last_cc = ((chunks - 1 - group) / kGroups * kGroups + group) * kChunkCols;     // this group's last one
+      if (group >= chunks) {        // none: the accumulator is not waited for
+        if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
+        else mbar_arrive(&tempty_bar[buf]);
+      }
+      for (int cc = group * kChunkCols; group < chunks && cc <= last_cc; cc += kGroups * kChunkCols) {
         // Second-pass work items of this thread (16-byte pieces of output rows); their residual is fetched now
         // so that the loads are in flight while the accumulator is read.
-        constexpr int kItems = DUAL ? 2 : 4;
+        constexpr int kItems = kChunkCols * kRowsPerTile / 8 / 128;
         uint4 rv[kItems];
         bool item_ok[kItems];
 #pragma unroll
@@ -322,7 +341,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           rv[i] = make_uint4(0u, 0u, 0u, 0u);
           if (item_ok[i] && res != nullptr) rv[i] = *reinterpret_cast<const uint4*>(res + static_cast<size_t>(m_base + cc + c) * p.ldr + gn);
         }
-        float* stf = reinterpret_cast<float*>(staging);
+        float* stf = reinterpret_cast<float*>(my_staging);
 #pragma unroll
         for (int c0 = 0; c0 < kChunkCols; c0 += 16) {
           uint32_t g[16];
@@ -340,8 +359,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
           else mbar_arrive(&tempty_bar[buf]);
         }
-        epi_bar();
-        const float* st = reinterpret_cast<const float*>(staging);
+        epi_bar(group);
+        const float* st = reinterpret_cast<const float*>(my_staging);
 #pragma unroll
         for (int i = 0; i < kItems; ++i) {
           const int id = et + 128 * i;
@@ -397,7 +416,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
             if ((lane & 15) == 0 && cc + c < m_cnt && tile_n < p.ssq_stride) p.ssq_out[static_cast<size_t>(m) * p.ssq_stride + tile_n] = sq;
           }
         }
-        epi_bar();  // staging may be overwritten
+        epi_bar(group);  // staging may be overwritten
       }
     }
   }
@@ -451,7 +470,7 @@ static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(192);
+  cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes<kPair>;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -526,7 +545,7 @@ int launch_gemm_persistent(const void* X, const void* W, void* Y, const void* re
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    return launch_pdl(kern, dim3(grid), dim3(192), kSmemBytes<64>, stream, tmW, tmX, p);
+    return launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes<64>, stream, tmW, tmX, p);
   };
   const cudaError_t e = dual ? launch(gemm_persistent_kernel<true, false, 64>) : launch(gemm_persistent_kernel<false, false, 64>);
   eredu_count_launches(1);
@@ -546,7 +565,7 @@ static cudaError_t launch_grouped(const CUtensorMap& tmW, const CUtensorMap& tmX
     configured[dev] = true;
   }
   const int total = p.n_tiles * p.m_tiles;
-  return launch_pdl(gemm_persistent_kernel<DUAL, true, BOX>, dim3(total < sms ? total : sms), dim3(192), kSmemBytes<BOX>, stream, tmW, tmX, p);
+  return launch_pdl(gemm_persistent_kernel<DUAL, true, BOX>, dim3(total < sms ? total : sms), dim3(kThreads), kSmemBytes<BOX>, stream, tmW, tmX, p);
 }
 
 int launch_gemm_persistent_grouped(const void* X, const void* W, void* Y, const int* work, int n_work, int item_rows, int rows_cap, int N, int K,
