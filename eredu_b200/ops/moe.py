@@ -162,13 +162,13 @@ def pick_tile(expected_rows_per_expert: float) -> int:
 def expert_tile(routes: int, e_local: int, inter: int, hidden: int, plain: bool) -> int:
     """Rows of a work item: as many as an expert is expected to get, up to 128, or the 256 of the persistent form where it applies
     (SwiGLU without bias or limit). That form fetches a short item's rows in boxes of 64 and starts the next item's copies while the last
-    one is stored; it takes over where an expert's rows no longer fit one small item. Both grouped GEMMs, 128 experts of 768 x 2048, us with
-    items of 16 / 32 / 64 / 256 rows: 16 rows an expert 243 / 234 / 282 / 236, 32 rows 347 / 283 / 298 / 251, 64 rows 565 / 420 / 373 / 274.
-    Few experts have fewer of its tiles to spread over the SMs: 8 of 14336 x 4096 with items of 32 / 256 rows, 25 rows an expert 447 / 513,
-    32 rows 559 / 517; where all of them have fewer such tiles than there are SMs, later still: 4 of 1024 x 1024, 32 rows 26.1 / 29.5, 50 rows
-    31.5 / 29.5."""
+    one is stored; it takes over where an expert's rows no longer fit one small item, or a little earlier. Both grouped GEMMs, us with
+    items of 16 / 32 / 64 / 256 rows: 128 experts of 768 x 2048, 12 rows an expert 182 / 205 / 255 / 190, 16 rows 207 / 211 / 256 / 191, 24 rows 258 / 222 /
+    258 / 193, 64 rows 463 / 345 / 279 / 213; 64 of 1408 x 2048, 12 rows 169 / 187 / 224 / 175, 16 rows 183 / 190 / 224 / 175. Few experts have fewer of its
+    tiles to spread over the SMs: 8 of 14336 x 4096 with items of 32 / 256 rows, 32 rows an expert 434 / 467, 40 rows 713 / 470; where all of
+    them have fewer such tiles than there are SMs, later still: 4 of 1024 x 1024, 40 rows 16.5 / 17.3, 50 rows 19.3 / 17.8."""
     per = routes / max(1, e_local)
-    return 256 if plain and per > (24 if e_local >= 64 else 26 if e_local * inter > 148 * 64 else 40) and inter % 64 == 0 and hidden % 8 == 0 else pick_tile(per)
+    return 256 if plain and per > (14 if e_local >= 64 else 32 if e_local * inter > 148 * 64 else 40) and inter % 64 == 0 and hidden % 8 == 0 else pick_tile(per)
 
 
 def route_plan_gather(logits, x, k, scoring, renorm, scale, sel_bias, e0, n_local, n_group=1, topk_group=1):

@@ -451,7 +451,8 @@ def test_decode_attention_ahead_of_its_projection(D, n_q, n_kv, new, lens):
 
 @pytest.mark.parametrize("E,k,T,H,inter", [(8, 2, 100, 512, 1472), (8, 2, 108, 512, 1472), (8, 2, 512, 256, 192), (16, 4, 260, 256, 320),
                                            (48, 4, 48, 512, 1088), (48, 4, 148, 512, 1088), (48, 4, 180, 512, 1088), (64, 4, 420, 256, 128), (4, 2, 80, 512, 320),
-                                           (4, 2, 82, 512, 320)])
+                                           (4, 2, 82, 512, 320), (64, 4, 224, 256, 128), (64, 4, 225, 256, 128), (8, 2, 128, 512, 1472),
+                                           (8, 2, 132, 512, 1472)])
 def test_experts_at_the_borders_of_the_rule(E, k, T, H, inter):
     """Few experts with 25 to 128 rows each; experts whose rows fill one item of sixteen and such that need a second."""
     x = torch.randn(T, H, device=DEV).bfloat16()
