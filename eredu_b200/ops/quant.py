@@ -255,9 +255,11 @@ class QuantLinear:
         """silu(x Wgate^T) * (x Wup^T) for a weight that stacks gate rows over up rows: one kernel for decode-sized
         batches, the weight decoded once and the dense kernel with its SwiGLU epilogue for prompt-sized ones (70 B shape, 4096 tokens:
         137 us and a round trip of 470 MB less per layer than with the activation kernel), the projection followed by the activation
-        kernel otherwise. That includes prompts of many tokens where the sums are short: the epilogue of a gated tile takes longer than the
-        next tile's products (1000 tokens, us of the activation kernel and of the epilogue: 8192 x 1024 60 / 68, 2048 x 2048 29 / 32, 4096 x 2048
-        47 / 48, 8192 x 2048 86 / 83, 2048 x 4096 45 / 43; 400 tokens, 8192 x 1024 37 / 36)."""
+        kernel otherwise. That includes prompts of up to 2048 tokens where the sums are short: the epilogue of a gated tile takes longer
+        than the next tile's products, and only in longer prompts does the round trip of the sums take longer still (us of the activation
+        kernel and of the epilogue, inter x K: 8192 x 1024 with 520 / 1000 / 2000 / 4000 tokens 31 / 32, 45 / 48, 73 / 70, 142 / 124;
+        2048 x 1024 with 2000 and 4000 25.5 / 26.0, 39.9 / 39.8; 2048 x 2048 with 1000 and 4000 27.0 / 27.4, 56 / 51; 8192 x 2048 with 1000
+        69 / 64)."""
         inter = self.out_features // 2
         if x.is_cuda:
             assert x.shape[1] == self.in_features and x.dtype == torch.bfloat16 and x.stride(1) == 1
@@ -265,8 +267,8 @@ class QuantLinear:
             return self._gemv(x, bias, None, None, torch.bfloat16, True, limit or 0.0)
         from .core import gated_linear, silu_mul
 
-        short = self.in_features <= 1024 or (self.in_features <= 2048 and inter <= 2048)
-        if (x.is_cuda and x.shape[0] > self.DENSE_FALLBACK_TOKENS and not (short and x.shape[0] > 512) and not limit and inter % 8 == 0
+        short = 512 < x.shape[0] <= 2048 and (self.in_features <= 1024 or (self.in_features <= 2048 and inter <= 2048))
+        if (x.is_cuda and x.shape[0] > self.DENSE_FALLBACK_TOKENS and not short and not limit and inter % 8 == 0
                 and x.stride(0) % 8 == 0):
             return gated_linear(x, self._dense(), inter, bias=bias, dynamic_weight=True)
 

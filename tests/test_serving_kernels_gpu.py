@@ -210,6 +210,16 @@ def test_four_bit_rows_on_integer_products(M, N, K, group, gated, decades):
     assert bool(torch.isnan(ql.gated(x) if gated else ql(x)).all(-1)[0]) and (M == 1 or bool(torch.isfinite(ql(x)[1]).all()))
 
 
+@pytest.mark.parametrize("M,K", [(512, 1024), (513, 1024), (2048, 1024), (2049, 1024), (2049, 2048), (513, 2112), (4001, 64)])
+def test_gated_four_bit_prompts_of_short_sums(M, K):
+    """On either side of where the activation has a kernel of its own."""
+    ql = QuantLinear.from_dense((torch.randn(2 * 520, K, device=DEV) * 0.05).bfloat16(), 4, 64)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    y = x.double() @ ql.dequantize(torch.float32).double().t()
+    # the kernel of its own reads gate and up rounded to bf16, and both forms multiply bf16 weights
+    assert rel_l2(ql.gated(x), moe_ops.gated_act_ref(y[:, :520].float(), y[:, 520:].float())) < 3 * BF16
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 5, 64])
 @pytest.mark.parametrize("H,inter", [(256, 96), (2048, 768)])
 def test_experts_of_few_tokens(T, H, inter):
