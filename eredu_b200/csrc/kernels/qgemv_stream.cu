@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
     if (warp == 0 && p.ns > 1)
       for (int i = 0; i < 2; ++i) {
         mbar_init(&xbars[i], 1);
-        mbar_arrive_expect_tx(&xbars[i], static_cast<uint32_t>((p.ns - 1) * S * TOK * cols * 4));
+        mbar_arrive_expect_tx(&xbars[i], static_cast<uint32_t>(p.ns * S * TOK * cols * 4));
       }
     fence_mbar_init();
   }
@@ -291,13 +291,14 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
     if (p.out_fp32) static_cast<float*>(p.y)[static_cast<size_t>(m) * p.ldy + n] = out;
     else static_cast<__nv_bfloat16*>(p.y)[static_cast<size_t>(m) * p.ldy + n] = __float2bfloat16(out);
   };
-  // clusters: what the other CTAs have sent of round r, summed in rank order. A round later than it was sent, so that nobody waits for it. A
-  // buffer is written again two rounds later: by a CTA that has received this one's sums of the round between, which were sent after this
-  // read. Threads that read nothing do not wait either: they send nothing that would keep the barrier from running on.
+  // clusters: what all CTAs of the cluster, this one too, have sent of round r, summed in rank order. A round later than it was sent, so that nobody
+  // waits for it, and in front of the barrier behind which this CTA sends the next sums. A buffer is written again two rounds later, by a CTA that has
+  // received all that this one sent in the round between: behind that barrier, so after these reads. For the same reason no barrier
+  // completes a second phase before the first has been seen.
   const int part_floats = S * TOK * cols;
   auto finish_exchange = [&](int r) {
     if (threadIdx.x >= TOK * cols || !mbar_wait(&xbars[r & 1], (r >> 1) & 1, p.status, kStatusSmemEmptyTimeout)) return;
-    if (threadIdx.x == 0 && r + 2 < rounds) mbar_arrive_expect_tx(&xbars[r & 1], static_cast<uint32_t>((p.ns - 1) * part_floats * 4));
+    if (threadIdx.x == 0 && r + 2 < rounds) mbar_arrive_expect_tx(&xbars[r & 1], static_cast<uint32_t>(p.ns * part_floats * 4));
     const float* from = recv + (r & 1) * recv_floats(GATED, TOK);
     const int m = threadIdx.x / cols, c = threadIdx.x % cols;
     float v[S];
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
         if (t == 0) mine[((s / RT) * TOK + (j & 1)) * LDN + (s % RT) * 16 + g + (j >> 1) * 8] = v;
       }
     }
+    if (p.ns > 1 && r > 0) finish_exchange(r - 1);
     __syncthreads();
     if (p.ns == 1) {
       if (threadIdx.x < TOK * ROWS) {
@@ -355,22 +357,15 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv4_stream_kernel(const QGemvS
         for (int s = 0; s < S; ++s) v[s] = warps_sum(r, s, m, cl);
         finish(r, m, cl, v);
       }
-    } else {
-      if (r > 0) finish_exchange(r - 1);
-      if (threadIdx.x < S * TOK * ROWS) {
-        const int cl = threadIdx.x % ROWS, sm = threadIdx.x / ROWS, m = sm % TOK, s = sm / TOK;
-        const float v = warps_sum(r, s, m, cl);
-        const uint32_t owner = static_cast<uint32_t>(cl / cols);
-        const uint32_t off = ((r & 1) * recv_floats(GATED, TOK) + static_cast<int>(crank) * part_floats + sm * cols + cl % cols) * 4;
-        if (owner == crank) recv[off / 4] = v;
-        else store_async(mapa_shared(recv_addr + off, owner), v, mapa_shared(xbar_addr + (r & 1) * 8, owner));
-      }
+    } else if (threadIdx.x < S * TOK * ROWS) {
+      const int cl = threadIdx.x % ROWS, sm = threadIdx.x / ROWS, m = sm % TOK, s = sm / TOK;
+      const float v = warps_sum(r, s, m, cl);
+      const uint32_t owner = static_cast<uint32_t>(cl / cols);
+      const uint32_t off = ((r & 1) * recv_floats(GATED, TOK) + static_cast<int>(crank) * part_floats + sm * cols + cl % cols) * 4;
+      store_async(mapa_shared(recv_addr + off, owner), v, mapa_shared(xbar_addr + (r & 1) * 8, owner));
     }
   }
-  if (p.ns > 1) {
-    __syncthreads();
-    if (rounds > 0) finish_exchange(rounds - 1);
-  }
+  if (p.ns > 1 && rounds > 0) finish_exchange(rounds - 1);
   if (!ok) {
     // a copy never landed (status recorded): give the other copies of this warp their bounded wait before the memory goes away
     for (int i = 0; i < p.slots; ++i) {

@@ -38,3 +38,15 @@ def test_reading_of_blocks(text, lines):
 @pytest.mark.parametrize("name", sorted(p.name for p in KERNELS.glob("*.cu*")))
 def test_remote_stores_wait_for_their_target(name):
     assert unguarded_stores((KERNELS / name).read_text()) == []
+
+
+def round_of(source):
+    """Reads, barriers and sends of a round of the persistent 4-bit kernel, in the order of the source."""
+    loop = source[source.index("for (int r = 0; r < rounds; ++r)"):source.index("finish_exchange(rounds - 1)")]
+    return re.findall(r"finish_exchange|__syncthreads|store_async|recv\[", re.sub(r"//.*", "", loop))
+
+
+def test_sums_are_sent_behind_the_reads_of_the_round_before():
+    """A CTA sends behind a barrier that follows its reads of the round before, so that who has its sums may write over what it has read. Its own
+    sums take the same way: a plain store would need a barrier between itself and the reads as well."""
+    assert round_of((KERNELS / "qgemv_stream.cu").read_text()) == ["finish_exchange", "__syncthreads", "store_async"]

@@ -210,6 +210,19 @@ def test_four_bit_rows_on_integer_products(M, N, K, group, gated, decades):
     assert bool(torch.isnan(ql.gated(x) if gated else ql(x)).all(-1)[0]) and (M == 1 or bool(torch.isfinite(ql(x)[1]).all()))
 
 
+@pytest.mark.parametrize("M,N,K,group,gated", [(1, 9488, 18624, 64, False), (1, 2 * 4752, 20608, 128, True), (2, 9488, 9408, 64, False),
+                                               (2, 26000, 10624, 128, False), (2, 2 * 4752, 9280, 64, True), (2, 2 * 16400, 9344, 64, True)])
+def test_four_bit_rows_over_many_rounds_of_two_ctas(M, N, K, group, gated):
+    """Matrices of three and more rounds whose activations do not fit one CTA: the buffers and barriers of the exchange are used again."""
+    ql = QuantLinear.from_dense((torch.randn(N, K, device=DEV) * 0.05).bfloat16(), 4, group)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    y = x.double() @ ql.dequantize(torch.float32).double().t()
+    ref = moe_ops.gated_act_ref(y[:, :N // 2].float(), y[:, N // 2:].float()) if gated else y
+    got = [ql.gated(x) if gated else ql(x, out_dtype=torch.float32) for _ in range(20)]
+    assert rel_l2(got[0], ref) < (BF16 if gated else 2.0 ** -18)      # fp32 results as in test_four_bit_rows_on_integer_products
+    assert all(torch.equal(g, got[0]) for g in got)
+
+
 @pytest.mark.parametrize("M,K", [(512, 1024), (513, 1024), (2048, 1024), (2049, 1024), (2049, 2048), (513, 2112), (4001, 64)])
 def test_gated_four_bit_prompts_of_short_sums(M, K):
     """On either side of where the activation has a kernel of its own."""
