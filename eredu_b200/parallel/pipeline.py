@@ -35,6 +35,7 @@ class _StageModel:
         self.dtype = model.dtype
         self.n_kv_local = model.n_kv_local
         self.n_q_local = model.n_q_local
+        self.decode_rows = model.decode_rows
         self.first_layer = model.first_layer
         self.last_layer = model.last_layer
         topo = par.topology

@@ -258,6 +258,11 @@ class Engine:
             t = t.pin_memory().to(self.device, non_blocking=True)
         return t
 
+    def decode_splits(self, batch: int, longest: int) -> int:
+        """Split-KV factor of a step of ``batch`` sequences that bring one token each, the longest context of them ``longest`` tokens."""
+        rows = self.model.decode_rows
+        return ops.decode_splits(batch, self.model.n_kv_local, longest, self.sm_count, rows) if self.cuda else 1
+
     def _upload(self, **arrays) -> dict:
         """numpy arrays on the engine's device, as views of one buffer that travels in one copy: what describes a batch is six or seven short
         arrays, and a pinned buffer and a copy of its own cost each of them 20 us on the host (a turn of 45 tokens through eight layers 1175 -> 1081 us)."""
@@ -382,7 +387,7 @@ class Engine:
                 h[i, :len(tail)] = tail
             hist = self._t(h, torch.int32)
         max_len = int(pos.max()) + 1 + max(s.max_new_tokens for s in seqs)
-        splits = ops.decode_splits(B, self.model.n_kv_local, max_len, self.sm_count, self.model.decode_rows) if self.cuda else 1
+        splits = self.decode_splits(B, max_len)
         st = {
             "B": B,
             "seqs": list(seqs),
@@ -426,7 +431,7 @@ class Engine:
         if decode_form and max(counts) == 1:
             common = dict(self._upload(**arrays), sm_count=self.sm_count)
             longest = int(lens.max())
-            splits = ops.decode_splits(len(seqs), self.model.n_kv_local, longest, self.sm_count, self.model.decode_rows) if self.cuda else 1
+            splits = self.decode_splits(len(seqs), longest)
             return ForwardBatch(**common, is_prefill=False, q_per_seq=1, max_kv_len=longest, splits=splits)
         arrays["cu_q"] = np.concatenate(([0], np.cumsum(counts))).astype(np.int32)
         return ForwardBatch(**self._upload(**arrays), sm_count=self.sm_count, is_prefill=True, max_q_len=max(counts),
@@ -503,7 +508,7 @@ class Engine:
         dev = self.device
         rows = pack_rows([SamplingParams(temperature=0.0)] * B, [1] * B, hist_lens=[0] * B, stream_ids=[0] * B)
         max_len = max_context or self.max_seq_len
-        splits = ops.decode_splits(B, self.model.n_kv_local, max_len, self.sm_count, self.model.decode_rows) if self.cuda else 1
+        splits = self.decode_splits(B, max_len)
         st = {
             "B": B, "seqs": [None] * B, "slotted": True,
             "token_ids": torch.zeros(B, dtype=torch.int32, device=dev),

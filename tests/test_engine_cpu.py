@@ -146,3 +146,18 @@ def test_vision_language_checkpoint_as_text_model(tmp_path):
     req = MM.MultimodalRequest().text("what is this").image(MM.RgbImage(np.zeros((4, 4, 3), np.uint8)))
     with pytest.raises(MM.MultimodalPreparationError):
         MM.prepare_for_text_model(req, lm.encode)
+
+
+@pytest.mark.parametrize("kv_heads", [2, 4])
+def test_steps_of_a_pipeline_stage_are_split_like_those_of_its_model(kv_heads):
+    """The wrapper of a stage answers what the engine asks of a model for a decode step, on the CPU as on a GPU."""
+    from types import SimpleNamespace
+
+    from eredu_b200.parallel.pipeline import _StageModel
+
+    cfg = dataclasses.replace(C.tiny_llama(), num_attention_heads=4, num_key_value_heads=kv_heads, head_dim=64)
+    model = build(cfg, random_state(cfg, seed=0))
+    ends = SimpleNamespace(pipeline_predecessor=lambda r: None, pipeline_successor=lambda r: None)
+    stage = _StageModel(model, SimpleNamespace(topology=ends, rank=0))
+    assert stage.decode_rows == model.decode_rows == 4 // kv_heads
+    assert Engine(stage, max_batch=1, max_seq_len=64).decode_splits(1, 64) == 1
