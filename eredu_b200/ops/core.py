@@ -637,26 +637,43 @@ CLUSTER_SPLITS = 8      # splits the decode kernel combines through distributed 
 FUSED_ROPE_MAX_NEW = 8  # new tokens per sequence the fused RoPE + append decode path takes
 
 
-def decode_splits(batch, n_kv, max_kv_len, sm_count=148, rows=0):
+def decode_splits(batch, n_kv, max_kv_len, sm_count=148, rows=0, head_dim=128):
     """Split-KV factor: enough CTAs to fill the GPU once (a second wave costs more than it returns: the CTAs of the
     following kernel are already resident under programmatic dependent launch), at least 8 pages per split.
     ``rows``: query rows that share a key / value head where the caller knows that the plain kernel takes them (head sizes 64 and 128, at
-    most 16 rows), else 0. Its CTAs of eight warps run one to an SM, and as many splits as that allows are the best there are (us with the
-    splits of either rule: one sequence of 4096, 32 heads over 8, 13.8 with 32 and 10.2 with 8; eight of 1024, 64 heads over 8, 15.2 with 4 and
-    13.3 with 2; 32 of 1024, 32 heads over 4, 21.6 with 2 and 16.9 with 1)."""
+    most 16 rows), else 0. Its CTAs of eight warps run one to an SM, and as many splits as that allows are the best there are in contexts of
+    some length (us with the splits of either rule: one sequence of 4096, 32 heads over 8, 13.8 with 32 and 10.2 with 8; eight of 1024, 64 heads
+    over 8, 15.2 with 4 and 13.3 with 2; 32 of 1024, 32 heads over 4, 21.6 with 2 and 16.9 with 1). How long: see _one_round_pays."""
     ctas = max(1, batch * n_kv)
     pages = max(1, (max_kv_len + PAGE - 1) // PAGE)
-    if 0 < rows <= 16 and ctas <= sm_count:
-        # clusters of more than two CTAs, and of more than four, leave parts of a GPC empty
-        want = max(s for s in range(1, CLUSTER_SPLITS + 1) if ctas * s <= (sm_count if s <= 2 else sm_count * 7 // 8 if s <= 4 else sm_count * 2 // 3) or s == 1)
-        return max(1, min(want, pages // 8))
     want = max(1, (_SPLIT_WAVES * sm_count) // ctas)
     splits = int(max(1, min(want, pages // 8 if pages >= 8 else 1, 32)))
     # up to CLUSTER_SPLITS splits combine inside a thread-block cluster (no scratch, no second pass over global memory):
     # prefer that form while a split then still has at most 32 pages (8 per warp)
     if splits > CLUSTER_SPLITS and pages <= 32 * CLUSTER_SPLITS:
         splits = CLUSTER_SPLITS
+    if 0 < rows <= 16 and ctas <= sm_count:
+        # clusters of more than two CTAs, and of more than four, leave parts of a GPC empty
+        want = max(s for s in range(1, CLUSTER_SPLITS + 1) if ctas * s <= (sm_count if s <= 2 else sm_count * 7 // 8 if s <= 4 else sm_count * 2 // 3) or s == 1)
+        one_round = max(1, min(want, pages // 8))
+        if _one_round_pays(ctas, pages, one_round, splits, sm_count, head_dim):
+            return one_round
     return splits
+
+
+def _one_round_pays(ctas, pages, one_round, splits, sm_count, head_dim):
+    """Whether ``one_round`` splits, a CTA of eight warps to an SM, take no longer than the ``splits`` that are meant to fill the GPU.
+    Such a CTA walks a page in 0.17 us (head size 128) or 0.14 (64) whatever the others do, so that SMs without one are lost; the other form
+    ends when memory has delivered all pages - at what 7/8 of the SMs take that way (128), 8/7 of them (64) - or its own CTAs have walked theirs,
+    and costs 30 (20) pages' time more to combine clusters, 50 (40) to combine through scratch. us of one round / the other form, 128: one head,
+    8192 tokens 14.4 / 15.2, 16384 24.7 / 17.8, 131072 180 / 57; 8 heads, 8192 14.7 / 18.4, 16384 24.7 / 24.3, 32768 48 / 36, 131072 176 / 101;
+    10 x 8 heads, 1024 13.8 / 15.3, 2048 24.5 / 22.3, 8192 91 / 66; 16 x 8 heads, 32768 322 / 341. 64: 8 heads, 8192 12.5 / 14.3, 16384 20.7 /
+    18.2; 10 x 8 heads, 1024 11.6 / 10.3; 16 x 8 heads, 2048 21.1 / 21.2, 4096 40.1 / 38.2."""
+    if head_dim > 64 and 2 < splits <= CLUSTER_SPLITS and ctas * splits > (sm_count * 36 // 19 if splits <= 5 else sm_count * 25 // 14):
+        return True   # more clusters than run at once, two CTAs to an SM: 16384 tokens, 56 x 5 97 / 81, 58 x 5 97 / 137; 44 x 6 96 / 67, 46 x 6 96 / 113
+    combine = (50 if splits > CLUSTER_SPLITS else 30) if head_dim > 64 else (40 if splits > CLUSTER_SPLITS else 20)
+    at_full_rate = pages * ctas / (sm_count * 7 / 8 if head_dim > 64 else sm_count * 8 / 7)
+    return pages / one_round <= combine + max(at_full_rate, pages / splits)
 
 
 def attention_decode(q, k_cache, v_cache, block_table, seq_lens, q_per_seq, scale, splits=1, window=0, sinks=None,

@@ -261,7 +261,7 @@ class Engine:
     def decode_splits(self, batch: int, longest: int) -> int:
         """Split-KV factor of a step of ``batch`` sequences that bring one token each, the longest context of them ``longest`` tokens."""
         rows = self.model.decode_rows
-        return ops.decode_splits(batch, self.model.n_kv_local, longest, self.sm_count, rows) if self.cuda else 1
+        return ops.decode_splits(batch, self.model.n_kv_local, longest, self.sm_count, rows, self.cfg.head_dim) if self.cuda else 1
 
     def _upload(self, **arrays) -> dict:
         """numpy arrays on the engine's device, as views of one buffer that travels in one copy: what describes a batch is six or seven short

@@ -122,7 +122,7 @@ def test_four_bit_rows_at_the_borders_of_the_plan(M, N, K, group, gated):
 
 
 @pytest.mark.parametrize("B,n_q,n_kv,D,splits", [(1, 32, 8, 128, 8), (1, 4, 4, 64, 5), (2, 32, 8, 128, 6), (2, 32, 8, 128, 8), (32, 32, 4, 128, 1),
-                                                 (37, 64, 4, 128, 1), (38, 64, 4, 128, 1), (3, 16, 1, 64, 3)])
+                                                 (37, 64, 4, 128, 1), (38, 64, 4, 128, 1), (3, 16, 1, 64, 3), (1, 8, 1, 128, 32), (1, 32, 8, 64, 18), (3, 8, 1, 64, 49)])
 @pytest.mark.parametrize("length", [1, 16, 17, 128, 129, 1025])
 def test_decode_attention_of_one_new_token(B, n_q, n_kv, D, splits, length):
     """Grids on either side of where CTAs have eight warps; contexts that leave splits or warps without a page, new tokens that open a page; one
