@@ -428,7 +428,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         if (m_base + c < m_limit) {
           const float* src = p.ssq_in + static_cast<size_t>(m_base + c) * p.ssq_parts;
           int j = 0;
-          if ((p.ssq_parts & 3) == 0) {     // the same sum with eight 16-byte loads on their way
+          // the same sum with eight 16-byte loads on their way, where rows start on such a boundary
+          if ((p.ssq_parts & 3) == 0 && (reinterpret_cast<uintptr_t>(p.ssq_in) & 15) == 0) {
 #pragma unroll 8
             for (; j < p.ssq_parts; j += 4) {
               const float4 v = *reinterpret_cast<const float4*>(src + j);

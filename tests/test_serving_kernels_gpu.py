@@ -170,6 +170,20 @@ def test_split_sums_of_several_tokens(M, N, K, odd):
         assert rel_l2(ops.gated_linear(got, w2, 264, row_ssq=ssq, norm_eps=1e-6), moe_ops.gated_act_ref(z[:, :264].float(), z[:, 264:].float())) < BF16
 
 
+@pytest.mark.parametrize("M", [1, 5, 33, 100])
+@pytest.mark.parametrize("parts", [4, 7, 8])
+def test_sums_of_squares_that_start_anywhere(M, parts):
+    """Partial sums that are part of a larger buffer start on any float."""
+    N, K = 264, 1024
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(2 * N, K, device=DEV) * K ** -0.5).bfloat16()
+    ssq = torch.rand(M, parts, device=DEV) * 2 * K / parts
+    y = x.double() @ w.double().t() * (ssq.double().sum(-1, keepdim=True) / K + 1e-6).rsqrt()
+    for at in range(4):
+        part = torch.empty(M * parts + 4, device=DEV)[at:at + M * parts].view(M, parts).copy_(ssq)
+        assert rel_l2(ops.linear(x, w[:N], row_ssq=part, norm_eps=1e-6), y[:, :N]) < BF16
+        assert rel_l2(ops.gated_linear(x, w, N, row_ssq=part, norm_eps=1e-6), moe_ops.gated_act_ref(y[:, :N].float(), y[:, N:].float())) < BF16
+
+
 @pytest.mark.parametrize("M", [129, 161, 300, 777])
 @pytest.mark.parametrize("N,K", [(128, 1024), (136, 1024), (264, 1016), (392, 1088), (3848, 4096)])
 def test_projections_of_prompts_on_pairs_of_ctas(M, N, K):
