@@ -313,10 +313,9 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   plan_block(ids, routes, k, e0, e1, tile, seg, route_pos, row_token, work, n_work_cap, counts);
 }
 
-// The plan of at most 32 routes, at most `tile` of them to an expert: a lane of the first warp has a route and compares it with the others. The
-// segments, counters and scans above are five barriers and two passes over the routes (one token, 8 of 128 experts, with routing and gather
-// 7.8 us in a decode step, 5.1 now).
-__device__ __forceinline__ void plan_few(const int* s_ids, int routes, int k, int e0, int e1, int* s_token, int* s_done, int* __restrict__ seg,
+// The plan of at most 32 routes: a lane of the first warp has a route and compares it with the others. The segments, counters and scans above are
+// five barriers and two passes over the routes (one token, 8 of 128 experts, with routing and gather 7.8 us in a decode step, 5.1 now).
+__device__ __forceinline__ void plan_few(const int* s_ids, int routes, int k, int e0, int e1, int tile, int* s_token, int* s_done, int* __restrict__ seg,
                                          int* __restrict__ route_pos, int* __restrict__ row_token, int4* __restrict__ work, int n_work_cap,
                                          int* __restrict__ counts) {
   const int n_local = e1 - e0, lane = threadIdx.x & 31;
@@ -330,18 +329,20 @@ __device__ __forceinline__ void plan_few(const int* s_ids, int routes, int k, in
       before += other == e && r < lane;
       same += other == e;
     }
-    const unsigned firsts = __ballot_sync(0xffffffffu, e >= 0 && before == 0);
-    int item = 0;                               // experts in front
+    // (a token may choose an expert twice: where the kept groups hold fewer experts than it chooses)
+    const bool opens = e >= 0 && before % tile == 0;       // the first row of an item
+    const unsigned firsts = __ballot_sync(0xffffffffu, opens);
+    int item = 0;                               // items in front
     for (int r = 0; r < routes; ++r) {
       const int other = __shfl_sync(0xffffffffu, e, r);
-      item += ((firsts >> r) & 1u) && other < e;
+      item += ((firsts >> r) & 1u) && (other < e || (other == e && r < lane));
     }
     const int rows = __popc(__ballot_sync(0xffffffffu, e >= 0));
     if (lane < routes) route_pos[lane] = e >= 0 ? smaller + before : -1;
     if (e >= 0) {
       row_token[smaller + before] = lane / k;
       s_token[smaller + before] = lane / k;
-      if (before == 0 && item < n_work_cap) work[item] = make_int4(e, smaller, same, 0);
+      if (opens && item < n_work_cap) work[item] = make_int4(e, smaller + before, min(tile, same - before), 0);
     }
     if (lane == 0) {
       s_done[0] = counts[0] = rows;
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(1024) moe_route_plan_gather_kernel(
   __syncthreads();
   const bool few = T * p.k <= 32 && T <= tile;
   if (few) {
-    plan_few(s_ids, T * p.k, p.k, e0, e1, s_token, s_done, seg, route_pos, row_token, work, n_work_cap, counts);
+    plan_few(s_ids, T * p.k, p.k, e0, e1, tile, s_token, s_done, seg, route_pos, row_token, work, n_work_cap, counts);
   } else {
     plan_block(s_ids, T * p.k, p.k, e0, e1, tile, seg, route_pos, row_token, work, n_work_cap, counts);
     __syncthreads();

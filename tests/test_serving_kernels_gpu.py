@@ -404,6 +404,18 @@ def test_routes_of_few_tokens_are_planned_alike(T, E, e0, n_local, k):
     assert torch.equal(xp[:rows], x[want.row_token[:rows].long()])
 
 
+@pytest.mark.parametrize("T,k", [(16, 2), (10, 3), (9, 2), (1, 3)])
+def test_routes_of_few_tokens_that_choose_an_expert_twice(T, k):
+    """The one kept group holds one expert, so that the other routes of a token go to the first of what is left: more rows than an item has."""
+    logits, x = torch.randn(T, 8, device=DEV), torch.randn(T, 256, device=DEV).bfloat16()
+    logits[:, 0] = 9.0
+    ids, _, plan, xp = moe_ops.route_plan_gather(logits, x, k, "softmax", True, 1.0, None, 0, 8, n_group=8, topk_group=1)
+    want = moe_ops.ExpertPlan(ids, k, 0, 8, plan.tile, T * k)
+    assert torch.equal(plan.counts, want.counts) and torch.equal(plan.work, want.work) and torch.equal(plan.seg, want.seg)
+    assert torch.equal(plan.route_pos, want.route_pos) and torch.equal(plan.row_token, want.row_token)
+    assert torch.equal(xp, x[want.row_token.long()])
+
+
 @pytest.mark.parametrize("E,e0,e1,routes,k", [(8, 0, 8, 3000, 2), (9, 0, 9, 3000, 3), (20, 4, 20, 130, 2)])
 def test_expert_plan_of_few_experts(E, e0, e1, routes, k):
     """On either side of where lanes find their like by values instead of bits; batches of routes that end early."""
