@@ -1037,11 +1037,11 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   // A narrow output over many tokens (a router) fills the machine with small token tiles instead. K is not split: experts that score alike
-  // change places with the order of a sum, and this one is the same for every number of tokens. What smaller tiles save is the serial epilogue of
+  // change places with the order of a sum, and this one is the same for every number of tokens above 64. What smaller tiles save is the serial epilogue of
   // their columns, as long as one round of CTAs holds them: 1024 x 128 x 2048 10.6 us with 16 tokens, 4096 tokens 13.2 with 32. Few rows of
   // weights that all CTAs fetch at once stand a quarter of the CTAs (1024 x 8 x 2048: 15.5 to 24.8 us with 16 tokens, by where the rows lie,
   // 18.0 with 32).
-  const bool narrow = tn == 256 && out_fp32 && ((N + 127) / 128) * ((M + 255) / 256) * 2 <= sm_count;
+  const bool narrow = tn >= 128 && out_fp32 && ((N + 127) / 128) * ((M + 255) / 256) * 2 <= sm_count;
   if (narrow) {
     const int ctas = N > 16 ? sm_count : sm_count / 4;
     tn = 64;

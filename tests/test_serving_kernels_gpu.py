@@ -451,6 +451,13 @@ def test_router_sums_have_one_order(M, N, K):
     assert torch.equal(y, alone)
 
 
+@pytest.mark.parametrize("M", [65, 96, 100, 128, 129])
+@pytest.mark.parametrize("N,K", [(8, 4096), (128, 2048), (96, 320), (256, 4096), (9600, 1088)])
+def test_router_sums_of_short_prompts_have_the_same_order(M, N, K):
+    x, w = torch.randn(300, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    assert torch.equal(ops.linear(x[:M], w, out_dtype=torch.float32), ops.linear(x, w, out_dtype=torch.float32)[:M])
+
+
 @pytest.mark.parametrize("M,N,K", [(130, 1096, 256), (400, 4736, 128), (1250, 4096, 192), (1900, 2048, 128)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_prompt_gemm_tiles_of_fewer_tokens(M, N, K, gated):
