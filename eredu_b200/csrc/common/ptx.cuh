@@ -20,6 +20,7 @@ enum KernelStatus : int {
   kStatusAccumTimeout = 3,      // epilogue never saw the accumulator commit
   kStatusPeerFlagTimeout = 4,   // a flag another GPU should have written never arrived
   kStatusBadArgument = 5,
+  kStatusSharesTimeout = 6,     // what the other CTAs of a cluster send never arrived
 };
 
 // ~2 s at 1.9 GHz; long enough for any legitimate wait, short enough to keep the context usable.

@@ -63,6 +63,7 @@ struct AttnParams {
   const __nv_bfloat16* pk;
   const __nv_bfloat16* pv;
   int pool, pool_rows;
+  int* status;
 };
 constexpr int kMaxFusedNew = 8;       // new tokens per sequence the fused (RoPE + append) decode path handles
 constexpr int kMaxClusterSplits = 8;  // portable cluster size
@@ -858,7 +859,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 4 && MT == 1 ? (DK + DV <= 128 
     __syncthreads();               // this CTA's own share is in place
     // (a CTA that finishes nothing waits too: maxima and sums are on their way to it)
     if (threadIdx.x == 0 || static_cast<int>(threadIdx.x) < own) {
-      const bool all = mbar_wait(&s_sent, 0, nullptr, 0);
+      const bool all = mbar_wait(&s_sent, 0, p.status, kStatusSharesTimeout);
       for (int e = threadIdx.x; e < own && all; e += NT) {
         const int i = split * per + e, row = i / DV, d = i % DV;
         float M = -INFINITY;
@@ -1167,7 +1168,7 @@ static int launch_decode_all(AttnParams p, int batch, int q_per_seq, int n_q_hea
 static int attn_decode_impl(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
                             const int* seq_lens, const float* sinks, float* part_o, float* part_ml, int* counters,
                             int batch, int q_per_seq, int max_pages, int n_q_heads, int n_kv_heads, int key_dim, int value_dim,
-                            int splits, int window, int chunk, float scale, cudaStream_t stream, bool force_scratch) {
+                            int splits, int window, int chunk, float scale, int* status, cudaStream_t stream, bool force_scratch) {
   AttnParams p = {};
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k_cache = static_cast<const __nv_bfloat16*>(k_cache);
@@ -1187,18 +1188,19 @@ static int attn_decode_impl(const void* q, const void* k_cache, const void* v_ca
   p.window = window;
   p.chunk = chunk;
   p.scale_log2 = scale * 1.4426950408889634f;
+  p.status = status;
   return launch_decode_all(p, batch, q_per_seq, n_q_heads, n_kv_heads, key_dim, value_dim, stream, force_scratch);
 }
 
 // Up to 8 splits combine inside a thread-block cluster and ignore the scratch arguments (they may be null); more
-// splits need them.
+// splits need them. `status` (or null): an int32 word that says afterwards whether a wait of the kernel ran out.
 extern "C" int eredu_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
                                  const int* block_table, const int* seq_lens, const float* sinks, float* part_o,
                                  float* part_ml, int* counters, int batch, int q_per_seq, int max_pages, int n_q_heads,
                                  int n_kv_heads, int key_dim, int value_dim, int splits, int window, int chunk, float scale,
-                                 cudaStream_t stream) {
+                                 int* status, cudaStream_t stream) {
   return attn_decode_impl(q, k_cache, v_cache, out, block_table, seq_lens, sinks, part_o, part_ml, counters, batch, q_per_seq,
-                          max_pages, n_q_heads, n_kv_heads, key_dim, value_dim, splits, window, chunk, scale, stream, false);
+                          max_pages, n_q_heads, n_kv_heads, key_dim, value_dim, splits, window, chunk, scale, status, stream, false);
 }
 
 // Decode attention over the `window` newest tokens and the means of the blocks of `pool` tokens that end before them. pk / pv:
@@ -1242,7 +1244,7 @@ extern "C" int eredu_attn_decode_rope(const void* qkv, int ld_qkv, void* k_cache
                                       int q_per_seq, int max_pages, int n_q_heads, int n_kv_heads, int key_dim, int value_dim,
                                       int rot, int interleaved, int splits, int window, int chunk, int norm_whole,
                                       int value_norm, int append, float scale, float attn_factor, float norm_eps,
-                                      float norm_w_off, cudaStream_t stream) {
+                                      float norm_w_off, int* status, cudaStream_t stream) {
   if (qkv == nullptr || positions == nullptr || slots == nullptr || (inv_freq == nullptr && rot > 0)) return -1;
   if (rot < 0 || rot > key_dim || rot % 2 != 0 || ld_qkv % 2 != 0) return -1;
   if (norm_whole && (ld_qkv % 8 != 0 || (reinterpret_cast<uintptr_t>(qkv) & 15) != 0)) return -1;
@@ -1280,6 +1282,7 @@ extern "C" int eredu_attn_decode_rope(const void* qkv, int ld_qkv, void* k_cache
   p.splits = splits < 1 ? 1 : (splits > 64 ? 64 : splits);
   p.window = window;
   p.scale_log2 = scale * 1.4426950408889634f;
+  p.status = status;
   return launch_decode_all(p, batch, q_per_seq, n_q_heads, n_kv_heads, key_dim, value_dim, stream);
 }
 
@@ -1327,5 +1330,5 @@ extern "C" int eredu_attn_decode_static(const void* q, const void* k_cache, cons
   }
   // always the scratch form of the split reduction: that is the form whose scratch this entry point provides
   return attn_decode_impl(q, k_cache, v_cache, out, block_table, seq_lens, sinks, part_o, part_ml, counters, batch, q_per_seq,
-                          max_pages, n_q_heads, n_kv_heads, head_dim, head_dim, splits, window, 0, scale, stream, true);
+                          max_pages, n_q_heads, n_kv_heads, head_dim, head_dim, splits, window, 0, scale, nullptr, stream, true);
 }

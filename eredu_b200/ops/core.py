@@ -701,7 +701,8 @@ def attention_decode(q, k_cache, v_cache, block_table, seq_lens, q_per_seq, scal
         assert counters.numel() >= B * k_cache.shape[1] and counters.dtype == torch.int32
     code = lib().eredu_attn_decode(ptr(q), ptr(k_cache), ptr(v_cache), ptr(out), ptr(block_table), ptr(seq_lens),
                                    ptr(sinks), ptr(part_o), ptr(part_ml), ptr(counters), B, q_per_seq, block_table.stride(0), n_q,
-                                   k_cache.shape[1], q.shape[2], D, splits, window, chunk, scale, stream_ptr(q.device))
+                                   k_cache.shape[1], q.shape[2], D, splits, window, chunk, scale, ptr(status_word(q.device)),
+                                   stream_ptr(q.device))
     check(code, "eredu_attn_decode")
     return out
 
@@ -749,7 +750,7 @@ def attention_decode_rope(qkv, k_cache, v_cache, block_table, seq_lens, q_per_se
                                         block_table.stride(0), n_q, n_kv, head_dim, value_dim,
                                         head_dim if rot is None else rot, 1 if interleaved else 0, splits, window, chunk,
                                         int(norm_whole), int(value_norm), int(append) | (2 if settled else 0), scale, attn_factor, norm_eps,
-                                        norm_w_off, stream_ptr(qkv.device))
+                                        norm_w_off, ptr(status_word(qkv.device)), stream_ptr(qkv.device))
     check(code, "eredu_attn_decode_rope")
     return out
 

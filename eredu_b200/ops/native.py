@@ -21,12 +21,12 @@ _SIGNATURES = {
     "eredu_gemm_pick_split": (I, [I, I, I, I]),
     "eredu_gemm_bf16": (I, [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P, I, F, I, P, I, F, F, P]),
     "eredu_attn_prefill": (I, [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P]),
-    "eredu_attn_decode": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, P]),
+    "eredu_attn_decode": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, P, P]),
     "eredu_peer_send": (I, [P, I, I, P, L, P, I, P, P]),
     "eredu_peer_recv": (I, [P, I, I, P, L, P, I, P, P]),
     "eredu_attn_prefill_tc": (I, [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, F, P, P]),
     "eredu_attn_decode_scratch_elems": (None, [I, I, I, I, I, POINTER(L), POINTER(L)]),
-    "eredu_attn_decode_rope": (I, [P, I] + [P] * 14 + [I] * 15 + [F, F, F, F, P]),
+    "eredu_attn_decode_rope": (I, [P, I] + [P] * 14 + [I] * 15 + [F, F, F, F, P, P]),
     "eredu_rmsnorm": (I, [P, P, P, P, P, I, I, F, F, P]),
     "eredu_rope_kv": (I, [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, F, F, P]),
     "eredu_embedding": (I, [P, P, P, I, I, I, I, F, P, P]),
@@ -116,6 +116,7 @@ STATUS_NAMES = {
     3: "accumulator never committed",
     4: "peer flag never arrived",
     5: "bad argument",
+    6: "sums of another CTA never arrived",
 }
 
 

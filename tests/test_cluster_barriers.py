@@ -50,3 +50,27 @@ def test_sums_are_sent_behind_the_reads_of_the_round_before():
     """A CTA sends behind a barrier that follows its reads of the round before, so that who has its sums may write over what it has read. Its own
     sums take the same way: a plain store would need a barrier between itself and the reads as well."""
     assert round_of((KERNELS / "qgemv_stream.cu").read_text()) == ["finish_exchange", "__syncthreads", "store_async"]
+
+
+def silent_decisions(source):
+    """Lines that go by the outcome of a wait without a status word."""
+    return [number for number, line in enumerate(source.splitlines(), 1)
+            if re.search(r"mbar_wait\w*\([^;]*, nullptr, 0\)", line) and not re.search(r"^\s*(for \([^;]*;[^;]*;[^;]*\) )?mbar_wait\w*\(", line)]
+
+
+@pytest.mark.parametrize("text, lines", [("  for (int i = 0; i < n; ++i) mbar_wait(&full[i], 0, nullptr, 0);\n  mbar_wait(&bars[i], parity, nullptr, 0);", []),
+                                         ("const bool all = mbar_wait(&sent, 0, nullptr, 0);", [1]), ("if (!mbar_wait(&sent, 0, nullptr, 0)) return;", [1])])
+def test_reading_of_waits(text, lines):
+    assert silent_decisions(text) == lines
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in KERNELS.glob("*.cu*")))
+def test_waits_that_run_out_say_so(name):
+    """Results that a wait decides on are missing when it runs out; only copies on their way out of a kernel are waited for without a word."""
+    assert silent_decisions((KERNELS / name).read_text()) == []
+
+
+def test_status_codes_have_names():
+    codes = re.findall(r"kStatus\w+ = (\d+)", (KERNELS.parent / "common" / "ptx.cuh").read_text())
+    from eredu_b200.ops.native import STATUS_NAMES
+    assert sorted(map(int, codes)) == sorted(STATUS_NAMES)
