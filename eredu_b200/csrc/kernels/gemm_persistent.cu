@@ -180,10 +180,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (PAIR) {   // the other CTA's barriers and tensor memory are ready too
-    cluster_arrive_release();
-    cluster_wait_acquire();
-  }
+  // the other CTA's barriers and tensor memory are ready too
+  if (PAIR) cluster_arrive_release();
+  if (PAIR) cluster_wait_acquire();
   tc_fence_after_sync();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   pdl_wait();

@@ -7,12 +7,17 @@ import pytest
 KERNELS = Path(__file__).resolve().parents[1] / "eredu_b200" / "csrc" / "kernels"
 
 
+# what reaches into another CTA: stores by their instruction, and calls of the helpers around st.async, remote arrivals and copies that count there
+REMOTE = re.compile(r"st\.shared::cluster|(?<!void )\b(st_async\w*|store_async|mbar_arrive_cluster|tma_load_2d_pair_hint|umma_commit_pair)\(")
+HELPERS = re.compile(r"__device__ __forceinline__ void (\w+)\([^{]*\{[^}]*?(?:st\.async|mbarrier\.arrive\.shared::cluster|\.cta_group::2\.L2|multicast::cluster)")
+
+
 def unguarded_stores(source):
-    """Lines of remote stores that no wait on the cluster barrier dominates: a wait counts while the block that it stands in is open."""
+    """Lines of remote accesses that no wait on the cluster barrier dominates: a wait counts while the block that it stands in is open."""
     found, depth, waits = [], 0, []
     for number, line in enumerate(source.splitlines(), 1):
         code = re.sub(r"//.*", "", line)
-        if "st.shared::cluster" in code and not waits:
+        if REMOTE.search(code) and not waits:
             found.append(number)
         code = re.sub(r'"[^"]*"', '""', code)
         for token in re.findall(r"[{}]|cluster_wait_acquire\(\)", code):
@@ -30,9 +35,19 @@ def unguarded_stores(source):
 @pytest.mark.parametrize("text, lines", [
     ("void f() {\n cluster_wait_acquire();\n if (a) {\n  asm(\"st.shared::cluster.f32 [%0], {%1};\");\n }\n}", []),
     ("void f() {\n if (a) {\n  cluster_wait_acquire();\n }\n asm(\"st.shared::cluster.f32\");\n}", [5]),
-    ("void f() {\n cluster_wait_acquire();\n}\nvoid g() {\n asm(\"st.shared::cluster.f32\");\n}", [5])])
+    ("void f() {\n cluster_wait_acquire();\n}\nvoid g() {\n asm(\"st.shared::cluster.f32\");\n}", [5]),
+    ("void st_async(uint32_t a) {\n asm(\"st.async.weak\");\n}\nvoid f() {\n st_async(a);\n cluster_wait_acquire();\n st_async(b);\n}", [5]),
+    ("void f() {\n store_async(a, v, b);\n st_async_f32(a, v, b);\n mbar_arrive_cluster(b);\n umma_commit_pair(b);\n}", [2, 3, 4, 5]),
+    ("void f() {\n if (PAIR) cluster_wait_acquire();\n if (PAIR) tma_load_2d_pair_hint(a);\n}", [])])
 def test_reading_of_blocks(text, lines):
     assert unguarded_stores(text) == lines
+
+
+def test_helpers_of_remote_accesses_are_known():
+    """A helper around one of these instructions is looked for by its name."""
+    sources = sorted(KERNELS.glob("*.cu*")) + [KERNELS.parent / "common" / "ptx.cuh"]
+    names = {name for path in sources for name in HELPERS.findall(path.read_text())}
+    assert len(names) >= 6 and all(REMOTE.search(f" {name}(") for name in names), names
 
 
 @pytest.mark.parametrize("name", sorted(p.name for p in KERNELS.glob("*.cu*")))
