@@ -67,6 +67,13 @@ class SpeculativeDecoder:
         pages = np.asarray(seq.pages, dtype=np.int64)
         return pages[positions // PAGE] * PAGE + (positions % PAGE)
 
+    @staticmethod
+    def _splits(eng: Engine, batch: int, tokens: int, longest: int) -> int:
+        """Split-KV factor of a step of ``tokens`` per sequence: a drafter's single tokens are split like those of any decode step."""
+        if tokens == 1:
+            return eng.decode_splits(batch, longest)
+        return ops.decode_splits(batch, eng.model.n_kv_local, longest, eng.sm_count) if eng.cuda else 1
+
     def _multi_token_step(self, eng: Engine, seqs, tokens: list[list[int]], all_rows: bool, uniform: bool, prepare=None):
         """Feed ``tokens[i]`` to sequence i starting at its kv_len. Returns logits of every fed row (all_rows) or
         of the last row of each sequence. Uniform token counts use the split-KV decode kernel, ragged counts the
@@ -82,7 +89,7 @@ class SpeculativeDecoder:
                       slots=eng._t(np.concatenate([self._slots(s, p) for s, p in zip(seqs, pos)]), torch.int64),
                       block_table=eng._block_table(seqs), seq_lens=eng._t(kv_after, torch.int32), logit_rows=rows)
         if uniform and len(set(lens)) == 1:
-            splits = ops.decode_splits(len(seqs), eng.model.n_kv_local, int(kv_after.max()), eng.sm_count) if eng.cuda else 1
+            splits = self._splits(eng, len(seqs), lens[0], int(kv_after.max()))
             batch = ForwardBatch(is_prefill=False, q_per_seq=lens[0], splits=splits, **common)
         else:
             batch = ForwardBatch(is_prefill=True, cu_q=eng._t(cu.astype(np.int32), torch.int32), max_q_len=max(lens),
@@ -715,7 +722,7 @@ class GraphSpeculativeDecoder(SpeculativeDecoder):
             "all_greedy": sp.greedy, "graph": None,
         }
         for name, eng, q in (("d2", d, 2), ("d1", d, 1), ("tv", t, k + 1)):
-            splits = ops.decode_splits(B, eng.model.n_kv_local, max_len + k + 2, eng.sm_count)
+            splits = self._splits(eng, B, q, max_len + k + 2)
             st[name + "_splits"] = splits
             st[name + "_scratch"] = (ops.decode_scratch(B, q, eng.model.n_q_local, eng.cfg.head_dim, splits, dev)
                                      if splits > 1 else None)

@@ -34,6 +34,16 @@ def _run(device, dtype, draft_seed, sp, k=4, n_new=30):
     return plain, spec, dec.stats.summary()
 
 
+def test_single_drafted_tokens_are_split_like_a_decode_step(monkeypatch):
+    """A drafter's steps of one token run the kernels of any decode step, and take their plan; the verification of several has its own."""
+    asked = []
+    monkeypatch.setattr(Engine, "decode_splits", lambda self, batch, longest: asked.append((self, batch, longest)) or 1)
+    cfg, target, draft = _models("cpu", torch.float32, 7)
+    dec = SpeculativeDecoder(Engine(target, max_batch=2, max_seq_len=128), Engine(draft, max_batch=2, max_seq_len=128), k=4)
+    dec.generate([[1, 2, 3], [4, 5, 6, 7]], SamplingParams(temperature=0.0), 8)
+    assert asked and all(eng is dec.d and batch in (1, 2) and longest > 4 for eng, batch, longest in asked)
+
+
 @pytest.mark.parametrize("draft_seed", [None, 7])
 def test_greedy_speculation_is_exact_cpu(draft_seed):
     plain, spec, stats = _run("cpu", torch.float32, draft_seed, SamplingParams(temperature=0.0))
