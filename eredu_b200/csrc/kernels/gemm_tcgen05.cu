@@ -389,12 +389,12 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       if (lane == 0) s_ssq[q][c] = sq;
     }
   };
-  // After every owned column went through finish(): publish the per-row partial sums of squares.
-  auto publish_ssq = [&](int c_first, int c_step) {
+  // After every column went through finish(): publish the per-row partial sums of squares.
+  auto publish_ssq = [&]() {
     if (p.ssq_out == nullptr) return;
     epi_barrier();
     for (int c = et; c < TN; c += 128) {
-      if (c >= c_first && (c - c_first) % c_step == 0 && m_base + c < m_limit)
+      if (m_base + c < m_limit)
         p.ssq_out[static_cast<size_t>(m_base + c) * gridDim.x + tile_n] = s_ssq[0][c] + s_ssq[1][c] + s_ssq[2][c] + s_ssq[3][c];
     }
   };
@@ -445,19 +445,14 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
       epi_barrier();
     }
-    // Residual values of the first kPre columns (COMM_AR: column pairs) this thread will finish: the loads are
-    // in flight while the tensor cores work, instead of one dependent load per finished column.
-    if (has_res) {
+    // COMM_AR: residual values of the first kPre column pairs this thread will finish: the loads are in flight while the tensor cores
+    // work, instead of one dependent load per finished column.
+    if (COMM == COMM_AR && has_res) {
 #pragma unroll
       for (int j = 0; j < kPre; ++j) {
-        if (COMM == COMM_AR) {
-          const int c = 2 * (own_first + j * own_step);
-          if (c < m_end) rpre[2 * j] = residual_at(p, m_base + c, n);
-          if (c + 1 < m_end) rpre[2 * j + 1] = residual_at(p, m_base + c + 1, n);
-        } else if (SPLIT && COMM != COMM_NONE) {
-          const int c = own_first + j * own_step;
-          if (c < m_end) rpre[j] = residual_at(p, m_base + c, n);
-        }
+        const int c = 2 * (own_first + j * own_step);
+        if (c < m_end) rpre[2 * j] = residual_at(p, m_base + c, n);
+        if (c + 1 < m_end) rpre[2 * j + 1] = residual_at(p, m_base + c + 1, n);
       }
     }
     if (kQuads) {
@@ -576,7 +571,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         }
       }
     } else if (!SPLIT && COMM == COMM_NONE) {
-      publish_ssq(0, 1);
+      publish_ssq();
     }
   }
 
@@ -727,42 +722,21 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
     }
   } else if (SPLIT) {
+    // COMM_AG: the sums go to every rank, without a residual
     if (warp >= 2) {
       cg::cluster_group cluster = cg::this_cluster();
       const float* peers[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r) peers[r] = cluster.map_shared_rank(red, r < nsplit ? r : 0);
-      // all remote loads of a column are issued together; the sum runs in cluster-rank order (deterministic)
-      auto reduce_col = [&](int c, float& g, float& u) {
-        float pg[8], pu[8];
+      for (int c = split; c < m_end; c += nsplit) {  // warp-uniform
+        // all remote loads of a column are issued together; the sum runs in cluster-rank order (deterministic)
+        float part[8], g = 0.f;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          pg[r] = (r < nsplit) ? peers[r][c * 128 + row] : 0.f;
-          if (DUAL) pu[r] = (r < nsplit) ? peers[r][(TN + c) * 128 + row] : 0.f;
-        }
-        g = 0.f;
-        u = 0.f;
+        for (int r = 0; r < 8; ++r) part[r] = (r < nsplit) ? peers[r][c * 128 + row] : 0.f;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          g += pg[r];
-          if (DUAL) u += pu[r];
-        }
-      };
-#pragma unroll
-      for (int j = 0; j < kPre; ++j) {
-        const int c = split + j * nsplit;
-        if (c < m_end) {  // warp-uniform
-          float g, u;
-          reduce_col(c, g, u);
-          finish(g, u, c, true, rpre[j]);
-        }
+        for (int r = 0; r < 8; ++r) g += part[r];
+        finish(g, 0.f, c, true, 0.f);
       }
-      for (int c = split + kPre * nsplit; c < m_end; c += nsplit) {
-        float g, u;
-        reduce_col(c, g, u);
-        finish(g, u, c, true, has_res ? residual_at(p, m_base + c, n) : 0.f);
-      }
-      if (COMM == COMM_NONE) publish_ssq(split, nsplit);
     }
   }
   if (SPLIT && !pushed) {

@@ -553,8 +553,8 @@ extern "C" int eredu_qgemv4(const void* X, const void* wq, const void* dq, void*
     p.use_comm = 1;
     p.comm = *pc;
   }
-  // One or two tokens of larger matrices: the persistent kernel on integer products (force_wk = -1, with force_ns: always; -2: never)
-  if (group >= 64 && force_exact_bf16 == 0 && comm == nullptr && M <= kQGemvStreamTokens && (force_wk == -1 || (force_wk == 0 && force_ns == 0))) {
+  // One or two tokens of larger matrices: the persistent kernel on integer products
+  if (group >= 64 && force_exact_bf16 == 0 && comm == nullptr && M <= kQGemvStreamTokens && force_wk == 0 && force_ns == 0) {
     QGemvStreamParams q = {};
     q.x = p.x;
     q.wq = p.wq;
@@ -572,7 +572,7 @@ extern "C" int eredu_qgemv4(const void* X, const void* wq, const void* dq, void*
     q.out_fp32 = p.out_fp32;
     q.limit = p.limit;
     q.status = p.status;
-    const int r = launch_qgemv_stream(q, gated != 0, force_wk == -1 ? std::max(1, force_ns) : 0, sm_count, stream);
+    const int r = launch_qgemv_stream(q, gated != 0, sm_count, stream);
     if (r != kQGemvStreamUnsupported) return r;
   }
   // Row tiles of a warp and K splits. Four tiles take the fewest instructions per row and win wherever the kernel is bound by issue; a matrix

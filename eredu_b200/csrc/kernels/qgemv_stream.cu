@@ -444,15 +444,15 @@ static int pick_splits(const QGemvStreamParams& p, bool gated, int sms) {
   return p.kblocks * tiles >= (p.M == 1 ? 480 : p.kblocks >= 48 ? 440 : 1000) ? 1 : 0;
 }
 
-int launch_qgemv_stream(QGemvStreamParams p, bool gated, int force_ns, int sm_count, cudaStream_t stream) {
+int launch_qgemv_stream(QGemvStreamParams p, bool gated, int sm_count, cudaStream_t stream) {
   if (p.M < 1 || p.M > kQGemvStreamTokens || p.group_shift < 6 || p.group_shift > 7) return kQGemvStreamUnsupported;
   const int sms = sm_count > 0 ? sm_count : 148;
   p.units = (p.n_out + 15) / 16;
-  p.ns = force_ns > 0 ? force_ns : pick_splits(p, gated, sms);
+  p.ns = pick_splits(p, gated, sms);
   if (p.ns == 0) return kQGemvStreamUnsupported;
   p.kb_cta = ((p.kblocks + p.ns - 1) / p.ns + kChunk - 1) / kChunk * kChunk;          // starts on a group
-  if (p.ns > 8 || (p.ns & (p.ns - 1)) != 0 || smem_bytes(p, gated, p.ns, p.kb_cta, 2) > kMaxSmem) return kQGemvStreamUnsupported;
-  const int clusters = std::min(p.units, std::max(1, (p.ns > 2 ? sms * 7 / 8 : sms) / p.ns));     // clusters of more than two find seven eighths of the SMs
+  if (smem_bytes(p, gated, p.ns, p.kb_cta, 2) > kMaxSmem) return kQGemvStreamUnsupported;
+  const int clusters = std::min(p.units, std::max(1, sms / p.ns));
   p.kb_warp = ((p.kb_cta + kWarps - 1) / kWarps + kChunk - 1) / kChunk * kChunk;   // a warp's slots start on a group
   p.slots = 2;
   while (p.slots < kMaxSlots && smem_bytes(p, gated, p.ns, p.kb_cta, p.slots + 1) <= kMaxSmem) ++p.slots;

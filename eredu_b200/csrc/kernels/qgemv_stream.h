@@ -1,5 +1,5 @@
 // Launcher of the persistent 4-bit decode kernel (qgemv_stream.cu), called by eredu_qgemv4. Returns a cudaError_t, or
-// kQGemvStreamUnsupported where the activations of a CTA do not fit in its shared memory.
+// kQGemvStreamUnsupported where the register kernel (qgemv_mma.cu) is the faster one or the activations of a CTA do not fit in its shared memory.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -27,10 +27,10 @@ struct QGemvStreamParams {
   // set by the launcher
   int units;            // tiles of 16 output rows
   int kb_cta, kb_warp;  // K blocks of a CTA of the cluster, and of a warp
-  int ns;               // CTAs of a cluster, which split K
+  int ns;               // CTAs of a cluster, which split K: one or two
   int slots;            // of a warp's ring
 };
 
-int launch_qgemv_stream(QGemvStreamParams p, bool gated, int force_ns, int sm_count, cudaStream_t stream);
+int launch_qgemv_stream(QGemvStreamParams p, bool gated, int sm_count, cudaStream_t stream);
 
 }  // namespace eredu
