@@ -54,7 +54,7 @@ struct AttnParams {
   int norm_whole;   // the norms run over the whole q and the whole k projection (weights of that size) instead of per head
   int value_norm;   // weight-free RMSNorm of every new value head
   int append;       // 0: qkv rows hold queries only, the keys and values of the step are in the pages already
-  int settled;      // the kernel just before this one writes none of the pages, tables and lengths (only qkv): see attn_decode_kernel
+  int settled;      // the kernel just before this one writes qkv only: no pages, tables, lengths, positions, slots or frequencies, see attn_decode_kernel
   // splits > 1: 1 = the `splits` CTAs of a (sequence, kv head) form a thread-block cluster and combine their partial
   // results through distributed shared memory (no global scratch, no arrival tickets); 0 = scratch + last-arriver.
   int cluster_reduce;
@@ -406,9 +406,9 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(AttnParams p) {
 // walked like a page, in front of the pages of the window.
 // A step of one sequence is bound by a chain of latencies: length, table, first pages, rows of the projection and their turn, then little
 // arithmetic and the exchange of the splits. The turn of a single new token and its slot are taken, and three pages asked for, before the rows
-// are waited for (one sequence of 2048, 32 heads of 128 over 8: 10.0 -> 8.8 us, 7.5 with eight warps). With p.settled only the projection comes from the kernel before this one - what the lengths, tables and pages
-// hold was written by kernels that had ended when that one passed its own dependency wait - so the first links run ahead of the
-// wait, under the tail of the projection. That holds because a kernel releases the next one behind its own wait; a build that releases at
+// are waited for (one sequence of 2048, 32 heads of 128 over 8: 10.0 -> 8.8 us, 7.5 with eight warps). With p.settled only the projection comes
+// from the kernel before this one - what the lengths, tables, pages, positions and slots hold was written by kernels that had ended when that
+// one passed its own dependency wait - so the first links run ahead of the wait, under the tail of the projection. That holds because a kernel releases the next one behind its own wait; a build that releases at
 // entry (EREDU_PDL_EARLY=1) waits first. Measured over whole decode steps: one sequence, 16 layers of 64-wide heads, three draft passes
 // 2917 -> 2870 us; one sequence, 32 layers of 128-wide heads 3687 -> 3660 us; 32 sequences of the same 5499 -> 5475 us.
 template <int DK, int DV, int MT, bool EXT, bool POOL, int NW>
@@ -1236,7 +1236,7 @@ extern "C" int eredu_attn_decode_pooled(const void* q, const void* k_cache, cons
 // the new k rows by `positions`, appends the new k / v rows at `slots` (page * 16 + offset; negative: not stored)
 // and attends - the RoPE + KV-append launch of the unfused path disappears. Every new row is appended by the one CTA
 // whose page range contains it, before that CTA fetches the page. append: bit 0 as said, bit 1: the kernel launched just before this call
-// writes neither pages nor tables nor lengths (`settled`). Other arguments as eredu_attn_decode.
+// writes qkv only - no pages, tables, lengths, positions, slots or frequencies (`settled`). Other arguments as eredu_attn_decode.
 extern "C" int eredu_attn_decode_rope(const void* qkv, int ld_qkv, void* k_cache, void* v_cache, void* out,
                                       const int* block_table, const int* seq_lens, const float* sinks, float* part_o,
                                       float* part_ml, int* counters, const int* positions, const long long* slots,

@@ -716,8 +716,8 @@ def attention_decode_rope(qkv, k_cache, v_cache, block_table, seq_lens, q_per_se
     head sizes without a kernel compose the two reference operators.
     ``norm_whole`` / ``value_norm`` / ``append``: the preparation of :func:`qkv_prepare` (norms over whole projections, value
     heads of width ``value_dim``, rows that hold queries only) instead of that of :func:`rope_kv`.
-    ``settled``: the kernel enqueued just before this call writes ``qkv`` only, not the pages, ``block_table`` or ``seq_lens`` (the
-    projection of a decode step); these are then read ahead of the stream dependency on it."""
+    ``settled``: the kernel enqueued just before this call writes ``qkv`` only, not the pages, ``block_table``, ``seq_lens``, ``positions``, ``slots``
+    or ``inv_freq`` (the projection of a decode step); these are then read ahead of the stream dependency on it."""
     value_dim = value_dim or head_dim
     if norm_whole or value_norm or not append or value_dim != head_dim or chunk:
         whole = (qkv.is_cuda and qkv.dtype == torch.bfloat16 and _tma_rows(qkv) and head_dim % 8 == 0 and value_dim % 8 == 0

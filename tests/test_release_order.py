@@ -21,3 +21,14 @@ def test_norm_weights_are_read_behind_the_wait():
     kernel = source[source.index("rmsnorm_kernel(const"):]
     ahead = kernel[:kernel.index("pdl_wait();")]
     assert not re.search(r"\(w\)\[|= w\[", ahead)
+
+
+def test_what_decode_attention_reads_ahead_is_promised_by_its_caller():
+    """Everything that the kernel reads in front of its wait when its surroundings are settled is named where callers say that they are."""
+    from eredu_b200 import ops
+    source = (KERNELS / "attention.cu").read_text()
+    kernel = source[source.index("attn_decode_kernel(AttnParams p) {"):]
+    ahead = kernel[:kernel.index("if (settled) {")]
+    arrays = set(re.findall(r"p\.(block_table|seq_lens|positions|slots|q_norm_w|k_norm_w|sinks)\b", ahead)) | ({"inv_freq"} if "turn_at" in ahead else set())
+    promise = ops.attention_decode_rope.__doc__.partition("``settled``")[2]
+    assert {"positions", "slots"} <= arrays and all(f"``{name}``" in promise for name in arrays), arrays
