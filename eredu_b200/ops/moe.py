@@ -165,10 +165,12 @@ def expert_tile(routes: int, e_local: int, inter: int, hidden: int, plain: bool)
     one is stored; it takes over where an expert's rows no longer fit one small item, or a little earlier. Both grouped GEMMs, us with
     items of 16 / 32 / 64 / 256 rows: 128 experts of 768 x 2048, 12 rows an expert 182 / 205 / 255 / 190, 16 rows 207 / 211 / 256 / 191, 24 rows 258 / 222 /
     258 / 193, 64 rows 463 / 345 / 279 / 213; 64 of 1408 x 2048, 12 rows 169 / 187 / 224 / 175, 16 rows 183 / 190 / 224 / 175. Few experts have fewer of its
-    tiles to spread over the SMs: 8 of 14336 x 4096 with items of 32 / 256 rows, 32 rows an expert 434 / 467, 40 rows 713 / 470; where all of
-    them have fewer such tiles than there are SMs, later still: 4 of 1024 x 1024, 40 rows 16.5 / 17.3, 50 rows 19.3 / 17.8."""
+    tiles to spread over the SMs. Routes are not even: with 27 rows an expert some have more than 32 and a second item (items of 32 / 256 rows, logits drawn
+    at random: 8 of 14336 x 4096, 24 rows 442 / 477, 28 rows 459 / 478, 32 rows 557 / 479; 16 of 2048 x 2048, 26 rows 86.5 / 85.4, 30 rows 105.5 / 85.3; 32 of
+    512 x 1024, 28 rows 46.3 / 36.1). Where all of them have fewer such tiles than there are SMs, later still: 4 of 1024 x 1024, 40 rows 24.5 / 25.1, 44
+    rows 27.3 / 25.2."""
     per = routes / max(1, e_local)
-    return 256 if plain and per > (14 if e_local >= 64 else 32 if e_local * inter > 148 * 64 else 40) and inter % 64 == 0 and hidden % 8 == 0 else pick_tile(per)
+    return 256 if plain and per > (14 if e_local >= 64 else 26 if e_local * inter > 148 * 64 else 40) and inter % 64 == 0 and hidden % 8 == 0 else pick_tile(per)
 
 
 def route_plan_gather(logits, x, k, scoring, renorm, scale, sel_bias, e0, n_local, n_group=1, topk_group=1):

@@ -2,7 +2,7 @@
 import pytest
 
 from eredu_b200 import ops
-from eredu_b200.ops import native
+from eredu_b200.ops import moe, native
 
 
 @pytest.mark.parametrize("sms", [132, 148, 160])
@@ -24,3 +24,10 @@ def test_long_contexts_do_not_leave_most_of_the_gpu_idle(ctas, head_dim):
     assert plan(512) <= ops.CLUSTER_SPLITS and plan(512) * ctas <= 148
     for tokens in (32768, 65536, 131072):
         assert plan(tokens) == ops.decode_splits(ctas, 1, tokens, 148)
+
+
+@pytest.mark.parametrize("experts, inter", [(8, 14336), (16, 2048), (32, 512), (48, 768)])
+def test_items_of_few_experts_leave_room_for_uneven_routes(experts, inter):
+    """With 27 rows an expert on average, some have more than the 32 of a small item."""
+    assert moe.expert_tile(26 * experts, experts, inter, 2048, True) == 32
+    assert all(moe.expert_tile(rows * experts, experts, inter, 2048, True) == 256 for rows in range(27, 34))
