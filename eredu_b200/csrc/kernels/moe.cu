@@ -329,13 +329,15 @@ __device__ __forceinline__ void plan_few(const int* s_ids, int routes, int k, in
       before += other == e && r < lane;
       same += other == e;
     }
-    // (a token may choose an expert twice: where the kept groups hold fewer experts than it chooses)
-    const bool opens = e >= 0 && before % tile == 0;       // the first row of an item
+    // A token may choose an expert twice, where the kept groups hold fewer experts than it chooses: only then can there be more rows than one item
+    // has (dividing by the size of an item in every plan: 4.45 us for one token instead of 4.18, 7.8 instead of 7.0 for four).
+    const bool several = __any_sync(0xffffffffu, e >= 0 && same > tile);
+    const bool opens = e >= 0 && (before == 0 || (several && before % tile == 0));       // the first row of an item
     const unsigned firsts = __ballot_sync(0xffffffffu, opens);
-    int item = 0;                               // items in front
+    int item = several ? before / tile : 0;     // items in front: of this expert, and of those before it
     for (int r = 0; r < routes; ++r) {
       const int other = __shfl_sync(0xffffffffu, e, r);
-      item += ((firsts >> r) & 1u) && (other < e || (other == e && r < lane));
+      item += ((firsts >> r) & 1u) && other < e;
     }
     const int rows = __popc(__ballot_sync(0xffffffffu, e >= 0));
     if (lane < routes) route_pos[lane] = e >= 0 ? smaller + before : -1;
