@@ -1,4 +1,4 @@
-// Persistent tcgen05 GEMM for prefill-sized problems (more than 128 tokens): Y = X W^T with the same fused
+// Persistent tcgen05 GEMM for prefill-sized problems (more than 128 tokens, from 65 on where K is not split): Y = X W^T with the same fused
 // epilogues as the one-tile-per-CTA kernel (RMSNorm row scale, bias, residual, SwiGLU, sums of squares for the
 // next norm), built so that the tensor cores never wait for an epilogue:
 //

@@ -401,7 +401,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 
   // Split sums without a collective: a warp finishes a column at a time, a lane four of its rows (16 bytes of every CTA's partial sums, 8 of
   // the residual and of the result). With a row a thread and a column after the other, each of them waited for its remote loads: 0.4 us a
-  // column (4096 x 14336: 23.5 us with 45 tokens, 20.9 now; 6144 x 4096 with 64 18.4 and 13.1).
+  // column (4096 x 14336: 23.6 us with 45 tokens, 21.7 now; 6144 x 4096 with 64 17.7 and 14.1; 5120 x 2048 with 45 11.2 and 8.8).
   constexpr int kAhead = 4;
   const int qn = tile_n * 128 + lane * 4;      // first of the lane's rows
   const bool whole = (p.N & 3) == 0 && (p.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 &&
@@ -978,8 +978,10 @@ static int pick_split(int M, int N, int K, int tn, int ctas_per_sm, int sm_count
   const int kblocks = (K + 63) / 64;
   if (tn == 128) {
     // One CTA to an SM: clusters of eight find two thirds of the SMs and of four seven eighths; what splits less goes to the persistent kernel.
-    // 100 tokens: 4096 x 4096 22.6 us unsplit, 19.3 there, 14.3 split four times, 4096 x 14336 52.9, 52.5 and 26.3, 2048 x 4096 21.9, 18.6 and 12.4
-    // (eight times 16.3); 6144 x 4096 23.5 and 20.3, split twice 21.1, 2 x 14336 x 4096 59 and 52, 2 x 8192 x 2048 34 and 20.8, split twice 26.4.
+    // 100 tokens: 4096 x 4096 22.3 us unsplit, 13.8 split four times, 4096 x 14336 52.8 and 25.5, 2048 x 4096 21.5 and 11.9 (eight times 16.2); 6144 x 4096
+    // 22.9, split twice 19.7, there 18.9, 14336 x 4096 30, 41 and 25.8, 2 x 14336 x 4096 59, 68 and 48, 2 x 6144 x 2048 33, 25 and 16.6. Short sums are over
+    // before a cluster has met: 4096 x 512 unsplit 10.9, split four times 8.9, there 6.0, 1024 x 256 9.9, 7.7 and 4.4, 4096 x 960 12.3, 9.5 and 7.8, 2 x 4096 x
+    // 512 22.9, 13.1 and 7.4; only narrow ones of 65 tokens have a little to lose (2 x 1024 x 960 28, 8.6 split eight times, there 10.0).
     return kblocks < 16 ? 1 : tiles * 8 <= sm_count / 2 ? 8 : tiles * 4 <= sm_count * 7 / 8 ? 4 : 1;
   }
   int s = 1;
@@ -1011,7 +1013,7 @@ extern "C" int eredu_gemm_bf16(const void* X, const void* W, void* Y, const void
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   // A narrow output over many tokens (a router) fills the machine with small token tiles instead. K is not split: experts that score alike
-  // change places with the order of a sum, and this one is the same for every number of tokens above 64. What smaller tiles save is the serial epilogue of
+  // change places with the order of a sum, and this one is the same for every number of tokens above 64 (128 x 2048, 100 tokens: 11.2 us, split 6.6). What smaller tiles save is the serial epilogue of
   // their columns, as long as one round of CTAs holds them: 1024 x 128 x 2048 10.6 us with 16 tokens, 4096 tokens 13.2 with 32. Few rows of
   // weights that all CTAs fetch at once stand a quarter of the CTAs (1024 x 8 x 2048: 15.5 to 24.8 us with 16 tokens, by where the rows lie,
   // 18.0 with 32).
